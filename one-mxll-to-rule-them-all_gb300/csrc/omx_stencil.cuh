@@ -541,8 +541,30 @@ __global__ void k_e1(FieldPtrs<R> F, GridArgs<R> G)
 }
 
 // ===================================================================================== launchers
-constexpr int KCH3 = 16;   // planes marched per 3D thread
-constexpr int JCH2 = 32;   // rows marched per 2D thread
+// Planes (3D, at most 16) or rows (2D, at most 8) marched per thread: the longest power-of-two
+// march that still leaves `want` blocks of 128 threads per SM.  A longer march reads the carried
+// neighbour less often; a shorter one has more threads in flight, which decides on grids that do
+// not fill the GPU (with a march of 16 planes / 32 rows for every grid, a thread's serial chain of
+// memory trips was the whole pass there).  Measured, us per step at marches of 1, 2, 4, 8, 16 (32):
+// 3D FP32 32^3 11.5, 12.6, 16.7, 23.7, 37.2; 101 x 90 x 157 34.0, 28.0, 26.5, 28.3, 29.2;
+// 200 x 180 x 220 200, 158, 143, 141, 144; 3D FP64 (compute bound, so the reads it saves count
+// less) 64^3 91, 97, 111, 123, 150, 200^3 1253, 1244, 1236, 1257, 1277; 2D FP32 TMz 243 x 161 22.9,
+// 23.9, 25.0, 27.7, 31.9 (42.1), TEz 1531 x 1147 31.7, 27.1, 25.6, 29.4, 32.3 (52.2), 4096^2 288,
+// 219, 192, 180, 184 (196).
+inline int march_rule(long long tiles, int n, int most, int want)
+{
+    int m = most;
+    while (m > 1 && tiles * ((n + m - 1) / m) < 152LL * want) m /= 2;
+    return m;
+}
+template <class R> inline int march_of(const GridArgs<R> &G)
+{
+    const Lay &L = G.L;
+    if (G.march > 0) return G.march;
+    const bool f4 = sizeof(R) == 4;
+    if (L.dims == 3) return march_rule((long long)((L.nx + 31) / 32) * ((L.ny + 3) / 4), L.nz, 16, f4 ? 24 : 64);
+    return march_rule((L.nx + 127) / 128, L.ny, 8, 16);
+}
 
 template <class R, bool EXACT>
 void launch_h_impl(const FieldPtrs<R> &F, const GridArgs<R> &G, void *stream)
@@ -550,11 +572,11 @@ void launch_h_impl(const FieldPtrs<R> &F, const GridArgs<R> &G, void *stream)
     cudaStream_t s = (cudaStream_t)stream;
     const Lay &L = G.L;
     if (L.dims == 3) {
-        const int m = G.march > 0 ? G.march : KCH3;
+        const int m = march_of(G);
         dim3 b(32, 4, 1), g((L.nx + 31) / 32, (L.ny + 3) / 4, (L.nz + m - 1) / m);
         k_h3<R, EXACT><<<g, b, 0, s>>>(F, G, m);
     } else if (L.dims == 2) {
-        const int m = G.march > 0 ? G.march : JCH2;
+        const int m = march_of(G);
         dim3 b(128, 1, 1), g((L.nx + 127) / 128, (L.ny + m - 1) / m, 1);
         k_h2<R, EXACT><<<g, b, 0, s>>>(F, G, m);
     } else {
@@ -569,11 +591,11 @@ void launch_e_impl(const FieldPtrs<R> &F, const GridArgs<R> &G, void *stream)
     const Lay &L = G.L;
     if (G.ade_n > 0) k_ade<R><<<(G.ade_n + 127) / 128, 128, 0, s>>>(F, G);
     if (L.dims == 3) {
-        const int m = G.march > 0 ? G.march : KCH3;
+        const int m = march_of(G);
         dim3 b(32, 4, 1), g((L.nx + 31) / 32, (L.ny + 3) / 4, (L.nz + m - 1) / m);
         k_e3<R, EXACT><<<g, b, 0, s>>>(F, G, m);
     } else if (L.dims == 2) {
-        const int m = G.march > 0 ? G.march : JCH2;
+        const int m = march_of(G);
         dim3 b(128, 1, 1), g((L.nx + 127) / 128, (L.ny + m - 1) / m, 1);
         k_e2<R, EXACT><<<g, b, 0, s>>>(F, G, m);
     } else {

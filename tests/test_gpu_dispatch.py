@@ -1,0 +1,66 @@
+"""Kernel variants chosen by size, type and alignment, at the sizes where a choice or its remainder
+can go wrong, against the FP64 oracle or the general path."""
+import numpy as np
+import pytest
+
+import omx
+
+pytestmark = pytest.mark.gpu
+
+
+def seeded_pair(orc, dims, n, npml, bnd, dr, mode, amp, seed, precision="fp64"):
+    """A library grid and an oracle grid with the same random E fields of amplitude amp."""
+    dt = omx.units.yee_dt(dr)
+    gpu = omx.TMxll(dims, n, npml, bnd, dt, dr, mode=mode, precision=precision)
+    cpu = orc.Grid(dims, n, npml, bnd, dt, dr, mode=mode)
+    rng = np.random.default_rng(seed)
+    comps = {1: [1], 2: [3] if mode == omx.TMZ else [1, 2], 3: [1, 2, 3]}[dims]
+    for f in comps:
+        lo, hi = gpu.field_bounds(f)
+        a = np.zeros([h - b + 1 for b, h in zip(lo, hi)], order="F")
+        own = tuple(slice(1 - lo[x], 1 - lo[x] + n[x]) if x < dims else slice(None) for x in range(3))
+        a[own] = amp * rng.standard_normal(a[own].shape) * (rng.random(a[own].shape) < 0.8)
+        if dims == 1:
+            a[0] = a[-1] = 0.0
+        gpu.write_field(f, a)
+        cpu.write_field(f, a)
+    return gpu, cpu, dt
+
+
+def advance(gpu, cpu, dt, steps, calls=False):
+    if calls:
+        for tt in range(1, steps + 1):
+            gpu.td_propagate_H_field()
+            gpu.source_interactions(dt * (tt - 0.5))
+            gpu.td_propagate_E_field(dt * (tt - 0.5), 0.0)
+    else:
+        gpu.run(1, steps)
+    for tt in range(1, steps + 1):
+        cpu.td_propagate_H_field()
+        cpu.td_propagate_E_field(dt * (tt - 0.5), 0.0)
+
+
+FIELDS_OF = {(1, 1): [1, 5], (2, 1): [3, 4, 5], (2, 2): [1, 2, 6], (3, 1): [1, 2, 3, 4, 5, 6]}
+
+
+# sizes at the edges of the blocks (32 x 4 columns, 128 cells), of the marches (1..16 planes, 1..8 rows)
+# and of the CPML slabs
+@pytest.mark.parametrize("dims,n,npml,bnd,mode", [
+    (1, (64,), 6, (3, 1, 1), 1),
+    (2, (129, 33), 5, (3, 3, 1), 1),
+    (2, (127, 70), 5, (2, 3, 1), 2),
+    (2, (640, 641), 6, (3, 2, 1), 2),
+    (3, (33, 29, 26), 4, (3, 3, 3), 1),
+    (3, (31, 17, 65), 5, (2, 3, 3), 1),
+])
+@pytest.mark.parametrize("amp,dr", [(1.0, 37.794522518155646)])
+def test_fp64_passes_bit_identical(orc, dims, n, npml, bnd, mode, amp, dr):
+    gpu, cpu, dt = seeded_pair(orc, dims, n, npml, bnd, dr, mode, amp, sum(n))
+    advance(gpu, cpu, dt, 5)
+    for f in FIELDS_OF[(dims, mode)]:
+        a, b = gpu.read_field(f), cpu.read_field(f)
+        lo, _ = gpu.field_bounds(f)
+        own = tuple(slice(1 - lo[x], 1 - lo[x] + n[x]) if x < dims else slice(None) for x in range(3))
+        assert np.array_equal(a[own], b[own])
+        assert amp < 1e-300 or np.max(np.abs(b[own])) > 0
+    gpu.kill()
