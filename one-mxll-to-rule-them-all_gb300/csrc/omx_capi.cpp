@@ -544,6 +544,12 @@ template <class R> GridArgs<R> grid_args(omx_ctx *c)
     G.dt_mu0 = (R)dt_mu0;
     G.dt_eps0 = (R)dt_eps0;
     G.dr = (R)c->desc.dr;
+    if (std::is_same<R, double>::value && c->desc.dr > 0x1p-100 && c->desc.dr < 0x1p100) {
+        // 1/dr as the sum of two doubles for div_dr: the remainder 1 - rdr_h * dr is exact
+        const double h = 1.0 / c->desc.dr;
+        G.rdr_h = (R)h;
+        G.rdr_l = (R)(std::fma(-h, c->desc.dr, 1.0) / c->desc.dr);
+    }
     for (int a = 0; a < 3; ++a) G.per[a] = c->per[a];
     G.npml = c->desc.npml;
     G.L2 = c->L2;

@@ -60,6 +60,7 @@ template <class R> struct GridArgs {
     Lay L;
     R dt_mu0, dt_eps0;
     R dr;              // used by the exact path's CPML division
+    R rdr_h, rdr_l;    // 1/dr rounded to R, and the rest of it (exact path; 0: divide by dr)
     int per[3];        // periodic axes
     int npml, L2;      // L2 = 2*(npml-1) psi layers per axis
     const R *den_e[3], *den_h[3];

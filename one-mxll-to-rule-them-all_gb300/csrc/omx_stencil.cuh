@@ -20,16 +20,35 @@
 
 namespace omx {
 
-template <class R, bool EXACT>
-__device__ __forceinline__ R psi3(R b, R psi, R c, R d, R dr)
+// x / dr of the exact path, correctly rounded, in four FP64 operations: a quotient good to one ulp
+// from 1/dr held as the sum of two doubles (Brisebarre, Muller and Raina, "Accelerating correctly
+// rounded floating-point division when the divisor is known in advance", IEEE TC 53(8), 2004),
+// then Markstein's correction (IBM J. R&D 34(1), 1990): the remainder x - q dr is exact and
+// q + rem * RN(1/dr) rounds to the quotient.  Arguments whose quotient or remainder could leave
+// the normal range (and zeros, infinities, NaN) take the division.  The FP64 pipe bounds the exact
+// path (2 operations per SM and cycle); with a division per CPML term a 128^3 step took 394 us,
+// with this 326 us.
+__device__ __forceinline__ double div_dr(double x, double dr, double rh, double rl)
 {
-    if (EXACT) return b * psi + c * d / dr;     // bh*psi + ch*(E(i+1)-E(i))/dr
+    const unsigned e = (unsigned)(__double2hiint(x) & 0x7ff00000) - 0x0c800000u;   // 2^-823 <= |x| < 2^824
+    if (e < 0x66f00000u && rh != 0.0) {
+        const double q = __fma_rn(x, rh, __dmul_rn(x, rl));
+        return __fma_rn(__fma_rn(-q, dr, x), rh, q);
+    }
+    if (x == 0.0) return x;   // dr > 0: the sign of zero stays
+    return x / dr;
+}
+
+template <class R, bool EXACT>
+__device__ __forceinline__ R psi3(R b, R psi, R c, R d, const GridArgs<R> &G)
+{
+    if constexpr (EXACT) return b * psi + div_dr(c * d, G.dr, G.rdr_h, G.rdr_l);   // bh*psi + ch*(E(i+1)-E(i))/dr
     return b * psi + c * d;
 }
 template <class R, bool EXACT>
-__device__ __forceinline__ R psi2(R b, R psi, R c, R d, R dr)
+__device__ __forceinline__ R psi2(R b, R psi, R c, R d, const GridArgs<R> &G)
 {
-    if (EXACT) return b * psi + c * (d / dr);   // rot = (E(i+1)-E(i))/dr ; bh*psi + ch*rot
+    if constexpr (EXACT) return b * psi + c * div_dr(d, G.dr, G.rdr_h, G.rdr_l);   // rot = (E(i+1)-E(i))/dr ; bh*psi + ch*rot
     return b * psi + c * d;
 }
 
@@ -145,7 +164,7 @@ __device__ __forceinline__ void h3_tile(const FieldPtrs<R> &F, const GridArgs<R>
     const long long sy = (j == L.ny && G.per[1]) ? (long long)(1 - L.ny) * L.px : (long long)L.px;
     const R dhx = G.den_h[0][i], dhy = G.den_h[1][j];
     const int lx = G.lH[0][i], ly = G.lH[1][j];
-    const R dt_mu0 = G.dt_mu0, dr = G.dr;
+    const R dt_mu0 = G.dt_mu0;
     long long idx = L.off + i + (long long)L.px * j + L.pz * k0;
     R ex_c = Ex[idx], ey_c = Ey[idx];
 #pragma unroll 2   // two planes of loads in flight (the E pass is faster without)
@@ -162,8 +181,8 @@ __device__ __forceinline__ void h3_tile(const FieldPtrs<R> &F, const GridArgs<R>
         if (lx >= 0) {  // mxll_3D_mod.f90:585-620
             const long long p = lx + (long long)G.L2 * ((j - 1) + (long long)L.ny * (k - 1));
             const R b = G.bH[0][i], c = G.cH[0][i];
-            const R v0 = psi3<R, EXACT>(b, G.psiH[0][0][p], c, ez_ip - ez_c, dr);
-            const R v1 = psi3<R, EXACT>(b, G.psiH[0][1][p], c, ey_c - ey_ip, dr);
+            const R v0 = psi3<R, EXACT>(b, G.psiH[0][0][p], c, ez_ip - ez_c, G);
+            const R v1 = psi3<R, EXACT>(b, G.psiH[0][1][p], c, ey_c - ey_ip, G);
             G.psiH[0][0][p] = v0;
             G.psiH[0][1][p] = v1;
             hy = hy + dt_mu0 * v0;
@@ -172,8 +191,8 @@ __device__ __forceinline__ void h3_tile(const FieldPtrs<R> &F, const GridArgs<R>
         if (ly >= 0) {  // :622-657
             const long long p = (i - 1) + (long long)L.nx * (ly + (long long)G.L2 * (k - 1));
             const R b = G.bH[1][j], c = G.cH[1][j];
-            const R v0 = psi3<R, EXACT>(b, G.psiH[1][0][p], c, ez_c - ez_jp, dr);
-            const R v1 = psi3<R, EXACT>(b, G.psiH[1][1][p], c, ex_jp - ex_c, dr);
+            const R v0 = psi3<R, EXACT>(b, G.psiH[1][0][p], c, ez_c - ez_jp, G);
+            const R v1 = psi3<R, EXACT>(b, G.psiH[1][1][p], c, ex_jp - ex_c, G);
             G.psiH[1][0][p] = v0;
             G.psiH[1][1][p] = v1;
             hx = hx + dt_mu0 * v0;
@@ -183,8 +202,8 @@ __device__ __forceinline__ void h3_tile(const FieldPtrs<R> &F, const GridArgs<R>
         if (lz >= 0) {  // :659-694
             const long long p = (i - 1) + (long long)L.nx * ((j - 1) + (long long)L.ny * lz);
             const R b = G.bH[2][k], c = G.cH[2][k];
-            const R v0 = psi3<R, EXACT>(b, G.psiH[2][0][p], c, ey_kp - ey_c, dr);
-            const R v1 = psi3<R, EXACT>(b, G.psiH[2][1][p], c, ex_c - ex_kp, dr);
+            const R v0 = psi3<R, EXACT>(b, G.psiH[2][0][p], c, ey_kp - ey_c, G);
+            const R v1 = psi3<R, EXACT>(b, G.psiH[2][1][p], c, ex_c - ex_kp, G);
             G.psiH[2][0][p] = v0;
             G.psiH[2][1][p] = v1;
             hx = hx + dt_mu0 * v0;
@@ -243,7 +262,7 @@ __device__ __forceinline__ void e3_tile(const FieldPtrs<R> &F, const GridArgs<R>
     const long long my = (j == 1 && G.per[1]) ? (long long)(L.ny - 1) * L.px : -(long long)L.px;
     const R dex = G.den_e[0][i], dey = G.den_e[1][j];
     const int lx = G.lE[0][i], ly = G.lE[1][j];
-    const R dt_eps0 = G.dt_eps0, dr = G.dr;
+    const R dt_eps0 = G.dt_eps0;
     const bool bb_ij = (i >= G.bb0[0] && i <= G.bb1[0] && j >= G.bb0[1] && j <= G.bb1[1]);
     long long idx = L.off + i + (long long)L.px * j + L.pz * k0;
     const long long mz0 = (k0 == 1 && G.per[2]) ? (long long)(L.nz - 1) * L.pz : -L.pz;
@@ -280,8 +299,8 @@ __device__ __forceinline__ void e3_tile(const FieldPtrs<R> &F, const GridArgs<R>
         if (lx >= 0) {  // mxll_3D_mod.f90:817-849
             const long long p = lx + (long long)G.L2 * ((j - 1) + (long long)L.ny * (k - 1));
             const R b = G.bE[0][i], c = G.cE[0][i];
-            const R v0 = psi3<R, EXACT>(b, G.psiE[0][0][p], c, hz_im - hz_c, dr);
-            const R v1 = psi3<R, EXACT>(b, G.psiE[0][1][p], c, hy_c - hy_im, dr);
+            const R v0 = psi3<R, EXACT>(b, G.psiE[0][0][p], c, hz_im - hz_c, G);
+            const R v1 = psi3<R, EXACT>(b, G.psiE[0][1][p], c, hy_c - hy_im, G);
             G.psiE[0][0][p] = v0;
             G.psiE[0][1][p] = v1;
             ey = ey + dt_eps0 * v0;
@@ -290,8 +309,8 @@ __device__ __forceinline__ void e3_tile(const FieldPtrs<R> &F, const GridArgs<R>
         if (ly >= 0) {  // :851-885
             const long long p = (i - 1) + (long long)L.nx * (ly + (long long)G.L2 * (k - 1));
             const R b = G.bE[1][j], c = G.cE[1][j];
-            const R v0 = psi3<R, EXACT>(b, G.psiE[1][0][p], c, hz_c - hz_jm, dr);
-            const R v1 = psi3<R, EXACT>(b, G.psiE[1][1][p], c, hx_jm - hx_c, dr);
+            const R v0 = psi3<R, EXACT>(b, G.psiE[1][0][p], c, hz_c - hz_jm, G);
+            const R v1 = psi3<R, EXACT>(b, G.psiE[1][1][p], c, hx_jm - hx_c, G);
             G.psiE[1][0][p] = v0;
             G.psiE[1][1][p] = v1;
             ex = ex + dt_eps0 * v0;
@@ -301,8 +320,8 @@ __device__ __forceinline__ void e3_tile(const FieldPtrs<R> &F, const GridArgs<R>
         if (lz >= 0) {  // :887-921
             const long long p = (i - 1) + (long long)L.nx * ((j - 1) + (long long)L.ny * lz);
             const R b = G.bE[2][k], c = G.cE[2][k];
-            const R v0 = psi3<R, EXACT>(b, G.psiE[2][0][p], c, hy_km - hy_c, dr);
-            const R v1 = psi3<R, EXACT>(b, G.psiE[2][1][p], c, hx_c - hx_km, dr);
+            const R v0 = psi3<R, EXACT>(b, G.psiE[2][0][p], c, hy_km - hy_c, G);
+            const R v1 = psi3<R, EXACT>(b, G.psiE[2][1][p], c, hx_c - hx_km, G);
             G.psiE[2][0][p] = v0;
             G.psiE[2][1][p] = v1;
             ex = ex + dt_eps0 * v0;
@@ -339,7 +358,7 @@ __global__ void __launch_bounds__(128) k_h2(FieldPtrs<R> F, GridArgs<R> G, int j
     const long long sx = (i == L.nx && G.per[0]) ? (long long)(1 - L.nx) : 1LL;
     const R dhx = G.den_h[0][i];
     const int lx = G.lH[0][i];
-    const R dt_mu0 = G.dt_mu0, dr = G.dr;
+    const R dt_mu0 = G.dt_mu0;
     long long idx = L.off + i + (long long)L.px * j0;
     if (G.mode2d == 1) {
         R *__restrict__ Ez = F.f[2];
@@ -353,14 +372,14 @@ __global__ void __launch_bounds__(128) k_h2(FieldPtrs<R> F, GridArgs<R> G, int j
             R hy = Hy[idx] + dt_mu0 * ((ez_ip - ez_c) * dhx);
             if (lx >= 0) {
                 const long long p = lx + (long long)G.L2 * (j - 1);
-                const R v = psi2<R, EXACT>(G.bH[0][i], G.psiH[0][0][p], G.cH[0][i], ez_ip - ez_c, dr);
+                const R v = psi2<R, EXACT>(G.bH[0][i], G.psiH[0][0][p], G.cH[0][i], ez_ip - ez_c, G);
                 G.psiH[0][0][p] = v;
                 hy = hy + dt_mu0 * v;
             }
             const int ly = G.lH[1][j];
             if (ly >= 0) {
                 const long long p = (i - 1) + (long long)L.nx * ly;
-                const R v = psi2<R, EXACT>(G.bH[1][j], G.psiH[1][0][p], G.cH[1][j], ez_c - ez_jp, dr);
+                const R v = psi2<R, EXACT>(G.bH[1][j], G.psiH[1][0][p], G.cH[1][j], ez_c - ez_jp, G);
                 G.psiH[1][0][p] = v;
                 hx = hx + dt_mu0 * v;
             }
@@ -382,14 +401,14 @@ __global__ void __launch_bounds__(128) k_h2(FieldPtrs<R> F, GridArgs<R> G, int j
             R hz = Hz[idx] + dt_mu0 * ((ey_c - ey_ip) * dhx + (ex_jp - ex_c) * G.den_h[1][j]);
             if (lx >= 0) {
                 const long long p = lx + (long long)G.L2 * (j - 1);
-                const R v = psi2<R, EXACT>(G.bH[0][i], G.psiH[0][0][p], G.cH[0][i], ey_c - ey_ip, dr);
+                const R v = psi2<R, EXACT>(G.bH[0][i], G.psiH[0][0][p], G.cH[0][i], ey_c - ey_ip, G);
                 G.psiH[0][0][p] = v;
                 hz = hz + dt_mu0 * v;
             }
             const int ly = G.lH[1][j];
             if (ly >= 0) {
                 const long long p = (i - 1) + (long long)L.nx * ly;
-                const R v = psi2<R, EXACT>(G.bH[1][j], G.psiH[1][0][p], G.cH[1][j], ex_jp - ex_c, dr);
+                const R v = psi2<R, EXACT>(G.bH[1][j], G.psiH[1][0][p], G.cH[1][j], ex_jp - ex_c, G);
                 G.psiH[1][0][p] = v;
                 hz = hz + dt_mu0 * v;
             }
@@ -417,7 +436,7 @@ __global__ void __launch_bounds__(128) k_e2(FieldPtrs<R> F, GridArgs<R> G, int j
     const long long mx = (i == 1 && G.per[0]) ? (long long)(L.nx - 1) : -1LL;
     const R dex = G.den_e[0][i];
     const int lx = G.lE[0][i];
-    const R dt_eps0 = G.dt_eps0, dr = G.dr;
+    const R dt_eps0 = G.dt_eps0;
     const bool bb_i = (i >= G.bb0[0] && i <= G.bb1[0]);
     long long idx = L.off + i + (long long)L.px * j0;
     const long long my0 = (j0 == 1 && G.per[1]) ? (long long)(L.ny - 1) * L.px : -(long long)L.px;
@@ -438,14 +457,14 @@ __global__ void __launch_bounds__(128) k_e2(FieldPtrs<R> F, GridArgs<R> G, int j
             }
             if (lx >= 0) {
                 const long long p = lx + (long long)G.L2 * (j - 1);
-                const R v = psi2<R, EXACT>(G.bE[0][i], G.psiE[0][0][p], G.cE[0][i], hy_c - hy_im, dr);
+                const R v = psi2<R, EXACT>(G.bE[0][i], G.psiE[0][0][p], G.cE[0][i], hy_c - hy_im, G);
                 G.psiE[0][0][p] = v;
                 ez = ez + dt_eps0 * v;
             }
             const int ly = G.lE[1][j];
             if (ly >= 0) {
                 const long long p = (i - 1) + (long long)L.nx * ly;
-                const R v = psi2<R, EXACT>(G.bE[1][j], G.psiE[1][0][p], G.cE[1][j], hx_jm - hx_c, dr);
+                const R v = psi2<R, EXACT>(G.bE[1][j], G.psiE[1][0][p], G.cE[1][j], hx_jm - hx_c, G);
                 G.psiE[1][0][p] = v;
                 ez = ez + dt_eps0 * v;
             }
@@ -472,14 +491,14 @@ __global__ void __launch_bounds__(128) k_e2(FieldPtrs<R> F, GridArgs<R> G, int j
             }
             if (lx >= 0) {
                 const long long p = lx + (long long)G.L2 * (j - 1);
-                const R v = psi2<R, EXACT>(G.bE[0][i], G.psiE[0][0][p], G.cE[0][i], hz_im - hz_c, dr);
+                const R v = psi2<R, EXACT>(G.bE[0][i], G.psiE[0][0][p], G.cE[0][i], hz_im - hz_c, G);
                 G.psiE[0][0][p] = v;
                 ey = ey + dt_eps0 * v;
             }
             const int ly = G.lE[1][j];
             if (ly >= 0) {
                 const long long p = (i - 1) + (long long)L.nx * ly;
-                const R v = psi2<R, EXACT>(G.bE[1][j], G.psiE[1][0][p], G.cE[1][j], hz_c - hz_jm, dr);
+                const R v = psi2<R, EXACT>(G.bE[1][j], G.psiE[1][0][p], G.cE[1][j], hz_c - hz_jm, G);
                 G.psiE[1][0][p] = v;
                 ex = ex + dt_eps0 * v;
             }
@@ -506,7 +525,7 @@ __global__ void k_h1(FieldPtrs<R> F, GridArgs<R> G)
     R hy = Hy[idx] + G.dt_mu0 * d * G.den_h[0][i];
     const int l = G.lH[0][i];
     if (l >= 0) {
-        const R v = psi3<R, EXACT>(G.bH[0][i], G.psiH[0][0][l], G.cH[0][i], d, G.dr);
+        const R v = psi3<R, EXACT>(G.bH[0][i], G.psiH[0][0][l], G.cH[0][i], d, G);
         G.psiH[0][0][l] = v;
         hy = hy + G.dt_mu0 * v;
     }
@@ -533,7 +552,7 @@ __global__ void k_e1(FieldPtrs<R> F, GridArgs<R> G)
     }
     const int l = G.lE[0][i];
     if (l >= 0) {
-        const R v = psi2<R, EXACT>(G.bE[0][i], G.psiE[0][0][l], G.cE[0][i], d, G.dr);
+        const R v = psi2<R, EXACT>(G.bE[0][i], G.psiE[0][0][l], G.cE[0][i], d, G);
         G.psiE[0][0][l] = v;
         ex = ex + G.dt_eps0 * v;
     }
@@ -548,7 +567,7 @@ __global__ void k_e1(FieldPtrs<R> F, GridArgs<R> G)
 // memory trips was the whole pass there).  Measured, us per step at marches of 1, 2, 4, 8, 16 (32):
 // 3D FP32 32^3 11.5, 12.6, 16.7, 23.7, 37.2; 101 x 90 x 157 34.0, 28.0, 26.5, 28.3, 29.2;
 // 200 x 180 x 220 200, 158, 143, 141, 144; 3D FP64 (compute bound, so the reads it saves count
-// less) 64^3 91, 97, 111, 123, 150, 200^3 1253, 1244, 1236, 1257, 1277; 2D FP32 TMz 243 x 161 22.9,
+// less) 64^3 70, 76, 88, 92, 104, 200^3 1086, 1055, 1048, 1065, 1073; 2D FP32 TMz 243 x 161 22.9,
 // 23.9, 25.0, 27.7, 31.9 (42.1), TEz 1531 x 1147 31.7, 27.1, 25.6, 29.4, 32.3 (52.2), 4096^2 288,
 // 219, 192, 180, 184 (196).
 inline int march_rule(long long tiles, int n, int most, int want)

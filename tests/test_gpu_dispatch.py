@@ -53,7 +53,9 @@ FIELDS_OF = {(1, 1): [1, 5], (2, 1): [3, 4, 5], (2, 2): [1, 2, 6], (3, 1): [1, 2
     (3, (33, 29, 26), 4, (3, 3, 3), 1),
     (3, (31, 17, 65), 5, (2, 3, 3), 1),
 ])
-@pytest.mark.parametrize("amp,dr", [(1.0, 37.794522518155646)])
+# amplitudes where quotients by dr are ordinary, and down to where they or their remainders leave
+# the normal range; spacings with short and with full mantissas
+@pytest.mark.parametrize("amp,dr", [(1.0, 37.794522518155646), (1e-250, 19.0), (3e-306, 0.7), (1e280, 1.0 / 3.0)])
 def test_fp64_passes_bit_identical(orc, dims, n, npml, bnd, mode, amp, dr):
     gpu, cpu, dt = seeded_pair(orc, dims, n, npml, bnd, dr, mode, amp, sum(n))
     advance(gpu, cpu, dt, 5)
