@@ -167,7 +167,7 @@ __device__ __forceinline__ void h3_tile(const FieldPtrs<R> &F, const GridArgs<R>
     const R dt_mu0 = G.dt_mu0;
     long long idx = L.off + i + (long long)L.px * j + L.pz * k0;
     R ex_c = Ex[idx], ey_c = Ey[idx];
-#pragma unroll 2   // two planes of loads in flight (the E pass is faster without)
+#pragma unroll (EXACT ? 1 : 2)   // FP32: two planes of loads in flight (the E pass is faster without)
     for (int k = k0; k <= k1; ++k, idx += L.pz) {
         const long long sz = (k == L.nz && G.per[2]) ? (long long)(1 - L.nz) * L.pz : L.pz;
         const R ez_c = Ez[idx], ez_jp = Ez[idx + sy], ez_ip = Ez[idx + sx];
@@ -234,9 +234,10 @@ __device__ __forceinline__ void h3_tile(const FieldPtrs<R> &F, const GridArgs<R>
 }
 
 // FP32: at most 48 registers, 10 blocks per SM (measured 8 % faster than the unbounded 64
-// registers at 512^3; the E pass takes its own bound, 9 blocks)
+// registers at 512^3; the E pass takes its own bound, 9 blocks).  FP64: 5 blocks per SM, the march
+// not unrolled (133 -> 96 registers: 128^3 310 -> 293 us per step)
 template <class R, bool EXACT>
-__global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 10 : 1)) k_h3(FieldPtrs<R> F, GridArgs<R> G, int kch)
+__global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 10 : 5)) k_h3(FieldPtrs<R> F, GridArgs<R> G, int kch)
 {
     h3_tile<R, EXACT>(F, G, kch, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -338,7 +339,7 @@ __device__ __forceinline__ void e3_tile(const FieldPtrs<R> &F, const GridArgs<R>
 // FP32: at most 56 registers, 9 blocks per SM (4 % faster than the unbounded 64 registers at
 // 512^3 and 256^3)
 template <class R, bool EXACT>
-__global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 9 : 1)) k_e3(FieldPtrs<R> F, GridArgs<R> G, int kch)
+__global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 9 : 5)) k_e3(FieldPtrs<R> F, GridArgs<R> G, int kch)
 {
     e3_tile<R, EXACT>(F, G, kch, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -351,9 +352,9 @@ __global__ void __launch_bounds__(128) k_h2(FieldPtrs<R> F, GridArgs<R> G, int j
 {
     const Lay L = G.L;
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (G.step_inc && i == 1 && blockIdx.y == 0) *G.step_inc += 1;   // device-loop step counter
-    if (i > L.nx) return;
-    const int j0 = 1 + blockIdx.y * jch;
+    const int j0 = 1 + (blockIdx.y * blockDim.y + threadIdx.y) * jch;
+    if (G.step_inc && i == 1 && j0 == 1) *G.step_inc += 1;   // device-loop step counter
+    if (i > L.nx || j0 > L.ny) return;
     const int j1 = min(L.ny, j0 + jch - 1);
     const long long sx = (i == L.nx && G.per[0]) ? (long long)(1 - L.nx) : 1LL;
     const R dhx = G.den_h[0][i];
@@ -430,8 +431,8 @@ __global__ void __launch_bounds__(128) k_e2(FieldPtrs<R> F, GridArgs<R> G, int j
 {
     const Lay L = G.L;
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > L.nx) return;
-    const int j0 = 1 + blockIdx.y * jch;
+    const int j0 = 1 + (blockIdx.y * blockDim.y + threadIdx.y) * jch;
+    if (i > L.nx || j0 > L.ny) return;
     const int j1 = min(L.ny, j0 + jch - 1);
     const long long mx = (i == 1 && G.per[0]) ? (long long)(L.nx - 1) : -1LL;
     const R dex = G.den_e[0][i];
@@ -572,17 +573,30 @@ __global__ void k_e1(FieldPtrs<R> F, GridArgs<R> G)
 // 219, 192, 180, 184 (196).
 inline int march_rule(long long tiles, int n, int most, int want)
 {
+    constexpr int GRID_YZ = 65535;   // blocks a launch takes along y or z
     int m = most;
-    while (m > 1 && tiles * ((n + m - 1) / m) < 152LL * want) m /= 2;
+    while ((n + m - 1) / m > GRID_YZ) m *= 2;
+    while (m > 1 && tiles * ((n + m - 1) / m) < 152LL * want && (n + m / 2 - 1) / (m / 2) <= GRID_YZ) m /= 2;
     return m;
+}
+// Threads of a block along x and y (128 in all).  FP32: whole 128-byte rows of 32 cells a warp.
+// FP64: 8 x 4 cells a warp.  The FP64 pipe bounds that path and charges a warp for all its lanes, so
+// a warp 32 cells wide pays for the CPML terms of an x slab (npml - 1 cells) in every row it touches,
+// and for the cells past a ragged edge; 8 doubles are still two whole sectors.  88 x 76 x 67 with an
+// 8-cell CPML: 124 -> 103 us per step, 200^3 periodic in x and y 805 -> 709 (16 x 8 threads: 115, 4 x 32: 113).
+struct BlockXY { int x, y; };
+template <class R> constexpr BlockXY block_xy(int dims)
+{
+    return sizeof(R) == 8 ? BlockXY{8, 16} : (dims == 3 ? BlockXY{32, 4} : BlockXY{128, 1});
 }
 template <class R> inline int march_of(const GridArgs<R> &G)
 {
     const Lay &L = G.L;
     if (G.march > 0) return G.march;
     const bool f4 = sizeof(R) == 4;
-    if (L.dims == 3) return march_rule((long long)((L.nx + 31) / 32) * ((L.ny + 3) / 4), L.nz, 16, f4 ? 24 : 64);
-    return march_rule((L.nx + 127) / 128, L.ny, 8, 16);
+    const BlockXY b = block_xy<R>(L.dims);
+    if (L.dims == 3) return march_rule((long long)((L.nx + b.x - 1) / b.x) * ((L.ny + b.y - 1) / b.y), L.nz, 16, f4 ? 24 : 64);
+    return march_rule((L.nx + b.x - 1) / b.x, (L.ny + b.y - 1) / b.y, 8, 16);
 }
 
 template <class R, bool EXACT>
@@ -592,11 +606,13 @@ void launch_h_impl(const FieldPtrs<R> &F, const GridArgs<R> &G, void *stream)
     const Lay &L = G.L;
     if (L.dims == 3) {
         const int m = march_of(G);
-        dim3 b(32, 4, 1), g((L.nx + 31) / 32, (L.ny + 3) / 4, (L.nz + m - 1) / m);
+        constexpr BlockXY t = block_xy<R>(3);
+        const dim3 b(t.x, t.y, 1), g((L.nx + t.x - 1) / t.x, (L.ny + t.y - 1) / t.y, (L.nz + m - 1) / m);
         k_h3<R, EXACT><<<g, b, 0, s>>>(F, G, m);
     } else if (L.dims == 2) {
         const int m = march_of(G);
-        dim3 b(128, 1, 1), g((L.nx + 127) / 128, (L.ny + m - 1) / m, 1);
+        constexpr BlockXY t = block_xy<R>(2);
+        const dim3 b(t.x, t.y, 1), g((L.nx + t.x - 1) / t.x, (L.ny + t.y * m - 1) / (t.y * m), 1);
         k_h2<R, EXACT><<<g, b, 0, s>>>(F, G, m);
     } else {
         k_h1<R, EXACT><<<(L.nx + 127) / 128, 128, 0, s>>>(F, G);
@@ -611,11 +627,13 @@ void launch_e_impl(const FieldPtrs<R> &F, const GridArgs<R> &G, void *stream)
     if (G.ade_n > 0) k_ade<R><<<(G.ade_n + 127) / 128, 128, 0, s>>>(F, G);
     if (L.dims == 3) {
         const int m = march_of(G);
-        dim3 b(32, 4, 1), g((L.nx + 31) / 32, (L.ny + 3) / 4, (L.nz + m - 1) / m);
+        constexpr BlockXY t = block_xy<R>(3);
+        const dim3 b(t.x, t.y, 1), g((L.nx + t.x - 1) / t.x, (L.ny + t.y - 1) / t.y, (L.nz + m - 1) / m);
         k_e3<R, EXACT><<<g, b, 0, s>>>(F, G, m);
     } else if (L.dims == 2) {
         const int m = march_of(G);
-        dim3 b(128, 1, 1), g((L.nx + 127) / 128, (L.ny + m - 1) / m, 1);
+        constexpr BlockXY t = block_xy<R>(2);
+        const dim3 b(t.x, t.y, 1), g((L.nx + t.x - 1) / t.x, (L.ny + t.y * m - 1) / (t.y * m), 1);
         k_e2<R, EXACT><<<g, b, 0, s>>>(F, G, m);
     } else {
         k_e1<R, EXACT><<<(L.nx + 127) / 128, 128, 0, s>>>(F, G);

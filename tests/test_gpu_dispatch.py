@@ -43,14 +43,17 @@ def advance(gpu, cpu, dt, steps, calls=False):
 FIELDS_OF = {(1, 1): [1, 5], (2, 1): [3, 4, 5], (2, 2): [1, 2, 6], (3, 1): [1, 2, 3, 4, 5, 6]}
 
 
-# sizes at the edges of the blocks (32 x 4 columns, 128 cells), of the marches (1..16 planes, 1..8 rows)
+# sizes at the edges of the blocks (8 x 16 cells), of the marches (1..16 planes, 1..8 rows)
 # and of the CPML slabs
 @pytest.mark.parametrize("dims,n,npml,bnd,mode", [
     (1, (64,), 6, (3, 1, 1), 1),
     (2, (129, 33), 5, (3, 3, 1), 1),
+    (2, (17, 9), 3, (2, 3, 1), 2),
     (2, (127, 70), 5, (2, 3, 1), 2),
     (2, (640, 641), 6, (3, 2, 1), 2),
+    (2, (8, 70001), 3, (2, 3, 1), 1),        # more rows than a launch takes blocks along y
     (3, (33, 29, 26), 4, (3, 3, 3), 1),
+    (3, (7, 16, 9), 3, (2, 3, 1), 1),
     (3, (31, 17, 65), 5, (2, 3, 3), 1),
 ])
 # amplitudes where quotients by dr are ordinary, and down to where they or their remainders leave
@@ -66,3 +69,13 @@ def test_fp64_passes_bit_identical(orc, dims, n, npml, bnd, mode, amp, dr):
         assert np.array_equal(a[own], b[own])
         assert amp < 1e-300 or np.max(np.abs(b[own])) > 0
     gpu.kill()
+
+
+def test_more_planes_than_blocks_along_z(orc):
+    """A grid with more planes (3D) or FP32 rows (2D) than a launch takes blocks along z or y."""
+    gpu, cpu, dt = seeded_pair(orc, 3, (4, 3, 66001), 2, (1, 1, 1), 19.0, omx.TMZ, 1.0, 3)
+    advance(gpu, cpu, dt, 2)
+    assert np.array_equal(gpu.read_field(1), cpu.read_field(1))
+    gpu, cpu, dt = seeded_pair(orc, 2, (9, 66003), 3, (1, 3, 1), 19.0, omx.TEZ, 1.0, 4, "fp32")
+    advance(gpu, cpu, dt, 2)
+    assert np.max(np.abs(gpu.read_field(6) - cpu.read_field(6))) < 1e-5 * np.max(np.abs(cpu.read_field(6)))
