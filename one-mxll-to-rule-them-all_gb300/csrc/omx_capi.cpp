@@ -13,10 +13,14 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <tuple>
 #include <type_traits>
 #include <unordered_map>
 #include <vector>
+
+#include <unistd.h>
 
 #include "../../include/omx_gpu.h"
 #include "omx_host.h"
@@ -119,6 +123,7 @@ struct GroupRec {
     // field words, and the current's points, sorted by cell too, read neighbouring dPt_dt rows):
     // emitter order[d] of the caller's list is device row d, and device row inv[e] is emitter e
     std::vector<int> order, inv;
+    DevBuf<int> order_d;   // order on the device (omx_qgroup_read)
     DevBuf<int> ci, cj, ck;
     DevBuf<double> par, rates, rho, E, dipole, dPdt;
     DevBuf<int> win;
@@ -288,6 +293,7 @@ struct omx_ctx {
     long long launches = 0;
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     DevBuf<float> flushbuf;
+    DevBuf<double> host_stage;   // dense FP64 rows on their way to or from the host (at most HOST_STAGE doubles, or one row)
     // FP32 fused 2D TMz step (ping-pong): second field / H-psi buffer set and the parity
     DevBuf<float> ff2[6];
     DevBuf<float> psiH2[3][2];
@@ -1956,41 +1962,95 @@ template <class R> int autotune_impl(omx_ctx *c, int reps)
     return pick;
 }
 
-template <class R> void read_field_impl(omx_ctx *c, int field, double *host)
+// Dense FP64 rows go to the host through a device buffer of this size: a kernel unpitches and
+// converts, and each chunk is one copy straight into the caller's pages.  (A copy of the padded FP32
+// array and a host loop over its cells took 40.6 ms for a 4096^2 component; this 2.6 ms.)
+constexpr size_t HOST_STAGE = (size_t)1 << 21;   // doubles (16 MB)
+
+double *host_stage(omx_ctx *c, size_t need)
+{
+    if (c->host_stage.n < need) c->host_stage.alloc(need, false);
+    return c->host_stage.p;
+}
+
+// Touch the pages of a large output from a few threads: fresh pages of the caller are cleared by
+// the kernel on first touch, which one thread does at a sixth of the copy's rate (134 MB: 5.2 ms with
+// one thread, 1.7 ms with four; the copy itself 0.8 ms).  Every byte is overwritten by the copy.
+void touch_pages(void *p, size_t bytes)
+{
+    if (bytes < ((size_t)8 << 20)) return;
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE), parts = 4;
+    auto touch = [=](size_t a, size_t b) {
+        for (size_t q = a; q < b; q += page) static_cast<volatile char *>(p)[q] = 0;
+    };
+    std::vector<std::thread> th;
+    size_t done = 0;
+    try {
+        for (size_t t = 0; t + 1 < parts; ++t) {
+            const size_t a = bytes / parts * t / page * page, b = bytes / parts * (t + 1) / page * page;
+            th.emplace_back(touch, a, b);
+            done = b;
+        }
+    } catch (const std::system_error &) {
+        // no more threads: this one touches the rest
+    }
+    touch(done, bytes);
+    for (auto &t : th) t.join();
+}
+
+PackArgs pack_args(const omx_ctx *c, int field, long long &rows)
 {
     int lo[3], hi[3];
     req(bounds_of(c, field, lo, hi), "field not present in this grid/mode");
-    const int q = field_code_to_index(field);
-    std::vector<R> tmp(c->felems);
+    PackArgs P;
+    P.L = c->L;
+    for (int a = 0; a < 3; ++a) {
+        P.lo[a] = lo[a];
+        // E ghost planes n+1 of periodic axes are closed by index remapping on the device (not
+        // stored); H ghost planes 0 hold the wrapped values as in the reference
+        P.zero[a] = (field <= OMX_EZ_FIELD && a < c->dims && c->per[a]) ? c->n[a] + 1 : -1;
+    }
+    P.ni = hi[0] - lo[0] + 1;
+    P.nj = hi[1] - lo[1] + 1;
+    rows = (long long)P.nj * (hi[2] - lo[2] + 1);
+    return P;
+}
+
+template <class R> void read_field_impl(omx_ctx *c, int field, double *host)
+{
+    long long rows;
+    const PackArgs P = pack_args(c, field, rows);
+    touch_pages(host, (size_t)rows * P.ni * sizeof(double));
     sync_checked(c, "sync");
-    ck(cudaMemcpy(tmp.data(), field_ptrs<R>(c).f[q], c->felems * sizeof(R), cudaMemcpyDeviceToHost), "read field");
-    long long o = 0;
-    for (int k = lo[2]; k <= hi[2]; ++k)
-        for (int j = lo[1]; j <= hi[1]; ++j)
-            for (int i = lo[0]; i <= hi[0]; ++i) {
-                // E ghost planes n+1 of periodic axes are closed by index remapping on the device
-                // (not stored); H ghost planes 0 hold the wrapped values as in the reference
-                bool ghost_periodic = false;
-                const int ijk[3] = {i, j, k};
-                for (int a = 0; a < c->dims; ++a)
-                    if (field <= OMX_EZ_FIELD && c->per[a] && ijk[a] == c->n[a] + 1) ghost_periodic = true;
-                host[o++] = ghost_periodic ? 0.0 : (double)tmp[(size_t)eindex(c, i, j, k)];
-            }
+    const long long per = std::max<long long>(1, (long long)HOST_STAGE / P.ni);
+    double *buf = host_stage(c, (size_t)std::min(per, rows) * P.ni);
+    const R *f = field_ptrs<R>(c).f[field_code_to_index(field)];
+    for (long long r = 0; r < rows; r += per) {
+        const long long m = std::min(per, rows - r);
+        launch_pack<R>(f, P, r, m, buf, c->stream);
+        ck(cudaPeekAtLastError(), "read field");
+        ck(cudaMemcpyAsync(host + r * P.ni, buf, (size_t)m * P.ni * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
+           "read field");
+    }
+    ck(cudaStreamSynchronize(c->stream), "read field");
 }
 
 template <class R> void write_field_impl(omx_ctx *c, int field, const double *host)
 {
-    int lo[3], hi[3];
-    req(bounds_of(c, field, lo, hi), "field not present in this grid/mode");
-    const int q = field_code_to_index(field);
-    std::vector<R> tmp(c->felems);
+    long long rows;
+    const PackArgs P = pack_args(c, field, rows);
     sync_checked(c, "sync");
-    ck(cudaMemcpy(tmp.data(), field_ptrs<R>(c).f[q], c->felems * sizeof(R), cudaMemcpyDeviceToHost), "read field");
-    long long o = 0;
-    for (int k = lo[2]; k <= hi[2]; ++k)
-        for (int j = lo[1]; j <= hi[1]; ++j)
-            for (int i = lo[0]; i <= hi[0]; ++i) tmp[(size_t)eindex(c, i, j, k)] = (R)host[o++];
-    h2d(field_ptrs<R>(c).f[q], tmp.data(), c->felems * sizeof(R), "write field");
+    const long long per = std::max<long long>(1, (long long)HOST_STAGE / P.ni);
+    double *buf = host_stage(c, (size_t)std::min(per, rows) * P.ni);
+    R *f = field_ptrs<R>(c).f[field_code_to_index(field)];
+    for (long long r = 0; r < rows; r += per) {
+        const long long m = std::min(per, rows - r);
+        ck(cudaMemcpyAsync(buf, host + r * P.ni, (size_t)m * P.ni * sizeof(double), cudaMemcpyHostToDevice, c->stream),
+           "write field");
+        launch_unpack<R>(f, P, r, m, buf, c->stream);
+        ck(cudaPeekAtLastError(), "write field");
+    }
+    ck(cudaStreamSynchronize(c->stream), "write field");
 }
 
 }  // namespace
@@ -2552,6 +2612,7 @@ int omx_qgroup_create(omx_ctx *c, const omx_qgroup_desc *d, const int32_t *cell,
         return cell_key(c, ci[a], cj[a], ckk[a]) < cell_key(c, ci[b], cj[b], ckk[b]);
     });
     for (int r = 0; r < n; ++r) G->inv[G->order[r]] = r;
+    G->order_d.upload(G->order);
     std::vector<int> di(n), dj(n), dk(n);
     std::vector<double> par((size_t)n * G->npar);
     for (int r = 0; r < n; ++r) {
@@ -2714,19 +2775,20 @@ int omx_qgroup_read(omx_ctx *c, int gid, double *dipole, double *dPdt, double *e
     GroupRec &g = *c->groups[gid];
     ck(cudaStreamSynchronize(c->stream), "sync");
     const size_t n = (size_t)g.d.n_systems;
-    // device rows back into the caller's emitter order
-    std::vector<double> tmp;
+    // device rows back into the caller's emitter order, on the device
+    double *buf = host_stage(c, n * (size_t)std::max(3, g.nst));
     auto get = [&](double *out, const double *dev, int w) {
         if (!out) return;
-        tmp.resize(n * w);
-        ck(cudaMemcpy(tmp.data(), dev, n * w * sizeof(double), cudaMemcpyDeviceToHost), "read");
-        for (size_t r = 0; r < n; ++r)
-            std::copy(tmp.begin() + r * w, tmp.begin() + (r + 1) * w, out + (size_t)g.order[r] * w);
+        launch_scatter_rows(dev, g.order_d.p, (long long)n, w, buf, c->stream);
+        ck(cudaPeekAtLastError(), "read");
+        ck(cudaMemcpyAsync(out, buf, n * w * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "read");
+        ck(cudaStreamSynchronize(c->stream), "read");
     };
     get(dipole, g.dipole.p, 3);
     get(dPdt, g.dPdt.p, 3);
     get(efield, g.E.p, 3);
     get(rho, g.rho.p, g.nst);
+    if (c->host_stage.n > HOST_STAGE) c->host_stage.release();
     OMX_API_END(c)
 }
 

@@ -174,6 +174,17 @@ template <class R> void launch_emit(const FieldPtrs<R> &F, const Lay &L, const E
 void launch_scatter(const JState &J, const ScatArgs &S, StepParam move, void *stream);
 template <class R> void launch_sample(const FieldPtrs<R> &F, const DetArgs &D, StepParam slot, StepParam time, void *stream);
 void launch_step_advance(int *step, void *stream);
+// Rows row0 .. row0 + rows - 1 (row = (j - lo[1]) + nj * (k - lo[2]), ni values each) of a field over
+// the reference's bounds, between the padded device array and a dense FP64 buffer in Fortran order.
+// zero: index n + 1 of an axis whose plane reads back as zero (an E ghost of a periodic axis), else -1.
+struct PackArgs {
+    Lay L;
+    int lo[3], ni, nj, zero[3];
+};
+template <class R> void launch_pack(const R *field, const PackArgs &P, long long row0, long long rows, double *out, void *stream);
+template <class R> void launch_unpack(R *field, const PackArgs &P, long long row0, long long rows, const double *in, void *stream);
+// out[order[r] * w + q] = in[r * w + q]: device rows back into the caller's order
+void launch_scatter_rows(const double *in, const int *order, long long n, int w, double *out, void *stream);
 // FP32 fused TMz step: reads the in buffers, writes the out buffers (see omx_fused2d.cuh)
 struct Fused2Args {
     const float *ez_in, *hx_in, *hy_in;

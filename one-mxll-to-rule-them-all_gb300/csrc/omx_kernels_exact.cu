@@ -74,6 +74,22 @@ template <class R> void launch_sample(const FieldPtrs<R> &F, const DetArgs &D, S
     const int n = D.n > 0 ? D.n : 1;
     k_sample<R><<<(n + 127) / 128, 128, 0, (cudaStream_t)s>>>(F, D, slot, time);
 }
+static dim3 pack_grid(const PackArgs &P, long long rows)
+{
+    return dim3((unsigned)((P.ni + 127) / 128), (unsigned)(rows < 32768 ? rows : 32768));
+}
+template <class R> void launch_pack(const R *f, const PackArgs &P, long long row0, long long rows, double *out, void *s)
+{
+    k_pack<R, true><<<pack_grid(P, rows), 128, 0, (cudaStream_t)s>>>(const_cast<R *>(f), P, row0, rows, out);
+}
+template <class R> void launch_unpack(R *f, const PackArgs &P, long long row0, long long rows, const double *in, void *s)
+{
+    k_pack<R, false><<<pack_grid(P, rows), 128, 0, (cudaStream_t)s>>>(f, P, row0, rows, const_cast<double *>(in));
+}
+void launch_scatter_rows(const double *in, const int *order, long long n, int w, double *out, void *s)
+{
+    if (n > 0) k_scatter_rows<<<(unsigned)((n * w + 255) / 256), 256, 0, (cudaStream_t)s>>>(in, order, n, w, out);
+}
 void launch_step_advance(int *step, void *s)
 {
     k_step_advance<<<1, 32, 0, (cudaStream_t)s>>>(step);
@@ -125,6 +141,8 @@ void launch_flush(float *buf, long long n, void *s)
                                    StepParam, double, void *);                                           \
     template void launch_emit<R>(const FieldPtrs<R> &, const Lay &, const EmitArgs &, StepParam, void *); \
     template void launch_sample<R>(const FieldPtrs<R> &, const DetArgs &, StepParam, StepParam, void *); \
+    template void launch_pack<R>(const R *, const PackArgs &, long long, long long, double *, void *);    \
+    template void launch_unpack<R>(R *, const PackArgs &, long long, long long, const double *, void *);  \
     template void launch_src_batch<R>(const BatchSrc<R> *, int, long long, void *);                      \
     template void launch_sample_batch<R>(const BatchDet<R> *, int, long long, void *);
 OMX_INST(float)

@@ -171,6 +171,34 @@ __global__ void k_sample(FieldPtrs<R> F, DetArgs D, StepParam slot_p, StepParam 
     sample_point<R>(F, D, slot_p, time_p, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
+// ---- field and emitter reads: dense FP64 rows for the host ----------------------------------------
+// One thread per value, rows over blockIdx.y; both directions move each value once (a 4096^2 FP32
+// component: 67 MB in, 134 MB out), far below the host copy beside them.
+template <class R, bool OUT>
+__global__ void k_pack(R *field, PackArgs P, long long row0, long long rows, double *buf)
+{
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= P.ni) return;
+    const int i = P.lo[0] + x;
+    for (long long r = blockIdx.y; r < rows; r += gridDim.y) {
+        const long long row = row0 + r;
+        const int j = P.lo[1] + (int)(row % P.nj), k = P.lo[2] + (int)(row / P.nj);
+        const long long idx = P.L.off + i + (long long)P.L.px * j + P.L.pz * k;
+        if (OUT) {
+            const bool ghost = i == P.zero[0] || j == P.zero[1] || k == P.zero[2];
+            buf[r * P.ni + x] = ghost ? 0.0 : (double)field[idx];
+        } else {
+            field[idx] = (R)buf[r * P.ni + x];
+        }
+    }
+}
+
+__global__ void k_scatter_rows(const double *in, const int *order, long long n, int w, double *out)
+{
+    const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (q < n * w) out[(long long)order[q / w] * w + q % w] = in[q];
+}
+
 __global__ void k_step_advance(int *step)
 {
     if (threadIdx.x == 0 && blockIdx.x == 0) *step = *step + 1;

@@ -79,3 +79,25 @@ def test_more_planes_than_blocks_along_z(orc):
     gpu, cpu, dt = seeded_pair(orc, 2, (9, 66003), 3, (1, 3, 1), 19.0, omx.TEZ, 1.0, 4, "fp32")
     advance(gpu, cpu, dt, 2)
     assert np.max(np.abs(gpu.read_field(6) - cpu.read_field(6))) < 1e-5 * np.max(np.abs(cpu.read_field(6)))
+
+
+@pytest.mark.parametrize("dims,n,bnd,mode,field,precision", [
+    (1, (2_200_003,), (3, 1, 1), 1, 1, "fp64"),           # one row longer than a chunk of the staging buffer
+    (2, (1701, 1301), (2, 3, 1), 1, 3, "fp32"),           # two chunks, the second partial; periodic ghost column
+    (2, (5, 3), (1, 1, 1), 2, 6, "fp64"),
+    (3, (131, 129, 130), (2, 2, 2), 1, 2, "fp32"),
+    (3, (131, 129, 130), (3, 3, 3), 1, 5, "fp64"),
+])
+def test_field_round_trip(dims, n, bnd, mode, field, precision):
+    """omx_write_field then omx_read_field returns the values, the E ghosts of periodic axes as zero."""
+    g = omx.TMxll(dims, n, 4, bnd, 0.07, 19.0, mode=mode, precision=precision)
+    lo, hi = g.field_bounds(field)
+    shape = [h - b + 1 for b, h in zip(lo, hi)]
+    a = np.asfortranarray(np.random.default_rng(1).standard_normal(shape).astype(np.float32).astype(np.float64))
+    g.write_field(field, a)
+    want = a.copy(order="F")
+    for x in range(dims):
+        if field <= 3 and bnd[x] == 2 and hi[x] == n[x] + 1:
+            want[tuple(-1 if y == x else slice(None) for y in range(3))] = 0.0
+    assert np.array_equal(g.read_field(field), want)
+    g.kill()
