@@ -58,9 +58,23 @@ template <class R> void launch_inject(const FieldPtrs<R> &F, const JState &J, co
     if (I.n <= 0) return;
     k_inject<R><<<(I.n + 127) / 128, 128, 0, (cudaStream_t)s>>>(F, J, I, t, ts, dt_eps0);
 }
+// Emitters up to which a group is stepped with one lane per state word (k_emit_lanes) instead of one
+// thread per emitter: few emitters wait on one warp's chain of FP64 instructions, which the lanes
+// shorten, many on the FP64 pipe, for which the lanes' extra instructions count.  Measured, us for the
+// emitter step and scatter, a thread / lanes per emitter: 2-level 300 12.6 / 10.5, 2000 13.7 / 10.5,
+// 10000 15.3 / 13.7, 20000 17.4 / 18.7; 3-level 300 20.9 / 12.7, 2000 21.8 / 12.7, 5000 21.9 / 17.7,
+// 10000 22.9 / 22.9, 20000 29.0 / 36.3.
+constexpr int EMIT_LANES_MOST[2] = {8192, 6144};   // 2-level, 3-level
 template <class R> void launch_emit(const FieldPtrs<R> &F, const Lay &L, const EmitArgs &A, StepParam move, void *s)
 {
     if (A.n <= 0) return;
+    if (A.n <= EMIT_LANES_MOST[A.model == 1 ? 0 : 1]) {
+        const long long t = (long long)A.n * (A.model == 1 ? 4 : 8);
+        const unsigned nb = (unsigned)((t + 63) / 64);
+        if (A.model == 1) k_emit_lanes<R, 4><<<nb, 64, 0, (cudaStream_t)s>>>(F, L, A, move);
+        else k_emit_lanes<R, 8><<<nb, 64, 0, (cudaStream_t)s>>>(F, L, A, move);
+        return;
+    }
     // one warp per block: the FP64 work of a few thousand emitters spreads over every SM
     k_emit<R><<<(A.n + 31) / 32, 32, 0, (cudaStream_t)s>>>(F, L, A, move);
 }

@@ -115,6 +115,58 @@ __global__ void k_emit(FieldPtrs<R> F, Lay L, EmitArgs A, StepParam move_p)
     }
 }
 
+// k_emit with LANES lanes per emitter (rk4_lane): the same arithmetic per word, dipole axis and
+// field component.  Lane a of the group gathers component a and writes axis a.
+template <class R, int LANES>
+__global__ void __launch_bounds__(64) k_emit_lanes(FieldPtrs<R> F, Lay L, EmitArgs A, StepParam move_p)
+{
+    constexpr unsigned FULL = 0xffffffffu;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int l = t % LANES, n0 = t / LANES;
+    if (sp_get(move_p) == 0.0) return;
+    if (A.only_if && *A.only_if == 0) return;
+    const bool live = n0 < A.n;
+    const int n = live ? n0 : A.n - 1;            // lanes past the end follow the last emitter, without writes
+    const long long c = L.off + A.ci[n] + (long long)L.px * A.cj[n] + L.pz * A.ck[n];
+    double E = 0.0;
+    if (l < 3) {
+        const bool avg = A.dims == 3 || (A.dims == 2 && A.mode2d == 2 && l < 2);
+        const bool one = (A.dims == 2 && A.mode2d != 2 && l == 2) || (A.dims == 1 && l == 0);
+        const R *f = F.f[l];
+        if (avg) {
+            const long long s = l == 0 ? 1 : (l == 1 ? (long long)L.px : L.pz);
+            E = 0.5 * ((double)f[c - s] + (double)f[c]);
+        } else if (one) {
+            E = (double)f[c];
+        }
+    }
+    const double *pr = A.par + (long long)n * A.npar;
+    const double *u = pr + (A.npar - 3);
+    const double E0 = __shfl_sync(FULL, E, 0, LANES), E1 = __shfl_sync(FULL, E, 1, LANES),
+                 E2 = __shfl_sync(FULL, E, 2, LANES);
+    const double E_u = u[0] * E0 + u[1] * E1 + u[2] * E2;
+    constexpr int NST = LANES == 8 ? 8 : 3;
+    const int w = min(l, NST - 1);
+    double *st = A.rho + (long long)n * NST;
+    const EmitLane q = emit_lane<LANES>(w, pr, E_u, A.rates[2 * n], A.rates[2 * n + 1]);
+    const double x = rk4_lane<LANES>(q, w, st[w], A.dt, A.h2, A.h6);
+    if (live && l < NST) st[l] = x;
+    double d;
+    if (LANES == 4) {
+        d = 2.0 * pr[1] * __shfl_sync(FULL, x, 1, LANES);
+    } else {
+        const double x2 = __shfl_sync(FULL, x, 2, LANES), x4 = __shfl_sync(FULL, x, 4, LANES);
+        d = 2.0 * pr[2] * x2 + 2.0 * pr[3] * x4;
+    }
+    if (live && l < 3) {
+        const double old = A.dipole[3 * n + l];
+        const double nw = d * u[l];
+        A.dipole[3 * n + l] = nw;
+        A.dPdt[3 * n + l] = A.inv_dt != 0.0 ? (nw - old) * A.inv_dt : (nw - old) / A.dt;
+        A.E[3 * n + l] = E;
+    }
+}
+
 // send_J_to_E_ranks (interactions_mod.f90:1046-1220): J_old = J; J(point) = wk*dPt_dt of the
 // last emitter writing the point (assignment); dJ = (J - J_old)/dt (times 1/dt with FP32 fields,
 // as dPt_dt in k_emit).  Points this group does not write keep J, so their dJ becomes zero, as

@@ -101,3 +101,31 @@ def test_field_round_trip(dims, n, bnd, mode, field, precision):
             want[tuple(-1 if y == x else slice(None) for y in range(3))] = 0.0
     assert np.array_equal(g.read_field(field), want)
     g.kill()
+
+
+@pytest.mark.parametrize("model,n", [(1, 1), (1, 9), (1, 8192), (1, 8193), (2, 1), (2, 5), (2, 6144), (2, 6145)])
+def test_emitter_forms_bit_identical(orc, model, n):
+    """One lane per state word up to a number of emitters, one thread per emitter above: the first
+    and last sizes of each, partly filled warps."""
+    gpu, cpu, dt = seeded_pair(orc, 3, (20, 18, 22), 3, (3, 2, 1), 37.8, omx.TMZ, 1e-3, n)
+    rng = np.random.default_rng(n)
+    cells = np.stack([rng.integers(2, m, n) for m in (20, 18, 22)], 1).astype(np.int32)
+    u = rng.standard_normal((n, 3))
+    levels = [rng.uniform(0.05, 0.12, n) for _ in range(model)]
+    mu = [rng.uniform(1.0, 4.0, n) for _ in range(model)]
+    par = np.stack(levels + mu + [rng.uniform(2e3, 4e4, n), rng.uniform(1e3, 4e3, n)], 1)
+    par = np.concatenate([par, u / np.linalg.norm(u, axis=1, keepdims=True)], 1)
+    gg = gpu.add_q_group(omx.Q_MATERIAL, model, cells, par, 1e-6, dt)
+    before = gg.read()
+    for tt in range(1, 4):
+        gpu.run(tt, 1)
+        a = gg.read()
+        E_u = par[:, -3] * a["E"][:, 0] + par[:, -2] * a["E"][:, 1] + par[:, -1] * a["E"][:, 2]
+        rho = np.array([orc.emitter_step(model, par[e], before["rho"][e], E_u[e], dt) for e in range(n)])
+        d = 2.0 * par[:, 1] * rho[:, 1] if model == 1 else 2.0 * par[:, 2] * rho[:, 2] + 2.0 * par[:, 3] * rho[:, 4]
+        dip = d[:, None] * par[:, -3:]
+        assert np.array_equal(a["rho"], rho) and np.max(np.abs(rho)) > 0
+        assert np.array_equal(a["dipole"], dip)
+        assert np.array_equal(a["dPt_dt"], (dip - before["dipole"]) / dt)
+        before = a
+    gpu.kill()
