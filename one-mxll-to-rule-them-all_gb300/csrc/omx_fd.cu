@@ -8,10 +8,12 @@
 // The operator kernel keeps the reference's operand order with FMA contraction off (this file is
 // compiled with -fmad=false), so A f equals the FP64 oracle bit for bit.  The solver's scalar
 // recursion runs on the host exactly as the oracle's; its dot products are reduced on the device
-// per block and summed on the host in block order (deterministic, not the oracle's order).
+// per row of cells and summed on the host in row order (deterministic, not the oracle's order).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -47,7 +49,7 @@ struct FdGeom {
     long long px, pxy, len;   // padded row and plane pitch, elements per component
     int per[3];
     double coef[9];
-    double w0, sign;
+    double w0, w0_half, sign;
 };
 
 __device__ inline long long fd_at(const FdGeom &G, int i, int j, int k)   // 1-based interior indices
@@ -82,13 +84,21 @@ __global__ void k_fd_ghosts(cplx *f, FdGeom G, int axis)
     if (hi) v[at(na + t)] = v[at(t)];
 }
 
-// apply_operator_3D: one thread per interior cell
-__global__ void __launch_bounds__(128) k_fd_apply(const cplx *__restrict__ f, cplx *__restrict__ Af, FdGeom G,
-                                                  const cplx *__restrict__ sx, const cplx *__restrict__ sy,
-                                                  const cplx *__restrict__ sz, const cplx *__restrict__ eps)
+// The operator's cell functions.  fd_cell drops what is exact in finite arithmetic: the zero centre
+// tap and products with the zero parts of C1..C4 and with a stretch factor of 1 (282 of 476 FP64
+// operations a cell left in 3D at n_der 2, and 72 more in cells with PML on every axis).  Infinities
+// and NaN spread differently through the dropped products, so a component that meets one is computed
+// again by the full form below, which writes every product out as the reference's complex
+// arithmetic does.
+struct FdTables {
+    const cplx *sx, *sy, *sz, *eps;
+};
+
+// component c of apply_operator_3D at one cell, written out
+__device__ __noinline__ void fd_full3(const cplx *f, cplx *Af, const FdGeom &G, const FdTables &T, int i, int j, int k,
+                                     int c)
 {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, j = 1 + blockIdx.y, k = 1 + blockIdx.z;
-    if (i > G.nx) return;
+    const cplx *sx = T.sx, *sy = T.sy, *sz = T.sz, *eps = T.eps;
     const long long p = fd_at(G, i, j, k);
     const cplx *plx = f, *ply = f + G.len, *plz = f + 2 * G.len, *mix = f + 3 * G.len, *miy = f + 4 * G.len,
                *miz = f + 5 * G.len;
@@ -137,21 +147,22 @@ __global__ void __launch_bounds__(128) k_fd_apply(const cplx *__restrict__ f, cp
     const cplx C1 = {0.0, G.sign}, mC1 = {-0.0, -G.sign}, C2 = {0.0, -G.w0}, C3 = {0.0, -G.w0 / 2.0}, C4 = {1.0, 0.0};
     const cplx e = eps[(long long)(i - 1) + (long long)G.nx * ((j - 1) + (long long)G.ny * (k - 1))];
     const cplx m3 = cmul(C3, csub(e, C4));
-    Af[p] = cadd(cadd(cmul(C1, csub(dpzdy, dpydz)), cmul(C2, plx[p])), cmul(m3, Ex));
-    Af[p + G.len] = cadd(cadd(cmul(C1, csub(dpxdz, dpzdx)), cmul(C2, ply[p])), cmul(m3, Ey));
-    Af[p + 2 * G.len] = cadd(cadd(cmul(C1, csub(dpydx, dpxdy)), cmul(C2, plz[p])), cmul(m3, Ez));
-    Af[p + 3 * G.len] = cadd(cadd(cmul(mC1, csub(dmzdy, dmydz)), cmul(C2, mix[p])), cmul(m3, Ex));
-    Af[p + 4 * G.len] = cadd(cadd(cmul(mC1, csub(dmxdz, dmzdx)), cmul(C2, miy[p])), cmul(m3, Ey));
-    Af[p + 5 * G.len] = cadd(cadd(cmul(mC1, csub(dmydx, dmxdy)), cmul(C2, miz[p])), cmul(m3, Ez));
+    cplx out[6];
+    out[0] = cadd(cadd(cmul(C1, csub(dpzdy, dpydz)), cmul(C2, plx[p])), cmul(m3, Ex));
+    out[1] = cadd(cadd(cmul(C1, csub(dpxdz, dpzdx)), cmul(C2, ply[p])), cmul(m3, Ey));
+    out[2] = cadd(cadd(cmul(C1, csub(dpydx, dpxdy)), cmul(C2, plz[p])), cmul(m3, Ez));
+    out[3] = cadd(cadd(cmul(mC1, csub(dmzdy, dmydz)), cmul(C2, mix[p])), cmul(m3, Ex));
+    out[4] = cadd(cadd(cmul(mC1, csub(dmxdz, dmzdx)), cmul(C2, miy[p])), cmul(m3, Ey));
+    out[5] = cadd(cadd(cmul(mC1, csub(dmydx, dmxdy)), cmul(C2, miz[p])), cmul(m3, Ez));
+    for (int y = 0; y < 6; ++y)
+        if (y == c) Af[p + c * G.len] = out[y];
 }
 
-// apply_operator_1D: one thread per cell; the products keep the reference's order C1 * d * s_inv,
+// apply_operator_1D at one cell; the products keep the reference's order C1 * d * s_inv,
 // and the y components carry no medium term (as written in the reference)
-__global__ void __launch_bounds__(128) k_fd_apply1(const cplx *__restrict__ f, cplx *__restrict__ Af, FdGeom G,
-                                                   const cplx *__restrict__ sx, const cplx *__restrict__ eps)
+__device__ void fd_cell1(const cplx *f, const FdGeom &G, const FdTables &T, int i, cplx *out)
 {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > G.nx) return;
+    const cplx *sx = T.sx, *eps = T.eps;
     const long long p = fd_at(G, i, 1, 1);
     const cplx *plx = f, *ply = f + G.len, *mix = f + 2 * G.len, *miy = f + 3 * G.len;
     const int n = G.n_der;
@@ -167,20 +178,17 @@ __global__ void __launch_bounds__(128) k_fd_apply1(const cplx *__restrict__ f, c
     const cplx Ex = cadd(plx[p], mix[p]);
     const cplx s = sx[i - 1], e = eps[i - 1];
     const cplx m3 = cmul(C3, csub(e, C4));
-    Af[p] = cadd(cadd(cmul(cmul(mC1, dpydz), s), cmul(C2, plx[p])), cmul(m3, Ex));
-    Af[p + G.len] = cadd(cmul(cmul(C1, dpxdz), s), cmul(C2, ply[p]));
-    Af[p + 2 * G.len] = cadd(cadd(cmul(cmul(C1, dmydz), s), cmul(C2, mix[p])), cmul(m3, Ex));
-    Af[p + 3 * G.len] = cadd(cmul(cmul(mC1, dmxdz), s), cmul(C2, miy[p]));
+    out[0] = cadd(cadd(cmul(cmul(mC1, dpydz), s), cmul(C2, plx[p])), cmul(m3, Ex));
+    out[1] = cadd(cmul(cmul(C1, dpxdz), s), cmul(C2, ply[p]));
+    out[2] = cadd(cadd(cmul(cmul(C1, dmydz), s), cmul(C2, mix[p])), cmul(m3, Ex));
+    out[3] = cadd(cmul(cmul(mC1, dmxdz), s), cmul(C2, miy[p]));
 }
 
-// apply_operator_2D: one thread per cell; the curl terms carry the opposite sign of the 3D
+// component c of apply_operator_2D at one cell, written out; the curl terms carry the opposite sign of the 3D
 // operator's (as written in the reference)
-__global__ void __launch_bounds__(128) k_fd_apply2(const cplx *__restrict__ f, cplx *__restrict__ Af, FdGeom G,
-                                                   const cplx *__restrict__ sx, const cplx *__restrict__ sy,
-                                                   const cplx *__restrict__ eps)
+__device__ __noinline__ void fd_full2(const cplx *f, cplx *Af, const FdGeom &G, const FdTables &T, int i, int j, int c)
 {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, j = 1 + blockIdx.y;
-    if (i > G.nx) return;
+    const cplx *sx = T.sx, *sy = T.sy, *eps = T.eps;
     const long long p = fd_at(G, i, j, 1);
     const cplx *plx = f, *ply = f + G.len, *plz = f + 2 * G.len, *mix = f + 3 * G.len, *miy = f + 4 * G.len,
                *miz = f + 5 * G.len;
@@ -215,49 +223,226 @@ __global__ void __launch_bounds__(128) k_fd_apply2(const cplx *__restrict__ f, c
     const cplx C1 = {0.0, G.sign}, mC1 = {-0.0, -G.sign}, C2 = {0.0, -G.w0}, C3 = {0.0, -G.w0 / 2.0}, C4 = {1.0, 0.0};
     const cplx e = eps[(long long)(i - 1) + (long long)G.nx * (j - 1)];
     const cplx m3 = cmul(C3, csub(e, C4));
-    Af[p] = cadd(cadd(cmul(mC1, dpzdy), cmul(C2, plx[p])), cmul(m3, Ex));
-    Af[p + G.len] = cadd(cadd(cmul(C1, dpzdx), cmul(C2, ply[p])), cmul(m3, Ey));
-    Af[p + 2 * G.len] = cadd(cadd(cmul(mC1, csub(dpydx, dpxdy)), cmul(C2, plz[p])), cmul(m3, Ez));
-    Af[p + 3 * G.len] = cadd(cadd(cmul(C1, dmzdy), cmul(C2, mix[p])), cmul(m3, Ex));
-    Af[p + 4 * G.len] = cadd(cadd(cmul(mC1, dmzdx), cmul(C2, miy[p])), cmul(m3, Ey));
-    Af[p + 5 * G.len] = cadd(cadd(cmul(C1, csub(dmydx, dmxdy)), cmul(C2, miz[p])), cmul(m3, Ez));
+    cplx out[6];
+    out[0] = cadd(cadd(cmul(mC1, dpzdy), cmul(C2, plx[p])), cmul(m3, Ex));
+    out[1] = cadd(cadd(cmul(C1, dpzdx), cmul(C2, ply[p])), cmul(m3, Ey));
+    out[2] = cadd(cadd(cmul(mC1, csub(dpydx, dpxdy)), cmul(C2, plz[p])), cmul(m3, Ez));
+    out[3] = cadd(cadd(cmul(C1, dmzdy), cmul(C2, mix[p])), cmul(m3, Ex));
+    out[4] = cadd(cadd(cmul(mC1, dmzdx), cmul(C2, miy[p])), cmul(m3, Ey));
+    out[5] = cadd(cadd(cmul(C1, csub(dmydx, dmxdy)), cmul(C2, miz[p])), cmul(m3, Ez));
+    for (int y = 0; y < 6; ++y)
+        if (y == c) Af[p + c * G.len] = out[y];
 }
 
-// vector operations over the interior of every component (rs_operations_subs_mod.f90)
-// mode 0: v1 = v1 + a v2;  mode 1: v1 = a v1 + v2;  mode 2: v1 = a v1
-__global__ void k_fd_lin(cplx *v1, const cplx *v2, cplx a, FdGeom G, int mode)
+// derivative of one component along the axis of pitch o: the taps in the reference's order
+template <int N> __device__ __forceinline__ cplx fd_der(const cplx *v, long long o, const double *coef)
 {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, j = 1 + blockIdx.y, k = 1 + blockIdx.z;
-    if (i > G.nx) return;
+    cplx d = cscale(v[-N * o], coef[0]);
+#pragma unroll
+    for (int q = -N + 1; q <= N; ++q)
+        if (q != 0) d = cadd(d, cscale(v[q * o], coef[N + q]));
+    return d;
+}
+// The tests and sign changes below are integer operations: the FP64 pipe is what the pass waits for.
+__device__ __forceinline__ bool fd_is(double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); }
+__device__ __forceinline__ double fd_flip(double a, bool neg)
+{
+    return __longlong_as_double(__double_as_longlong(a) ^ (neg ? (long long)0x8000000000000000ull : 0ll));
+}
+__device__ __forceinline__ cplx fd_stretch(cplx d, cplx s) { return fd_is(s.re, 1.0) && fd_is(s.im, 0.0) ? d : cmul(d, s); }
+// (s i) x with s = -1 (neg) or +1, and -(w i) x
+__device__ __forceinline__ cplx fd_times_i(cplx x, bool neg) { return {fd_flip(x.im, !neg), fd_flip(x.re, neg)}; }
+__device__ __forceinline__ cplx fd_times_mwi(cplx x, double w) { return {w * x.im, -(w * x.re)}; }
+__device__ __forceinline__ bool fd_nonfinite(cplx a)
+{
+    return (__double2hiint(a.re) & 0x7ff00000) == 0x7ff00000 || (__double2hiint(a.im) & 0x7ff00000) == 0x7ff00000;
+}
+
+// Component c of A f at one cell (2D, 3D).  Component 3 h + q of half h takes the curl component q of
+// that half's three: the difference of the derivatives of its v1 along one axis and v2 along another.
+template <int DIMS, int N>
+__device__ __forceinline__ cplx fd_cell(const cplx *__restrict__ f, const FdGeom &G, const FdTables &T, int i, int j, int k,
+                                        int c, bool &bad)
+{
     const long long p = fd_at(G, i, j, k);
-    for (int c = 0; c < G.ncomp; ++c) {
-        const long long q = p + c * G.len;
-        const cplx x = v1[q];
-        if (mode == 0) v1[q] = cadd(x, cmul(a, v2[q]));
-        else if (mode == 1) v1[q] = cadd(cmul(a, x), v2[q]);
-        else v1[q] = cmul(a, x);
+    const int h = c >= 3 ? 3 : 0, q = c - h;
+    const cplx e = T.eps[(long long)(i - 1) + (long long)G.nx * ((j - 1) + (long long)G.ny * (k - 1))];
+    const cplx m3 = fd_times_mwi(cplx{e.re - 1.0, e.im}, G.w0_half);
+    const cplx x = f[p + c * G.len];
+    const cplx med = cmul(m3, cadd(f[p + q * G.len], f[p + (q + 3) * G.len]));
+    const bool neg = (h == 0) != (G.sign > 0.0);
+    // 3D: z along y - y along z;  x along z - z along x;  y along x - x along y.  2D: the z terms vanish
+    const cplx *v1 = f + p + (h + (q == 0 ? 2 : (q == 1 ? (DIMS == 3 ? 0 : 2) : 1))) * G.len;
+    const cplx *v2 = f + p + (h + (q == 0 ? 1 : (q == 1 ? 2 : 0))) * G.len;
+    cplx cu;
+    bad = fd_nonfinite(v1[0]);
+    if (DIMS == 3 || q == 2) {
+        const long long o1 = q == 0 ? G.px : (q == 1 ? G.pxy : 1), o2 = q == 0 ? G.pxy : (q == 1 ? 1 : G.px);
+        const cplx t1 = q == 0 ? T.sy[j - 1] : (q == 1 ? T.sz[k - 1] : T.sx[i - 1]);
+        const cplx t2 = q == 0 ? T.sz[k - 1] : (q == 1 ? T.sx[i - 1] : T.sy[j - 1]);
+        bad |= fd_nonfinite(v2[0]);
+        const cplx d = csub(fd_stretch(fd_der<N>(v1, o1, G.coef), t1), fd_stretch(fd_der<N>(v2, o2, G.coef), t2));
+        cu = fd_times_i(d, DIMS == 3 ? neg : !neg);
+    } else {
+        cu = fd_times_i(fd_stretch(fd_der<N>(v1, q == 0 ? G.px : 1, G.coef), q == 0 ? T.sy[j - 1] : T.sx[i - 1]),
+                        q == 0 ? !neg : neg);
+    }
+    const cplx out = cadd(cadd(cu, fd_times_mwi(x, G.w0)), med);
+    bad |= fd_nonfinite(out);
+    return out;
+}
+
+// component c of A f at one cell, into Af
+template <int DIMS, int N>
+__device__ __forceinline__ void fd_apply_value(const cplx *__restrict__ f, cplx *Af, const FdGeom &G, const FdTables &T, int i,
+                                               int j, int k, int c)
+{
+    cplx *dst = Af + fd_at(G, i, j, k) + c * G.len;
+    if (DIMS == 1) {
+        cplx all[4];
+        fd_cell1(f, G, T, i, all);
+        *dst = c == 0 ? all[0] : (c == 1 ? all[1] : (c == 2 ? all[2] : all[3]));
+        return;
+    }
+    bool bad;
+    *dst = fd_cell<DIMS == 1 ? 2 : DIMS, N>(f, G, T, i, j, k, c, bad);
+    if (bad) {
+        if (DIMS == 3) fd_full3(f, Af, G, T, i, j, k, c);
+        else fd_full2(f, Af, G, T, i, j, c);
     }
 }
 
-// per-block partial sums of conj(v1) v2 over the interior (one block per (j, k) row)
-__global__ void k_fd_dot(const cplx *v1, const cplx *v2, FdGeom G, cplx *part)
+// One launch of the solver between two of its dot products: A f (optional), a list of vector
+// operations over the interior of every component (rs_operations_subs_mod.f90), the periodic ghost
+// copies of the vector the next operator application reads, and the row partials of up to three
+// dot products.  All of it but the operator's taps is local to a value, so a thread that owns
+// the cells i, i + T, ... of one row (or one component of them) needs no synchronisation between
+// the parts.
+struct FdLin {
+    cplx *v1;
+    const cplx *v2;
+    cplx a;
+    int mode;   // 0: v1 = v1 + a v2;  1: v1 = a v1 + v2;  2: v1 = a v1
+};
+constexpr int FD_LIN_MAX = 26, FD_DOT_MAX = 3;
+struct FdPass {
+    const cplx *f;           // operator application Af = A f, or null
+    cplx *Af;
+    int nlin, ndot;
+    FdLin lin[FD_LIN_MAX];
+    const cplx *da[FD_DOT_MAX], *db[FD_DOT_MAX];   // sum conj(da) db
+    cplx *ghost;             // vector whose periodic ghosts are refreshed, or null
+    cplx *part;              // [ndot][rows] row partials, in host memory
+    unsigned *done;          // finished blocks (device), zero between launches
+    unsigned *flag, seq;     // *flag = seq once every partial is written (host memory)
+};
+
+__device__ __forceinline__ void fd_lin_value(const FdLin &o, long long q)
 {
-    __shared__ cplx sh[128];
-    const int j = 1 + blockIdx.x, k = 1 + blockIdx.y;
-    cplx s = {0, 0};
-    for (int c = 0; c < G.ncomp; ++c)
-        for (int i = 1 + threadIdx.x; i <= G.nx; i += blockDim.x) {
-            const long long q = fd_at(G, i, j, k) + c * G.len;
-            const cplx a = {v1[q].re, -v1[q].im};
-            s = cadd(s, cmul(a, v2[q]));
-        }
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] = cadd(sh[threadIdx.x], sh[threadIdx.x + o]);
-        __syncthreads();
+    const cplx x = o.v1[q];
+    if (o.mode == 0) o.v1[q] = cadd(x, cmul(o.a, o.v2[q]));
+    else if (o.mode == 1) o.v1[q] = cadd(cmul(o.a, x), o.v2[q]);
+    else o.v1[q] = cmul(o.a, x);
+}
+
+// k_fd_ghosts' copies of component c of the cell (i, j, k), by the thread that owns it
+__device__ __forceinline__ void fd_ghost_value(cplx *f, const FdGeom &G, int i, int j, int k, int c)
+{
+    const int at[3] = {i, j, k}, n[3] = {G.nx, G.ny, G.nz};
+    const long long pitch[3] = {1, G.px, G.pxy};
+    cplx *v = f + fd_at(G, i, j, k) + c * G.len;
+    for (int a = 0; a < G.dims; ++a) {
+        if (!G.per[a]) continue;
+        const bool quirk = a == 1 && G.dims == 3;
+        if (at[a] > n[a] - G.g && !(quirk && c == 4)) v[-n[a] * pitch[a]] = v[0];
+        if (at[a] <= G.g && !(quirk && c == 3)) v[n[a] * pitch[a]] = v[0];
     }
-    if (threadIdx.x == 0) part[blockIdx.x + (long long)gridDim.x * blockIdx.y] = sh[0];
+}
+
+// T threads (32, 64 or 128) along a row of cells.  The FP64 pipe bounds the pass; it takes a warp's
+// instruction every 64 cycles per sub-partition.  SPLIT: one row per block, a thread row per
+// component, for grids with few rows -- with a thread per cell a 30 x 27 x 25 grid is 675 warps on 608
+// sub-partitions, two rounds of the longest chain (294 us an outer iteration of BiCGStab(2)); split, it
+// is 4050 short ones (223 us).  Otherwise a thread per cell and 128 / T rows per block: the medium
+// term is formed once for a component pair (60^3: 1.43 against 1.59 ms split).  Before, every dot,
+// vector operation and operator was a launch of its own: 457 us and 2.00 ms.
+// A row's dot partial is summed per thread over its cells (components outermost) and then over the T
+// threads by halving: the order of a 128-thread block per row whose threads past nx hold zeros, for
+// every T >= nx.
+constexpr int fd_threads(bool split, int dims, int T) { return split ? T * (dims == 1 ? 4 : 6) : 128; }
+constexpr int fd_min_blocks(bool split, int T) { return split ? (T == 32 ? 5 : (T == 64 ? 2 : 1)) : 4; }
+template <int DIMS, int N, int T, bool SPLIT>
+__global__ void __launch_bounds__(fd_threads(SPLIT, DIMS, T), fd_min_blocks(SPLIT, T))
+    k_fd_pass(const __grid_constant__ FdPass P, const __grid_constant__ FdGeom G, const __grid_constant__ FdTables A)
+{
+    constexpr int NC = DIMS == 1 ? 4 : 6, RPB = SPLIT ? 1 : 128 / T;
+    __shared__ cplx sh[FD_DOT_MAX][SPLIT ? NC : RPB][T];
+    const int t = threadIdx.x, ty = threadIdx.y;
+    const int rows = G.ny * G.nz, row = blockIdx.x * RPB + (SPLIT ? 0 : ty);
+    const bool live = row < rows;
+    const int j = 1 + row % G.ny, k = 1 + row / G.ny;
+    // blockIdx.y: pieces of a long row (launches without dots only)
+    const int i0 = 1 + t + T * blockIdx.y, i1 = live ? G.nx : 0, step = T * gridDim.y;
+    if (P.f)
+        for (int i = i0; i <= i1; i += step) {
+            if (SPLIT) {
+                fd_apply_value<DIMS, N>(P.f, P.Af, G, A, i, j, k, ty);
+            } else {
+#pragma unroll
+                for (int c = 0; c < NC; ++c) fd_apply_value<DIMS, N>(P.f, P.Af, G, A, i, j, k, c);
+            }
+        }
+    if (P.nlin || P.ghost)
+        for (int i = i0; i <= i1; i += step)
+            for (int c = SPLIT ? ty : 0; c < (SPLIT ? ty + 1 : NC); ++c) {
+                const long long q = fd_at(G, i, j, k) + c * G.len;
+                for (int o = 0; o < P.nlin; ++o) fd_lin_value(P.lin[o], q);
+                if (P.ghost) fd_ghost_value(P.ghost, G, i, j, k, c);
+            }
+    if (P.ndot == 0) return;
+    // product of one value pair, and a thread's sum over its cells
+    auto product = [&](int d, long long q) {
+        const cplx va = P.da[d][q], vb = P.db[d][q];
+        return cmul(cplx{va.re, -va.im}, vb);
+    };
+    auto row_sum = [&](int d) {
+        cplx s = {0, 0};
+        for (int y = 0; y < NC; ++y)
+            for (int i = 1 + t; i <= i1; i += T) s = cadd(s, product(d, fd_at(G, i, j, k) + y * G.len));
+        return s;
+    };
+    const bool one = G.nx <= T;             // a cell per thread: split, the products by component in parallel
+    if (SPLIT && one) {
+        const long long q = fd_at(G, min(1 + t, G.nx), j, k) + ty * G.len;
+        for (int d = 0; d < P.ndot; ++d) sh[d][ty][t] = t < G.nx ? product(d, q) : cplx{0.0, 0.0};
+    }
+    if (SPLIT) __syncthreads();             // and the values that other components' threads wrote
+    // split: thread row d sums dot d; else a row's threads sum every dot
+    const int d0 = SPLIT ? ty : 0, d1 = SPLIT ? min(ty + 1, P.ndot) : P.ndot, slot = SPLIT ? 0 : ty;
+    for (int d = d0; d < d1; ++d) {
+        cplx s = {0, 0};
+        if (SPLIT && one)
+            for (int y = 0; y < NC; ++y) s = cadd(s, sh[d][y % (SPLIT ? NC : RPB)][t]);
+        else
+            s = row_sum(d);
+        sh[d][slot][t] = s;
+    }
+    for (int o = T / 2; o > 0; o >>= 1) {
+        if (T == 32) __syncwarp();          // a thread row is a warp
+        else __syncthreads();
+        if (t < o)
+            for (int d = d0; d < d1; ++d) sh[d][slot][t] = cadd(sh[d][slot][t], sh[d][slot][t + o]);
+    }
+    if (t == 0 && live && d0 < d1) {
+        for (int d = d0; d < d1; ++d) P.part[(long long)d * rows + row] = sh[d][slot][0];
+        __threadfence_system();
+    }
+    __syncthreads();
+    if (ty == 0 && t == 0 && atomicAdd(P.done, 1u) == gridDim.x - 1) {
+        *P.done = 0;
+        __threadfence_system();
+        *(volatile unsigned *)P.flag = P.seq;
+    }
 }
 
 }  // namespace
@@ -266,7 +451,9 @@ struct omx_fdop {
     FdGeom G{};
     cudaStream_t s = nullptr;
     cplx *sx = nullptr, *sy = nullptr, *sz = nullptr, *eps = nullptr;
-    cplx *part = nullptr, *hpart = nullptr;
+    cplx *hpart = nullptr;      // [FD_DOT_MAX][rows] partials, then the flag word (pinned, written by the device)
+    unsigned *done = nullptr;
+    unsigned seq = 0;
     std::vector<cplx *> vecs;   // solver work vectors
     ~omx_fdop()
     {
@@ -274,7 +461,7 @@ struct omx_fdop {
         cudaFree(sy);
         cudaFree(sz);
         cudaFree(eps);
-        cudaFree(part);
+        cudaFree(done);
         if (hpart) cudaFreeHost(hpart);
         for (auto *v : vecs) cudaFree(v);
         if (s) cudaStreamDestroy(s);
@@ -298,8 +485,54 @@ void fck(cudaError_t e, const char *w)
     if (e != cudaSuccess) throw FdErr{OMX_ERR_CUDA, std::string(w) + ": " + cudaGetErrorString(e)};
 }
 
-dim3 cell_grid(const FdGeom &G) { return dim3((G.nx + 127) / 128, G.ny, G.nz); }
+template <int V> struct IntC {
+    static constexpr int value = V;
+};
+// call fn(dimensions, n_der) with both as compile-time constants
+template <class F> void by_shape(const FdGeom &G, F &&fn)
+{
+    auto order = [&](auto d) {
+        switch (G.n_der) {
+        case 1: fn(d, IntC<1>{}); break;
+        case 2: fn(d, IntC<2>{}); break;
+        case 3: fn(d, IntC<3>{}); break;
+        default: fn(d, IntC<4>{}); break;
+        }
+    };
+    if (G.dims == 1) fn(IntC<1>{}, IntC<1>{});   // the 1D cell reads n_der itself
+    else if (G.dims == 2) order(IntC<2>{});
+    else order(IntC<3>{});
+}
 
+// Rows up to this long go through one launch a pass.  Longer ones are cut into pieces for the
+// operator and the vector operations, and the dots get a launch of their own: one block a row would
+// leave a grid of few long rows to a handful of blocks.
+constexpr int FD_ROW_MAX = 256;
+// warps of one thread per cell below which a pass takes a thread per component (k_fd_pass)
+constexpr int FD_SPLIT_WARPS = 1024;
+
+void fd_launch_pass(omx_fdop *op, const FdPass &P)
+{
+    const FdGeom &G = op->G;
+    const int rows = G.ny * G.nz, T = G.nx <= 32 ? 32 : (G.nx <= 64 ? 64 : 128);
+    const unsigned pieces = P.ndot > 0 ? 1u : (unsigned)std::min((G.nx + T - 1) / T, 65535);
+    const bool split = (long long)rows * T / 32 < FD_SPLIT_WARPS;
+    const FdTables A{op->sx, op->sy, op->sz, op->eps};
+    by_shape(G, [&](auto dc, auto nc) {
+        constexpr int D = decltype(dc)::value, N = decltype(nc)::value, C = D == 1 ? 4 : 6;
+        auto go = [&](auto tc) {
+            constexpr int W = decltype(tc)::value, R = 128 / W;
+            if (split) k_fd_pass<D, N, W, true><<<dim3((unsigned)rows, pieces), dim3(W, C), 0, op->s>>>(P, G, A);
+            else k_fd_pass<D, N, W, false><<<dim3((unsigned)((rows + R - 1) / R), pieces), dim3(W, R), 0, op->s>>>(P, G, A);
+        };
+        if (T == 32) go(IntC<32>{});
+        else if (T == 64) go(IntC<64>{});
+        else go(IntC<128>{});
+    });
+    fck(cudaPeekAtLastError(), "launch");
+}
+
+// Af = A f for a vector whose periodic ghosts may be stale
 void fd_apply_dev(omx_fdop *op, cplx *f, cplx *Af)
 {
     const FdGeom &G = op->G;
@@ -309,26 +542,50 @@ void fd_apply_dev(omx_fdop *op, cplx *f, cplx *Af)
         const long long cnt = (long long)G.ncomp * G.g * n1 * n2;
         k_fd_ghosts<<<(unsigned)((cnt + 255) / 256), 256, 0, op->s>>>(f, G, a);
     }
-    if (G.dims == 1) k_fd_apply1<<<cell_grid(G), 128, 0, op->s>>>(f, Af, G, op->sx, op->eps);
-    else if (G.dims == 2) k_fd_apply2<<<cell_grid(G), 128, 0, op->s>>>(f, Af, G, op->sx, op->sy, op->eps);
-    else k_fd_apply<<<cell_grid(G), 128, 0, op->s>>>(f, Af, G, op->sx, op->sy, op->sz, op->eps);
+    FdPass P{};
+    P.f = f;
+    P.Af = Af;
+    fd_launch_pass(op, P);
 }
 
-void fd_lin(omx_fdop *op, cplx *v1, const cplx *v2, cplx a, int mode)
-{
-    k_fd_lin<<<cell_grid(op->G), 128, 0, op->s>>>(v1, v2, a, op->G, mode);
-}
-
-cplx fd_dot(omx_fdop *op, const cplx *v1, const cplx *v2)
+// Run a pass; with dots, wait for their partials and sum them in row order into dots[0..ndot-1].
+// The partials come straight into pinned memory and the host watches the flag word behind them
+// (a copy and a stream synchronisation per dot cost 10 us; this about 3).  The stream's own state
+// ends the wait when the launch failed.
+void fd_pass(omx_fdop *op, FdPass &P, cplx *dots = nullptr)
 {
     const FdGeom &G = op->G;
-    k_fd_dot<<<dim3(G.ny, G.nz), 128, 0, op->s>>>(v1, v2, G, op->part);
-    const size_t nb = (size_t)G.ny * G.nz;
-    fck(cudaMemcpyAsync(op->hpart, op->part, nb * sizeof(cplx), cudaMemcpyDeviceToHost, op->s), "dot");
-    fck(cudaStreamSynchronize(op->s), "dot");
-    cplx s = {0, 0};
-    for (size_t b = 0; b < nb; ++b) s = cadd(s, op->hpart[b]);
-    return s;
+    const size_t rows = (size_t)G.ny * G.nz;
+    const int ndot = P.ndot;
+    if (ndot > 0 && G.nx > FD_ROW_MAX && (P.f || P.nlin || P.ghost)) {
+        P.ndot = 0;
+        fd_launch_pass(op, P);
+        P.ndot = ndot;
+        P.f = nullptr;
+        P.nlin = 0;
+        P.ghost = nullptr;
+    }
+    unsigned *flag = reinterpret_cast<unsigned *>(op->hpart + FD_DOT_MAX * rows);
+    P.part = op->hpart;
+    P.done = op->done;
+    P.flag = flag;
+    P.seq = ++op->seq;
+    fd_launch_pass(op, P);
+    if (ndot == 0) return;
+    for (long long spin = 1; __atomic_load_n(flag, __ATOMIC_ACQUIRE) != P.seq; ++spin) {
+        if (spin % 4096) continue;
+        const cudaError_t e = cudaStreamQuery(op->s);
+        if (e == cudaErrorNotReady) continue;
+        fck(e, "dot");
+        fck(cudaStreamSynchronize(op->s), "dot");
+        if (__atomic_load_n(flag, __ATOMIC_ACQUIRE) != P.seq) throw FdErr{OMX_ERR_CUDA, "dot: the partial sums did not arrive"};
+        break;
+    }
+    for (int d = 0; d < ndot; ++d) {
+        cplx s = {0, 0};
+        for (size_t b = 0; b < rows; ++b) s = cadd(s, op->hpart[d * rows + b]);
+        dots[d] = s;
+    }
 }
 
 }  // namespace
@@ -370,6 +627,7 @@ int omx_fd_create(int dimensions, const int grid_Ndims[3], int n_pml, int n_der,
         G.len = G.pxy * (G.nz + 2 * G.gz);
         for (int a = 0; a < 3; ++a) G.per[a] = a < dimensions && boundaries[a] == 2;
         G.w0 = w0;
+        G.w0_half = w0 / 2.0;
         // operator_mod.f90:97-140: central-difference coefficients of order 2 n_der, / dr
         static const double C[4][9] = {{-0.5, 0.0, 0.5},
                                        {1.0 / 12.0, -2.0 / 3.0, 0.0, 2.0 / 3.0, -1.0 / 12.0},
@@ -404,8 +662,12 @@ int omx_fd_create(int dimensions, const int grid_Ndims[3], int n_pml, int n_der,
         fck(cudaMalloc(&op->eps, sizeof(cplx) * ncell), "alloc");
         fck(cudaMemcpy(op->eps, eps_r, sizeof(cplx) * ncell, cudaMemcpyHostToDevice), "upload");
         fck(cudaStreamSynchronize(0), "upload");   // pageable copies may return before their DMA ends
-        fck(cudaMalloc(&op->part, sizeof(cplx) * (size_t)G.ny * G.nz), "alloc");
-        fck(cudaMallocHost(&op->hpart, sizeof(cplx) * (size_t)G.ny * G.nz), "alloc");
+        const size_t hpart = sizeof(cplx) * (FD_DOT_MAX * (size_t)G.ny * G.nz + 1);
+        fck(cudaMallocHost(&op->hpart, hpart), "alloc");
+        std::memset(static_cast<void *>(op->hpart), 0, hpart);
+        fck(cudaMalloc(&op->done, sizeof(unsigned)), "alloc");
+        fck(cudaMemset(op->done, 0, sizeof(unsigned)), "memset");
+        fck(cudaStreamSynchronize(0), "memset");
     } catch (const FdErr &e) {
         delete op;
         return fd_fail(e.code, e.msg);
@@ -535,42 +797,102 @@ int omx_fd_solve(omx_fdop *op, const double *j_vec, double *f_io, int transpose,
         fck(cudaMemcpyAsync(jv, j_vec, bytes, cudaMemcpyHostToDevice, op->s), "upload");
         fck(cudaMemcpyAsync(f_out, f_io, bytes, cudaMemcpyHostToDevice, op->s), "upload");
         cplx tau[9][9] = {}, gam[9] = {}, gam_p[9] = {}, gam_pp[9] = {}, sig[9] = {};
-        cplx rho0 = {1, 0}, rho1 = {1, 0}, alpha = {1, 0}, omega = {1, 0}, beta, dot;
+        cplx rho0 = {1, 0}, rho1 = {1, 0}, alpha = {1, 0}, omega = {1, 0}, beta, dot[FD_DOT_MAX];
+        const bool per = G.per[0] || G.per[1] || G.per[2];
+        FdPass P{};
+        auto begin = [&]() {
+            P.f = nullptr;
+            P.nlin = P.ndot = 0;
+            P.ghost = nullptr;
+        };
+        auto lin = [&](cplx *v1, const cplx *v2, cplx a, int mode) { P.lin[P.nlin++] = FdLin{v1, v2, a, mode}; };
+        auto dots = [&](const cplx *v1, const cplx *v2) {
+            P.da[P.ndot] = v1;
+            P.db[P.ndot++] = v2;
+        };
+        // A x with the ghosts of x refreshed by the pass that wrote x
+        auto apply = [&](const cplx *x, cplx *Ax) {
+            P.f = x;
+            P.Af = Ax;
+        };
         fd_apply_dev(op, f, Af);
         fck(cudaMemcpyAsync(r0, jv, bytes, cudaMemcpyDeviceToDevice, op->s), "copy");
-        fd_lin(op, r0, Af, cplx{-1.0, 0.0}, 0);                 // r0 = j - A f
+        begin();
+        lin(r0, Af, cplx{-1.0, 0.0}, 0);                        // r0 = j - A f
+        dots(r0, r0);
+        dots(jv, jv);
+        fd_pass(op, P, dot);
         fck(cudaMemcpyAsync(r[0], r0, bytes, cudaMemcpyDeviceToDevice, op->s), "copy");
-        dot = fd_dot(op, r0, r0);
-        double norm_t = std::sqrt(dot.re);
-        fd_lin(op, r0, nullptr, cplx{1.0 / norm_t, 0.0}, 2);    // r0 = r0 / |r0|
-        dot = fd_dot(op, jv, jv);
-        norm_t = std::sqrt(dot.re);
+        double norm_t = std::sqrt(dot[0].re);
+        const double norm_j = std::sqrt(dot[1].re);
+        begin();
+        lin(r0, nullptr, cplx{1.0 / norm_t, 0.0}, 2);           // r0 = r0 / |r0|
+        dots(r0, r[0]);                                         // the first iteration's rho1
+        cplx next_rho = {0, 0};
+        fd_pass(op, P, dot);
+        next_rho = dot[0];
+        norm_t = norm_j;
         double err_r = 1.0;
         int n = 0, conv = 0;
+        // each pass ends with every dot product that its vectors already allow: (r0, r[l]) after the
+        // application that makes r[l], the first minimal-residual products after the last one, the
+        // next iteration's (r0, r[0]) with the residual norm
         while (n <= n_max && !conv) {
             rho0 = cmul(cscale(omega, -1.0), rho0);
             for (int l = 0; l <= L - 1; ++l) {
-                dot = fd_dot(op, r0, r[l]);
-                rho1 = dot;
+                rho1 = next_rho;
                 beta = cdiv(cmul(alpha, rho1), rho0);
                 rho0 = rho1;
-                for (int i = 0; i <= l; ++i) fd_lin(op, u[i], r[i], cscale(beta, -1.0), 1);
-                fd_apply_dev(op, u[l], u[l + 1]);
-                dot = fd_dot(op, r0, u[l + 1]);
-                alpha = cdiv(rho0, dot);
-                for (int i = 0; i <= l; ++i) fd_lin(op, r[i], u[i + 1], cscale(alpha, -1.0), 0);
-                fd_apply_dev(op, r[l], r[l + 1]);
-                fd_lin(op, f_out, u[0], alpha, 0);
-            }
-            for (int l = 1; l <= L; ++l) {
-                for (int i = 1; i <= l - 1; ++i) {
-                    dot = fd_dot(op, r[i], r[l]);
-                    tau[i][l] = cdiv(dot, sig[i]);
-                    fd_lin(op, r[l], r[i], cscale(tau[i][l], -1.0), 0);
+                begin();
+                for (int i = 0; i <= l; ++i) lin(u[i], r[i], cscale(beta, -1.0), 1);
+                if (per) P.ghost = u[l];
+                fd_pass(op, P);
+                begin();
+                apply(u[l], u[l + 1]);
+                dots(r0, u[l + 1]);
+                fd_pass(op, P, dot);
+                alpha = cdiv(rho0, dot[0]);
+                begin();
+                for (int i = 0; i <= l; ++i) lin(r[i], u[i + 1], cscale(alpha, -1.0), 0);
+                lin(f_out, u[0], alpha, 0);
+                if (per) P.ghost = r[l];
+                fd_pass(op, P);
+                begin();
+                apply(r[l], r[l + 1]);
+                if (l < L - 1) {
+                    dots(r0, r[l + 1]);
+                    fd_pass(op, P, dot);
+                    next_rho = dot[0];
                 }
-                sig[l] = fd_dot(op, r[l], r[l]);
-                dot = fd_dot(op, r[l], r[0]);
-                gam_p[l] = cdiv(dot, sig[l]);
+            }
+            // the last application's pass takes the minimal-residual part's first products along
+            for (int l = 1; l <= L; ++l) {
+                if (l == 1) {
+                    dots(r[1], r[1]);
+                    dots(r[1], r[0]);
+                    if (L > 1) dots(r[1], r[2]);
+                    fd_pass(op, P, dot);
+                    sig[1] = dot[0];
+                    gam_p[1] = cdiv(dot[1], sig[1]);
+                    if (L > 1) dot[0] = dot[2];
+                    continue;
+                }
+                for (int i = 1; i <= l - 1; ++i) {              // dot[0] = (r[i], r[l])
+                    tau[i][l] = cdiv(dot[0], sig[i]);
+                    begin();
+                    lin(r[l], r[i], cscale(tau[i][l], -1.0), 0);
+                    if (i < l - 1) {
+                        dots(r[i + 1], r[l]);
+                    } else {
+                        dots(r[l], r[l]);
+                        dots(r[l], r[0]);
+                        if (l < L) dots(r[1], r[l + 1]);
+                    }
+                    fd_pass(op, P, dot);
+                }
+                sig[l] = dot[0];
+                gam_p[l] = cdiv(dot[1], sig[l]);
+                if (l < L) dot[0] = dot[2];
             }
             gam[L] = gam_p[L];
             omega = gam[L];
@@ -582,16 +904,20 @@ int omx_fd_solve(omx_fdop *op, const double *j_vec, double *f_io, int transpose,
                 gam_pp[l] = gam[l + 1];
                 for (int i = l + 1; i <= L - 1; ++i) gam_pp[l] = cadd(gam_pp[l], cmul(tau[l][i], gam[i + 1]));
             }
-            fd_lin(op, f_out, r[0], gam[1], 0);
-            fd_lin(op, r[0], r[L], cscale(gam_p[L], -1.0), 0);
-            fd_lin(op, u[0], u[L], cscale(gam[L], -1.0), 0);
+            begin();
+            lin(f_out, r[0], gam[1], 0);
+            lin(r[0], r[L], cscale(gam_p[L], -1.0), 0);
+            lin(u[0], u[L], cscale(gam[L], -1.0), 0);
             for (int l = 1; l <= L - 1; ++l) {
-                fd_lin(op, u[0], u[l], cscale(gam[l], -1.0), 0);
-                fd_lin(op, f_out, r[l], gam_pp[l], 0);
-                fd_lin(op, r[0], r[l], cscale(gam_p[l], -1.0), 0);
+                lin(u[0], u[l], cscale(gam[l], -1.0), 0);
+                lin(f_out, r[l], gam_pp[l], 0);
+                lin(r[0], r[l], cscale(gam_p[l], -1.0), 0);
             }
-            dot = fd_dot(op, r[0], r[0]);
-            err_r = std::sqrt(dot.re);
+            dots(r[0], r[0]);
+            dots(r0, r[0]);
+            fd_pass(op, P, dot);
+            next_rho = dot[1];
+            err_r = std::sqrt(dot[0].re);
             n = n + 1;
             if (err_r <= tol * norm_t) conv = 1;
         }

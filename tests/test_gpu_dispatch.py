@@ -129,3 +129,146 @@ def test_emitter_forms_bit_identical(orc, model, n):
         assert np.array_equal(a["dPt_dt"], (dip - before["dipole"]) / dt)
         before = a
     gpu.kill()
+
+
+def bicgstab_rows(O, own, j, f0, L, its):
+    """BiCGStab(L) (bicgstab_mod.f90:76-243) with the oracle's operator, FP64 operations written out,
+    and the dot products in the library's order: per row of cells, 128 interleaved sums (components
+    outermost) halved together, then the rows one after the other.  Returns (f, |r| / |j|)."""
+    def mul(a, v):                                           # complex a times a vector (re, im)
+        return a[0] * v[0] - a[1] * v[1], a[0] * v[1] + a[1] * v[0]
+
+    def cmul(a, b):
+        return a[0] * b[0] - a[1] * b[1], a[0] * b[1] + a[1] * b[0]
+
+    def cdiv(a, b):
+        if abs(b[0]) < abs(b[1]):
+            t = b[0] / b[1]
+            d = b[0] * t + b[1]
+            return (a[0] * t + a[1]) / d, (a[1] * t - a[0]) / d
+        t = b[1] / b[0]
+        d = b[1] * t + b[0]
+        return (a[1] * t + a[0]) / d, (a[1] - a[0] * t) / d
+
+    def neg(a):
+        return a[0] * -1.0, a[1] * -1.0
+
+    def axpy(v, w, a):                                       # v + a w
+        m = mul(a, w)
+        return v[0] + m[0], v[1] + m[1]
+
+    def dot(a, b):
+        re = a[0] * b[0] - (-a[1]) * b[1]
+        im = a[0] * b[1] + (-a[1]) * b[0]
+        tot = []
+        for p in (re, im):
+            nx = p.shape[-1]
+            q = np.zeros((p.shape[0], p[0].size // nx, -(-nx // 128) * 128))
+            q[:, :, :nx] = p.reshape(p.shape[0], -1, nx)
+            s = np.zeros((q.shape[1], 128))
+            for c in range(q.shape[0]):
+                for x in range(0, q.shape[2], 128):
+                    s = s + q[c, :, x:x + 128]
+            o = 64
+            while o:
+                s = s[:, :o] + s[:, o:2 * o]
+                o //= 2
+            t = 0.0
+            for v in s[:, 0]:
+                t = t + float(v)
+            tot.append(t)
+        return tuple(tot)
+
+    def A(v):
+        x = np.zeros(j.shape, complex)
+        x[own].real, x[own].imag = v
+        y = O.apply(x)[own]
+        return y.real.copy(), y.imag.copy()
+
+    split = lambda v: (v[own].real.copy(), v[own].imag.copy())  # noqa: E731
+    jv, x = split(j), split(f0)
+    r0 = axpy(jv, A(x), (-1.0, 0.0))
+    zero = (np.zeros_like(jv[0]), np.zeros_like(jv[0]))
+    r, u = [r0] + [zero] * L, [zero] * (L + 1)
+    r0 = mul((1.0 / np.sqrt(dot(r0, r0)[0]), 0.0), r0)
+    nj = np.sqrt(dot(jv, jv)[0])
+    rho0, alpha, omega = (1.0, 0.0), (1.0, 0.0), (1.0, 0.0)
+    for _ in range(its):
+        rho0 = cmul(neg(omega), rho0)
+        for q in range(L):
+            rho1 = dot(r0, r[q])
+            beta = neg(cdiv(cmul(alpha, rho1), rho0))
+            rho0 = rho1
+            for i in range(q + 1):
+                m = mul(beta, u[i])
+                u[i] = (m[0] + r[i][0], m[1] + r[i][1])
+            u[q + 1] = A(u[q])
+            alpha = cdiv(rho0, dot(r0, u[q + 1]))
+            for i in range(q + 1):
+                r[i] = axpy(r[i], u[i + 1], neg(alpha))
+            r[q + 1] = A(r[q])
+            x = axpy(x, u[0], alpha)
+        tau, sig, gp = {}, [None] * (L + 1), [None] * (L + 1)
+        for q in range(1, L + 1):
+            for i in range(1, q):
+                tau[i, q] = cdiv(dot(r[i], r[q]), sig[i])
+                r[q] = axpy(r[q], r[i], neg(tau[i, q]))
+            sig[q] = dot(r[q], r[q])
+            gp[q] = cdiv(dot(r[q], r[0]), sig[q])
+        gam = gp[:]
+        omega = gam[L]
+        for q in range(L - 1, 0, -1):
+            for i in range(q + 1, L + 1):
+                m = cmul(tau[q, i], gam[i])
+                gam[q] = (gam[q][0] - m[0], gam[q][1] - m[1])
+        gpp = [None] * (L + 1)
+        for q in range(1, L):
+            gpp[q] = gam[q + 1]
+            for i in range(q + 1, L):
+                m = cmul(tau[q, i], gam[i + 1])
+                gpp[q] = (gpp[q][0] + m[0], gpp[q][1] + m[1])
+        x = axpy(x, r[0], gam[1])
+        r[0] = axpy(r[0], r[L], neg(gp[L]))
+        u[0] = axpy(u[0], u[L], neg(gam[L]))
+        for q in range(1, L):
+            u[0] = axpy(u[0], u[q], neg(gam[q]))
+            x = axpy(x, r[q], gpp[q])
+            r[0] = axpy(r[0], r[q], neg(gp[q]))
+        err = np.sqrt(dot(r[0], r[0])[0])
+    return x[0] + 1j * x[1], err / nj
+
+
+# row lengths at the edges of the thread groups per row (32, 64, 128) and of the split of long rows
+# (256); every stencil order; PML, periodic and closed faces
+@pytest.mark.parametrize("n,n_der,bnd", [
+    ((32, 5, 4), 1, (2, 2, 2)), ((33, 6, 7), 2, (3, 2, 1)), ((64, 4, 5), 3, (1, 2, 2)), ((65, 8, 8), 4, (2, 2, 2)),
+    ((128, 9), 2, (3, 2)), ((129, 7), 1, (2, 2)), ((256, 6), 3, (2, 3)), ((257, 5), 2, (2, 2)), ((300, 9), 4, (3, 2)),
+    ((31,), 2, (2,)), ((257,), 4, (3,)),
+])
+def test_fd_rows(orc, n, n_der, bnd):
+    """The solver's fused passes against the oracle: the operator bit for bit, infinities and NaN
+    included; two iterations of the solver bit for bit against the same recursion."""
+    rng = np.random.default_rng(sum(n) + n_der)
+    eps = 1.0 + 1.25 * (rng.random(n) < 0.4) + 0.3j
+    G = omx.FDOperator(n, 2, n_der, bnd, 0.25, 1.3, eps)
+    O = orc.FDOperator(n, 2, n_der, bnd, 0.25, 1.3, eps)
+    own = (slice(None),) + tuple(slice(n_der, n_der + m) for m in reversed(n))
+    f = G.zeros()
+    f[own] = rng.normal(size=f[own].shape) + 1j * rng.normal(size=f[own].shape)
+    for transpose in (False, True):
+        assert np.array_equal(G.apply(f, transpose)[own], O.apply(f, transpose)[own])
+    bad = f.copy()
+    flat = bad[own].reshape(-1).copy()
+    for q, v in zip(rng.choice(flat.size, 4, replace=False), (np.inf, -np.inf, np.nan, 1e308)):
+        flat[q] = v + 1j * flat[q].imag
+    bad[own] = flat.reshape(bad[own].shape)
+    with np.errstate(all="ignore"):
+        assert np.array_equal(G.apply(bad)[own], O.apply(bad)[own], equal_nan=True)
+    j = G.zeros()
+    j[own] = rng.normal(size=j[own].shape)
+    for L in (1, 2, 3):
+        got, _, err, its = G.solve(j, f, 1e-30, 1, L)        # two outer iterations
+        want, werr = bicgstab_rows(O, own, j, f, L, 2)
+        assert its == 2 and err == werr
+        assert np.array_equal(got[own], want)
+    G.kill()
