@@ -436,7 +436,9 @@ def measure(args, dist, config, grid, K, W, err_steps, cpu_seconds):
     if per["H"]["launches"] == 0:      # one fused pass per step
         per["fused_HE"] = per.pop("E")
         per.pop("H")
-        dom, kernel_name = "fused_HE", ("k_fused3_tma<TY, LEAN_ONLY> + k_f3g_h / k_f3g_e (3D H+E step in one "
+        dom, kernel_name = "fused_HE", ("k_f3p_h + k_f3p_e (3D H and E passes in place)"
+                                        if dims == 3 and shape is not None and shape < 1000 else
+                                        "k_fused3_tma<TY, LEAN_ONLY> + k_f3g_h / k_f3g_e (3D H+E step in one "
                                         "pass split by plane form, lean planes staged by TMA)"
                                         if dims == 3 else
                                         "k_fused_tmz_ws (H+E step in one pass; form from omx_autotune)")
@@ -535,8 +537,8 @@ def measure(args, dist, config, grid, K, W, err_steps, cpu_seconds):
     elif dims == 2:
         shape_desc = "fused-kernel form %d (omx_autotune)" % shape
     elif dims == 3:
-        shape_desc = "two half-step passes, %d planes marched per thread (omx_autotune: faster than the " \
-                     "fused pass at this size)" % shape
+        shape_desc = "two half-step passes in place, %d planes marched per thread (omx_autotune: faster than the " \
+                     "staged pass at this size)" % shape
     else:
         shape_desc = "planes marched per thread %d (omx_autotune)" % shape
     return {

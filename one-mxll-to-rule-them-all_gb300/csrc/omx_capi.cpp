@@ -221,7 +221,6 @@ struct omx_ctx {
     // and the fused-kernel form (-1 = default)
     int march = 0;
     int fused_form = -1;
-    int march_two_pass = 0;   // autotune: the two-pass candidate of a 3D FP32 fused-eligible grid is selected
     int tq_step_old = 0;
     double t_skip = 0.0;
     // run tables
@@ -303,6 +302,13 @@ struct omx_ctx {
     bool post_ok = false;       // the work after the fused pass goes in one launch (post_eligible)
     bool plane_fold = false;    // the 3D bulk E pass adds the plane source (plane_fold_eligible)
     bool fold3 = false;         // the fused 3D pass adds the single plane source (fold3_of)
+    // the fused 3D step runs in place (k_f3p_h / k_f3p_e) instead of through the staged pass: the rule's
+    // choice (prepare), or pinned by a launch shape (0: the rule, 1: in place, 2: staged; a batch needs
+    // the staged pass's buffers)
+    bool f3_inplace = false;
+    int f3_pin = 0;
+    bool taps_h = false;        // some detector samples an H component
+    bool side_wait = false;     // graph capture: the in-place step waits for ev_join where it must
     F3tMaps f3maps[2][2];       // tensor maps of the fused 3D pass: [in set][tile rows 8 / 16]
     const void *f3key[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};   // Ex buffer they were made for
     // runs {bx, by, k0, k1} of the fused 3D pass (general runs first, then lean ones), one list per
@@ -1006,6 +1012,31 @@ bool plane_fold_eligible(const omx_ctx *c)
 
 void f3t_plan(omx_ctx *c);
 
+// the other buffer set of a pass that reads one set and writes the other
+void second_set(omx_ctx *c)
+{
+    if (c->ff2[2].p) return;
+    for (int q = 0; q < 6; ++q)
+        if (c->field_used[q]) c->ff2[q].alloc(c->felems);
+    for (int a = 0; a < 3; ++a)
+        for (int q = 0; q < 2; ++q)
+            if (c->psif[a][1][q].p) c->psiH2[a][q].alloc(c->psif[a][1][q].n);
+    c->epoch++;
+}
+
+// In place or staged, for a grid that the fused 3D pass can step: in place up to F3_INPLACE_MOST
+// cells.  Measured, us per step with a gold sphere and 10-cell CPML on every face, in place / staged
+// (default shapes): 32^3 7.9 / 25.4, 64^3 10.8 / 27.4, 96^3 22.0 / 62.8, 128^3 44.4 / 99.4, 160^3
+// 104 / 139, 192^3 171 / 175, 224^3 257 / 236, 256^3 362 / 321.
+constexpr long long F3_INPLACE_MOST = 7000000;
+bool f3_inplace_rule(const omx_ctx *c)
+{
+    if (c->dims != 3) return false;
+    if (c->f3_pin) return c->f3_pin == 1;
+    if (c->step_form != OMX_STEP_DEFAULT) return false;
+    return (long long)c->n[0] * c->n[1] * c->n[2] <= F3_INPLACE_MOST;
+}
+
 void prepare(omx_ctx *c)
 {
     const bool recheck = c->j_dirty || c->fused_dirty;
@@ -1015,22 +1046,18 @@ void prepare(omx_ctx *c)
     c->started = true;
     if (c->fused_dirty) {
         c->fused_ok = fused_eligible(c);
+        c->f3_inplace = c->fused_ok && f3_inplace_rule(c);
         c->fused_dirty = false;
     }
+    c->taps_h = false;
+    for (int f : c->tap_field) c->taps_h = c->taps_h || f >= 3;
     if (recheck) {
         c->post_ok = post_eligible(c);
         c->plane_fold = plane_fold_eligible(c);
         c->fold3 = c->fused_ok && fold3_of(c);
     }
-    if (c->fused_ok && c->fp32 && c->dims == 3) f3t_plan(c);
-    if (c->fused_ok && !c->ff2[2].p) {
-        for (int q = 0; q < 6; ++q)
-            if (c->field_used[q]) c->ff2[q].alloc(c->felems);
-        for (int a = 0; a < 3; ++a)
-            for (int q = 0; q < 2; ++q)
-                if (c->psif[a][1][q].p) c->psiH2[a][q].alloc(c->psif[a][1][q].n);
-        c->epoch++;
-    }
+    if (c->fused_ok && c->fp32 && c->dims == 3 && !c->f3_inplace) f3t_plan(c);
+    if (c->fused_ok && !c->f3_inplace) second_set(c);
 }
 
 StepParam imm(double v) { return StepParam{v, nullptr, nullptr, 0}; }
@@ -1321,6 +1348,7 @@ void f3t_plan(omx_ctx *c)
 // the dispersive cells (ade); 3D: the dispersive cells are inside the pass, and so is the single
 // plane source when fold3 holds (`plane`: its amplitude).  The caller adds the other sources and
 // the emitter current to the new set.
+void join_side_kernels(omx_ctx *c);
 template <class R> void fused_step(omx_ctx *c, bool ade = true, const StepParam *plane = nullptr);
 template <> void fused_step<double>(omx_ctx *, bool, const StepParam *) {}
 template <> void fused_step<float>(omx_ctx *c, bool ade, const StepParam *plane)
@@ -1329,6 +1357,33 @@ template <> void fused_step<float>(omx_ctx *c, bool ade, const StepParam *plane)
     const int in = c->cur, out = 1 - c->cur;
     const FieldPtrs<float> Fin = field_ptrs<float>(c, in), Fout = field_ptrs<float>(c, out);
     GridArgs<float> G = grid_args<float>(c);
+    if (c->dims == 3 && c->f3_inplace) {
+        // H overwrites what the previous step's side work may sample, E what its emitters gather
+        auto wait_side = [&]() {
+            if (c->side_wait) ck(cudaStreamWaitEvent(c->stream, c->ev_join, 0), "wait");
+            else join_side_kernels(c);
+        };
+        Fused3Args A;
+        A.in = A.out = Fin;
+        for (int a = 0; a < 3; ++a)
+            for (int q = 0; q < 2; ++q) A.psiH_out[a][q] = G.psiH[a][q];
+        if (c->taps_h) wait_side();
+        ck(launch_fused3p(A, G, c->march, false, c->stream), "3D launch");
+        if (!c->taps_h) wait_side();
+        G.step_inc = nullptr;
+        if (c->fold3 && plane) {
+            const SourceRec &S = *c->sources[0];
+            G.pl_on = 1;
+            G.pl_comp = S.pd.comp - 1;
+            G.pl_axis = S.pd.plane_axis - 1;
+            G.pl_index = S.pd.plane_index;
+            G.pl_c_src = S.c_src;
+            G.pl_amp = *plane;
+        }
+        ck(launch_fused3p(A, G, c->march, true, c->stream), "3D launch");
+        c->launches += 2;
+        return;
+    }
     if (c->dims == 3) {
         Fused3Args A;
         A.in = Fin;
@@ -1633,7 +1688,11 @@ template <class R> void run_impl(omx_ctx *c, int tt0, int nsteps, int n_skip, in
     }
     struct Reset {
         omx_ctx *c;
-        ~Reset() { c->run_step = nullptr; }
+        ~Reset()
+        {
+            c->run_step = nullptr;
+            c->side_wait = false;
+        }
     } reset{c};
     const int W = plan.W;
     const bool has_det = plan.has_det;
@@ -1726,6 +1785,7 @@ template <class R> void run_impl(omx_ctx *c, int tt0, int nsteps, int n_skip, in
     // the wait on the scatter also orders it before the pass that overwrites its buffer set.
     // Same operations on the same values as one_step: results are identical.
     auto overlapped_step = [&](bool wait_prev) {
+        c->side_wait = wait_prev;     // the in-place 3D step waits inside, between its passes
         if (post) {
             fused_step<R>(c, false, pl3);
             if (wait_prev) ck(cudaStreamWaitEvent(c->stream, c->ev_join, 0), "wait");
@@ -1736,6 +1796,7 @@ template <class R> void run_impl(omx_ctx *c, int tt0, int nsteps, int n_skip, in
             if (wait_prev) ck(cudaStreamWaitEvent(c->stream, c->ev_join, 0), "wait");
             do_inject<R>(c, P(0), P(1));
         }
+        c->side_wait = false;
         ck(cudaEventRecord(c->ev_fork, c->stream), "fork");
         ck(cudaStreamWaitEvent(c->side, c->ev_fork, 0), "fork");
         std::swap(c->stream, c->side);
@@ -1852,18 +1913,20 @@ template <class R> void run_impl(omx_ctx *c, int tt0, int nsteps, int n_skip, in
 void apply_shape(omx_ctx *c, int v)
 {
     const bool fused = c->fp32 && fused_eligible(c);
-    c->march_two_pass = 0;
+    c->f3_pin = 0;
     if (v >= 1000) {
         c->fused_form = v / 1000;
         c->march = v % 1000;
+        c->f3_pin = 2;
     } else if (fused && c->dims == 3) {
-        c->march = v;                 // the two half-step passes, v planes per thread
-        c->march_two_pass = 1;
+        c->march = v;                 // in place through the two plain passes, v planes per thread
+        c->f3_pin = 1;
     } else if (fused) {
         c->fused_form = v;
     } else {
         c->march = v;
     }
+    c->f3_inplace = fused && f3_inplace_rule(c);
 }
 
 constexpr int AUTOTUNE_STEPS = 4;   // steps timed back to back per candidate and round
@@ -1874,10 +1937,11 @@ constexpr int AUTOTUNE_STEPS = 4;   // steps timed back to back per candidate an
 template <class R> int autotune_impl(omx_ctx *c, int reps)
 {
     const bool fused = std::is_same<R, float>::value && c->fused_ok;
-    // 3D FP32 with the fused pass eligible: the two half-step passes compete too (shapes below
-    // 1000: planes marched per thread); where their in-place buffers fit in L2 (small grids) they
-    // can beat the single pass, whose ping-pong sets take twice the room
+    // 3D FP32 with the fused pass eligible: the two half-step passes in place compete too (shapes
+    // below 1000: planes marched per thread); where their one buffer set fits in L2 (small grids)
+    // they can beat the staged pass, whose ping-pong sets take twice the room
     const bool both = fused && c->dims == 3 && c->step_form == OMX_STEP_DEFAULT;
+    if (fused) second_set(c);
     std::vector<int> cand;
     if (fused && c->dims == 3) {
         // fused 3D pass: (ring depth x 100 + tile rows) x 1000 + planes per block
@@ -1890,7 +1954,7 @@ template <class R> int autotune_impl(omx_ctx *c, int reps)
                     if (kch <= c->n[2] * 2 && f3t_smem_bytes(ring * 100 + ty) <= optin)
                         cand.push_back((ring * 100 + ty) * 1000 + kch);
         if (both)
-            for (int m : {1, 2, 4, 8, 16, 32}) cand.push_back(m);
+            for (int m : {1, 2, 4, 8, 16}) cand.push_back(m);
     } else if (fused) {
         cand = {0, 4, 5, 6, 8, 14, 15, 16, 24, 25, 34, 36, 44, 45};
     } else if (c->dims == 3) {
@@ -1902,7 +1966,7 @@ template <class R> int autotune_impl(omx_ctx *c, int reps)
     }
     auto select = [&](int v) { apply_shape(c, v); };
     auto once = [&]() {
-        if (fused && c->march_two_pass == 0) {
+        if (fused) {
             fused_step<R>(c);
         } else {
             do_H<R>(c);
@@ -1951,14 +2015,6 @@ template <class R> int autotune_impl(omx_ctx *c, int reps)
     }
     select(pick);
     ck(cudaPeekAtLastError(), "autotune");
-    if (both && pick < 1000) {
-        // the two half-step passes won: the grid steps with them from now on
-        c->step_form = OMX_STEP_TWO_PASS;
-        c->fused_dirty = true;
-        c->march_two_pass = 0;
-        c->march = pick;
-        prepare(c);
-    }
     return pick;
 }
 
@@ -3198,10 +3254,8 @@ int omx_set_launch_shape(omx_ctx *c, int shape)
     join_side(c);
     req(c && shape >= 1, "bad argument");
     if (c->dims == 3 && c->fp32 && fused_eligible(c) && shape < 1000) {
-        // 3D FP32: a shape below 1000 selects the two half-step passes (v planes per thread)
-        c->step_form = OMX_STEP_TWO_PASS;
+        // 3D FP32: a shape below 1000 selects the two half-step passes in place (that many planes per thread)
         c->fused_dirty = true;
-        c->march = shape;
     } else if (c->dims == 3 && c->fp32 && fused_eligible(c)) {
         const int form = shape / 1000, rows = form % 100, ring = form / 100;
         req((rows == 8 || rows == 16) && (ring == 0 || (ring >= 2 && ring <= F3T_RING_MAX)) && shape % 1000 >= 1 &&
@@ -3857,6 +3911,12 @@ void batch_decide(omx_batch *b)
     bool all = b->fp32;
     for (auto *c : b->ctx) all = all && fused_eligible(c);
     b->fused = all ? 1 : 0;
+    if (all)
+        for (auto *c : b->ctx) {
+            c->f3_pin = 2;             // the batched pass reads one buffer set and writes the other
+            c->fused_dirty = true;
+            c->epoch++;
+        }
     if (!all)
         for (auto *c : b->ctx) {
             c->step_form = OMX_STEP_TWO_PASS;
@@ -4086,7 +4146,10 @@ int omx_algorithmic_bytes(const omx_ctx *c, int kc, double *bytes)
         ade_bytes = (double)drude * 2.0 * w + (double)dl * (2.0 + 2.0 + 4.0 * c->P) * w;
     }
     const bool fused = c->fused_ok;   // FP32 fused (2D TMz, 3D): one pass per step (class KC_E)
-    if (kc == KC_H) {
+    if (fused && c->f3_inplace) {     // both half-step passes counted as one launch of class KC_E
+        b = kc != KC_E ? 0.0 : cells * w * 3.0 * (ncomp_e + ncomp_h) + (psi_cells_h + psi_cells_e) * 2.0 * w +
+                                   (double)c->bbV * ncomp_e + ade_bytes;
+    } else if (kc == KC_H) {
         b = fused ? 0.0 : cells * w * (ncomp_e + 2.0 * ncomp_h) + psi_cells_h * 2.0 * w;
     } else if (kc == KC_E) {
         if (fused)   // each field word read once and written once

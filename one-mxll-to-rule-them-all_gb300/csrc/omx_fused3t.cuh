@@ -244,13 +244,17 @@ __device__ __forceinline__ void f3t_curl(float hx, float hy, float hz, float hz_
 // ADE) or the vacuum update, then the CPML E psi of the x, y and z faces in the reference's order
 // (mxll_3D_mod.f90:740-921).  pe0, pe1, pe2: the cell's E psi indices (-1: no slab; in place: each
 // word is read and written by this thread only, all of them requested first); bz, cz: the z
-// face's coefficients of plane k; bbc: (i, j) lies in the media box's x-y extent.
-__device__ __forceinline__ void f3t_e_general(float &ex, float &ey, float &ez, float rx, float ry, float rz, float dhxk,
+// face's coefficients of plane k; bbc: (i, j) lies in the media box's x-y extent.  ADE_LIST: the
+// launch updates the dispersive component-cells through their list (f3p_ade_cell): they are left
+// alone here, psi included, and returned as bits (1 Ex, 2 Ey, 4 Ez).
+template <bool ADE_LIST = false>
+__device__ __forceinline__ int f3t_e_general(float &ex, float &ey, float &ez, float rx, float ry, float rz, float dhxk,
                                               float dhyk, float hx, float hy, float hz, float hz_im, float hy_im,
                                               float hz_jm, float hx_jm, int i, int j, int k, int pe0, int pe1, int pe2,
                                               float bz, float cz, bool bbc, float dt_eps0, const GridArgs<float> &G)
 {
     float qe[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    int skip = 0;
     if (pe0 >= 0) {
         qe[0] = __ldg(G.psiE[0][0] + pe0);
         qe[1] = __ldg(G.psiE[0][1] + pe0);
@@ -275,9 +279,17 @@ __device__ __forceinline__ void f3t_e_general(float &ex, float &ey, float &ez, f
     }
     if (bbc && k >= G.bb0[2] && k <= G.bb1[2]) {
         const int b = (i - G.bb0[0]) + G.bbd[0] * ((j - G.bb0[1]) + G.bbd[1] * (k - G.bb0[2]));
-        ex = f3t_media(ex, rx, 0, b, G);
-        ey = f3t_media(ey, ry, 1, b, G);
-        ez = f3t_media(ez, rz, 2, b, G);
+        if constexpr (ADE_LIST) {
+            const ClsR<float> cx = G.cls[G.mat[0][b]], cy = G.cls[G.mat[1][b]], cz = G.cls[G.mat[2][b]];
+            ex = __fmaf_rn(cx.coef, rx, ex);
+            ey = __fmaf_rn(cy.coef, ry, ey);
+            ez = __fmaf_rn(cz.coef, rz, ez);
+            skip = (cx.type != CLS_PLAIN ? 1 : 0) | (cy.type != CLS_PLAIN ? 2 : 0) | (cz.type != CLS_PLAIN ? 4 : 0);
+        } else {
+            ex = f3t_media(ex, rx, 0, b, G);
+            ey = f3t_media(ey, ry, 1, b, G);
+            ez = f3t_media(ez, rz, 2, b, G);
+        }
     } else {
         ex = __fmaf_rn(dt_eps0, rx, ex);
         ey = __fmaf_rn(dt_eps0, ry, ey);
@@ -287,8 +299,8 @@ __device__ __forceinline__ void f3t_e_general(float &ex, float &ey, float &ez, f
         const float b = __ldg(G.bE[0] + i), c = __ldg(G.cE[0] + i);
         const float v0 = f3t_psi(b, qe[0], c, __fsub_rn(hz_im, hz));
         const float v1 = f3t_psi(b, qe[1], c, __fsub_rn(hy, hy_im));
-        G.psiE[0][0][pe0] = v0;
-        G.psiE[0][1][pe0] = v1;
+        if (!(skip & 2)) G.psiE[0][0][pe0] = v0;
+        if (!(skip & 4)) G.psiE[0][1][pe0] = v1;
         ey = __fmaf_rn(dt_eps0, v0, ey);
         ez = __fmaf_rn(dt_eps0, v1, ez);
     }
@@ -296,19 +308,20 @@ __device__ __forceinline__ void f3t_e_general(float &ex, float &ey, float &ez, f
         const float b = __ldg(G.bE[1] + j), c = __ldg(G.cE[1] + j);
         const float v0 = f3t_psi(b, qe[2], c, __fsub_rn(hz, hz_jm));
         const float v1 = f3t_psi(b, qe[3], c, __fsub_rn(hx_jm, hx));
-        G.psiE[1][0][pe1] = v0;
-        G.psiE[1][1][pe1] = v1;
+        if (!(skip & 1)) G.psiE[1][0][pe1] = v0;
+        if (!(skip & 4)) G.psiE[1][1][pe1] = v1;
         ex = __fmaf_rn(dt_eps0, v0, ex);
         ez = __fmaf_rn(dt_eps0, v1, ez);
     }
     if (pe2 >= 0) {   // :887-921
         const float v0 = f3t_psi(bz, qe[4], cz, dhyk);
         const float v1 = f3t_psi(bz, qe[5], cz, dhxk);
-        G.psiE[2][0][pe2] = v0;
-        G.psiE[2][1][pe2] = v1;
+        if (!(skip & 1)) G.psiE[2][0][pe2] = v0;
+        if (!(skip & 2)) G.psiE[2][1][pe2] = v1;
         ex = __fmaf_rn(dt_eps0, v0, ex);
         ey = __fmaf_rn(dt_eps0, v1, ey);
     }
+    return skip;
 }
 
 template <int TY> constexpr int f3t_min_blocks() { return 2; }
@@ -845,7 +858,7 @@ __device__ __forceinline__ void f3g_h_run(const Fused3Args &A, const GridArgs<fl
 // One general run's new E; then, when G.step_inc is set, the last of the nblk blocks of this
 // grid's launch advances the grid's device-loop step counter (this launch ends the pass and holds
 // its only reads of the step's scalars).
-template <int TY>
+template <int TY, bool ADE_LIST = false>
 __device__ __forceinline__ void f3g_e_run(const Fused3Args &A, const GridArgs<float> &G, int4 it, unsigned nblk)
 {
     const Lay &L = G.L;
@@ -874,12 +887,13 @@ __device__ __forceinline__ void f3g_e_run(const Fused3Args &A, const GridArgs<fl
             hxm = hx;
             hym = hy;
             float ex = __ldcs(A.in.f[0] + idx), ey = __ldcs(A.in.f[1] + idx), ez = __ldcs(A.in.f[2] + idx);
-            f3t_e_general(ex, ey, ez, rx, ry, rz, dhxk, dhyk, hx, hy, hz, hz_im, hy_im, hz_jm, hx_jm, i, j, k,
-                          bxE >= 0 ? bxE + sX * (k - 1) : -1, byE >= 0 ? byE + sY * (k - 1) : -1,
-                          lez >= 0 ? bz0 + sZ * lez : -1, __ldg(G.bE[2] + k), __ldg(G.cE[2] + k), bbc, dt_eps0, G);
-            __stcs(A.out.f[0] + idx, ex);
-            __stcs(A.out.f[1] + idx, ey);
-            __stcs(A.out.f[2] + idx, ez);
+            const int skip = f3t_e_general<ADE_LIST>(
+                ex, ey, ez, rx, ry, rz, dhxk, dhyk, hx, hy, hz, hz_im, hy_im, hz_jm, hx_jm, i, j, k,
+                bxE >= 0 ? bxE + sX * (k - 1) : -1, byE >= 0 ? byE + sY * (k - 1) : -1, lez >= 0 ? bz0 + sZ * lez : -1,
+                __ldg(G.bE[2] + k), __ldg(G.cE[2] + k), bbc, dt_eps0, G);
+            if (!ADE_LIST || !(skip & 1)) __stcs(A.out.f[0] + idx, ex);
+            if (!ADE_LIST || !(skip & 2)) __stcs(A.out.f[1] + idx, ey);
+            if (!ADE_LIST || !(skip & 4)) __stcs(A.out.f[2] + idx, ez);
         }
     }
     if (G.step_inc) {
@@ -905,6 +919,87 @@ template <int TY>
 __global__ void __launch_bounds__(32 * TY, 1536 / (32 * TY)) k_f3g_e(Fused3Args A, GridArgs<float> G, const int4 *__restrict__ items)
 {
     f3g_e_run<TY>(A, G, items[blockIdx.x], gridDim.x);
+}
+
+// The step in place: every column through the two plain kernels, new H and then new E over the old
+// values of the one buffer set (a cell's old H and E words are read by the thread that overwrites
+// them, and a half step's kernel writes nothing else that it reads).  Blocks of 32 x 4 columns
+// marching kch planes.  Grids that fit in L2 step faster this way than through the staged pass: half
+// the working set, and thousands of short blocks instead of a hundred that march their planes one
+// by one (f3_inplace_rule has both sides' times).  The H launch advances the device-loop step counter.
+__global__ void __launch_bounds__(128, 10) k_f3p_h(Fused3Args A, GridArgs<float> G, int kch)
+{
+    if (G.step_inc && blockIdx.x + blockIdx.y + blockIdx.z == 0 && threadIdx.x + threadIdx.y == 0) *G.step_inc += 1;
+    const int k0 = 1 + (int)blockIdx.z * kch;
+    f3g_h_run<4>(A, G, make_int4((1 + 32 * (int)blockIdx.x) | (32 << 20), (1 + 4 * (int)blockIdx.y) | (4 << 20), k0,
+                                 min(G.L.nz, k0 + kch - 1)));
+}
+// New E of one dispersive component-cell (entry q of the grid's list): f3t_e_general's terms of that
+// component.  A thread per entry: marched inside the plane loop, a column of gold cells is a chain
+// of state reads (a 128^3 grid with a sphere of 20 cells radius: 51 us per step at best that way,
+// 62 us at four planes a thread; 44 us with the list).
+__device__ __forceinline__ void f3p_ade_cell(const Fused3Args &A, const GridArgs<float> &G, int q)
+{
+    const Lay &L = G.L;
+    const int4 en = G.ade_ent[q];
+    const int b = G.ade_b[q], i = en.x, j = en.y, k = en.z, c = en.w;
+    const int px_ = L.px, pz_ = (int)L.pz, idx = (int)L.off + i + px_ * j + pz_ * k;
+    const float *__restrict__ Hx = A.out.f[3];
+    const float *__restrict__ Hy = A.out.f[4];
+    const float *__restrict__ Hz = A.out.f[5];
+    // the curl's two differences: d1 along the lower of the two transverse axes, d2 along the higher
+    const float dex = G.den_e[0][i], dey = G.den_e[1][j], dez = G.den_e[2][k];
+    float d1, d2, rot;
+    if (c == 0) {
+        d1 = __fsub_rn(Hz[idx], Hz[idx - px_]);
+        d2 = __fsub_rn(Hy[idx - pz_], Hy[idx]);
+        rot = __fmaf_rn(d2, dez, __fmul_rn(d1, dey));
+    } else if (c == 1) {
+        d1 = __fsub_rn(Hz[idx - 1], Hz[idx]);
+        d2 = __fsub_rn(Hx[idx], Hx[idx - pz_]);
+        rot = __fmaf_rn(d2, dez, __fmul_rn(d1, dex));
+    } else {
+        d1 = __fsub_rn(Hy[idx], Hy[idx - 1]);
+        d2 = __fsub_rn(Hx[idx - px_], Hx[idx]);
+        rot = __fmaf_rn(d2, dey, __fmul_rn(d1, dex));
+    }
+    float e = A.in.f[c][idx];
+    if (G.pl_on && c == G.pl_comp && (G.pl_axis == 0 ? i : (G.pl_axis == 1 ? j : k)) == G.pl_index) {
+        const double a = sp_get(G.pl_amp);
+        if (a != 0.0) e = (float)__dadd_rn((double)e, __dmul_rn(G.pl_c_src, a));
+    }
+    const ClsR<float> cl = G.cls[G.mat[c][b]];
+    e = f3t_ade(e, rot, cl.type, G.med + cl.medium, G.ade + (long long)c * (2 + 2 * G.P) * G.bbV + b, G.bbV, G.P);
+    // CPML of the two transverse axes, the lower first
+    const int at[3] = {i, j, k};
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const int a = c == 0 ? 1 + s : (c == 1 ? 2 * s : s);
+        const int l = G.lE[a][at[a]];
+        if (l < 0) continue;
+        const int p = a == 0 ? l + G.L2 * ((j - 1) + L.ny * (k - 1))
+                             : (a == 1 ? (i - 1) + L.nx * (l + G.L2 * (k - 1)) : (i - 1) + L.nx * ((j - 1) + L.ny * l));
+        // psi 0 belongs to the first of axis a's two components in (Ey, Ez), (Ex, Ez), (Ex, Ey)
+        float *psi = G.psiE[a][a == 0 ? (c == 1 ? 0 : 1) : (c == 0 ? 0 : 1)] + p;
+        const float v = f3t_psi(G.bE[a][at[a]], *psi, G.cE[a][at[a]], s == 0 ? d1 : d2);
+        *psi = v;
+        e = __fmaf_rn(G.dt_eps0, v, e);
+    }
+    A.out.f[c][idx] = e;
+}
+
+// zl: leading block layers along z that take the list of dispersive component-cells
+__global__ void __launch_bounds__(128, 9) k_f3p_e(Fused3Args A, GridArgs<float> G, int kch, int zl)
+{
+    if ((int)blockIdx.z < zl) {
+        const int q = 128 * (int)(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)) +
+                      (int)(threadIdx.x + 32 * threadIdx.y);
+        if (q < G.ade_n) f3p_ade_cell(A, G, q);
+        return;
+    }
+    const int k0 = 1 + ((int)blockIdx.z - zl) * kch;
+    f3g_e_run<4, true>(A, G, make_int4((1 + 32 * (int)blockIdx.x) | (32 << 20), (1 + 4 * (int)blockIdx.y) | (4 << 20), k0,
+                                       min(G.L.nz, k0 + kch - 1)), 0u);
 }
 
 // Batched general runs of several grids: items[b].w carries the run's grid (k1 | g << 20); the

@@ -242,6 +242,10 @@ cudaError_t launch_fused3t_lean(const F3tMaps &M, const Fused3Args &A, const Gri
 // advances the device-loop step counter when G.step_inc is set).
 cudaError_t launch_fused3t_general(const Fused3Args &A, const GridArgs<float> &G, int form, const int4 *items, int n,
                                    bool e_half, void *stream);
+// The step in place (A.in and A.out are one buffer set, A.psiH_out the set's own H psi): new H
+// (e_half = false; it advances the device-loop step counter when G.step_inc is set), then new E
+// (step_inc null).  kch: planes per thread, 0 for the default.
+cudaError_t launch_fused3p(const Fused3Args &A, const GridArgs<float> &G, int kch, bool e_half, void *stream);
 // The batched fused pass split by plane form: every grid's general runs through the two plain
 // kernels (new H, then new E after the lean runs) and every grid's lean runs in one launch; run
 // lists as the single-grid ones with the grid's table index in k1's high bits (k1 | g << 20).

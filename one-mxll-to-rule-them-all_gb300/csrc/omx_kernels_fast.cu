@@ -227,6 +227,23 @@ cudaError_t launch_fused3t_general(const Fused3Args &A, const GridArgs<float> &G
     return cudaGetLastError();
 }
 
+cudaError_t launch_fused3p(const Fused3Args &A, const GridArgs<float> &G, int kch, bool e_half, void *sv)
+{
+    const Lay &L = G.L;
+    const dim3 b(32, 4);
+    // us per step at marches of 1, 2, 4, 8: 48^3 8.6, 9.1, 11.8, 19; 96^3 23.6, 22.0, 24.2, 22.2; 128^3 51,
+    // 45.6, 44.4, 48.6; 160^3 123, 108, 104, 105
+    int m = kch > 0 ? kch : march_rule((long long)((L.nx + 31) / 32) * ((L.ny + 3) / 4), L.nz, 4, 22);
+    dim3 g((L.nx + 31) / 32, (L.ny + 3) / 4, (L.nz + m - 1) / m);
+    if (e_half) {
+        const unsigned layer = g.x * g.y * 128, zl = ((unsigned)G.ade_n + layer - 1) / layer;
+        for (; g.z + zl > 65535; m *= 2) g.z = (L.nz + 2 * m - 1) / (2 * m);
+        g.z += zl;
+        k_f3p_e<<<g, b, 0, (cudaStream_t)sv>>>(A, G, m, (int)zl);
+    } else k_f3p_h<<<g, b, 0, (cudaStream_t)sv>>>(A, G, m);
+    return cudaGetLastError();
+}
+
 int f3t_smem_bytes(int form)
 {
     return f3t_rows(form) == 16 ? F3tShape<16>::smem(f3t_ring(form)) : F3tShape<8>::smem(f3t_ring(form));

@@ -272,3 +272,48 @@ def test_fd_rows(orc, n, n_der, bnd):
         assert its == 2 and err == werr
         assert np.array_equal(got[own], want)
     G.kill()
+
+
+# tiles cut by every edge (32 x 4 columns in place, 32 x 8 staged), periodic z, single and several
+# sources, detectors of E only and of H
+@pytest.mark.parametrize("n,bnd,src,taps_h", [
+    ((40, 36, 28), (3, 3, 3), "plane", False), ((33, 29, 31), (3, 3, 3), "radial", True),
+    ((65, 30, 26), (3, 3, 2), "plane", True), ((31, 37, 40), (1, 3, 1), "both", False),
+])
+def test_inplace_and_staged_3d_steps_bit_identical(n, bnd, src, taps_h):
+    """The FP32 3D step in place (two plain passes) and staged, through graphs, single launches,
+    one-step calls and the per-call sequence: every field, record and emitter bit for bit."""
+    from test_gpu_parity import fused3_deck
+    from gpu_harness import step_loop
+    from omx import decks
+
+    deck = fused3_deck(n, bnd, src=src)
+    steps = 23
+    out = []
+    for shape, mode in ((8064, "graph"), (None, "graph"), (None, "plain"), (None, "one"), (None, "calls"),
+                        (1, "graph"), (4, "one"), (16, "graph")):
+        g = omx.TMxll(3, deck["grid_Ndims"], deck["npml"], deck["boundaries"], deck["dt"], deck["dr"],
+                      precision="fp32")
+        groups = decks.apply_deck(g, deck, omx, decks.media_map(deck, omx.media_map_from_voxels))
+        for det in deck["detectors"]:
+            g.add_detector(det["type"], det["field"], det["idx"])
+        if taps_h:
+            g.add_detector(omx.POINT, "Hy", np.array([[n[0] // 2, n[1] // 2, 12]]))
+        if shape:
+            g.set_launch_shape(shape)
+        if mode == "calls":
+            step_loop(g, deck, groups, 1, steps, {"tq_old": 0, "t_skip": 0.0},
+                      sample=lambda t: g.write_detectors_outputs(t))
+        elif mode == "one":
+            for tt in range(1, steps + 1):
+                g.run(tt, 1, deck["n_skip"], 1)
+        else:
+            g.run(1, steps, deck["n_skip"], 1, use_graph=mode == "graph")
+        out.append([g.drain_detectors()[1]] + [g.read_field(f) for f in range(1, 7)] +
+                   [q for gr in groups for q in (gr.read()["rho"], gr.read()["dipole"])])
+        g.kill()
+    assert np.max(np.abs(out[0][0])) > 0
+    for o in out[1:]:
+        assert len(o) == len(out[0])
+        for a, b in zip(o, out[0]):
+            assert np.array_equal(a, b)
