@@ -338,7 +338,8 @@ int omx_set_launch_shape(omx_ctx *ctx, int shape);
  * general runs' new H on a second stream beside one launch of their lean runs, then their general
  * runs' new E, the other grids' one launch on that second stream too), one
  * launch per round of the other sources, the per-grid emitter work and one launch for the
- * detectors of every grid.  Otherwise each step runs ONE persistent launch for the H pass of
+ * detectors of every grid; a batch of grids that all step in place by themselves runs them side by
+ * side on a few streams instead, each grid's launches as its own omx_run issues them.  Otherwise each step runs ONE persistent launch for the H pass of
  * every grid (its blocks walk a list of all grids' tiles), one launch per round of radial sources
  * (round r: source r of every grid), the dispersive cells, ONE launch for the bulk E pass of every
  * grid, the per-grid emitter work and the detectors.  use_graph != 0 captures that step once and
@@ -352,7 +353,8 @@ int omx_batch_create(omx_ctx *const *ctxs, int n, omx_batch **out);
  * per tile: 4, 8, 16 or 32) of the two half-step passes, or for the fused pass
  * s x 1000000 + (ring depth x 100 + tile rows) x 1000 + planes per block: the s largest grids step
  * with the pass split by plane form, the others in one launch over their tiles (s = 0: every grid
- * in that launch); ring depth 0 for the default of 4 planes. */
+ * in that launch); ring depth 0 for the default of 4 planes.  Grids that step side by side in place
+ * keep doing so when that is faster than every shape; *choice is the fastest shape then too. */
 int omx_batch_autotune(omx_batch *batch, int reps, int *choice);
 /* No counterpart in the reference: sets the launch shape of the batched passes, encoded as
  * omx_batch_autotune's choice (a fused shape when every member steps with the fused FP32 pass,

@@ -3337,6 +3337,12 @@ struct omx_batch {
     // H on `aux` beside their lean runs, then their E), the others in one k_fused3_batch launch
     // (on `aux` after that H)
     int f3nsplit = 0;
+    // small grids (batch_inplace_rule): each member steps in place by itself, its launches on one of
+    // the lanes, so that the grids fill the GPU together
+    bool f3inplace = false;
+    static constexpr int LANES = 12;
+    cudaStream_t lane[LANES] = {};
+    cudaEvent_t ev_lane[LANES] = {};
     cudaStream_t aux = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_mixed = nullptr;
     // tables and captured step graphs, kept while the key (each member's configuration epoch,
@@ -3645,6 +3651,64 @@ template <class R> long long batch_fused_pass(omx_batch *b, const BatchTables<R>
     return k;
 }
 
+// the lanes' streams and events (before any capture)
+void batch_lanes(omx_batch *b)
+{
+    for (int l = 0; l < std::min((int)b->ctx.size(), omx_batch::LANES); ++l) {
+        if (b->lane[l]) continue;
+        ck(cudaEventCreateWithFlags(&b->ev_lane[l], cudaEventDisableTiming), "event");
+        ck(cudaStreamCreateWithFlags(&b->lane[l], cudaStreamNonBlocking), "stream");
+    }
+}
+
+// `steps` steps of every member in place: member i's own launches (H, E, sources, emitter work,
+// detectors, as its omx_run issues them) on lane i mod LANES, forked from the batch's stream and
+// joined to it at the end; no member waits for another.  plans null: the field passes alone.
+template <class R> long long batch_inplace_steps(omx_batch *b, const std::vector<RunPlan> *plans, int steps)
+{
+    // four lanes when the members are large (fewer buffer sets share L2), else every lane.  us per
+    // step with 1, 2, 3, 4, 12 lanes: twelve grids of 0.70 M cells 338, 270, 260, 261, 274; 32 of 0.99 M
+    // 1126, 901, 897, 906, 935; twelve of 0.11 M 114, 73, 59, 53, 48; sixteen of 0.03 M 129, 79, 64, 50, 37
+    const int n = (int)b->ctx.size();
+    long long cells = 0;
+    for (const auto *c : b->ctx) cells += (long long)c->n[0] * c->n[1] * c->n[2];
+    const int lanes = std::min(n, cells / n >= 400000 ? 4 : omx_batch::LANES);
+    long long k = 0;
+    ck(cudaEventRecord(b->ev_fork, b->stream), "event");
+    for (int l = 0; l < lanes; ++l) ck(cudaStreamWaitEvent(b->lane[l], b->ev_fork, 0), "event");
+    struct Route {
+        omx_batch *b;
+        ~Route()
+        {
+            for (auto *c : b->ctx) c->stream = b->stream;
+        }
+    } route{b};
+    for (int i = 0; i < n; ++i) b->ctx[i]->stream = b->lane[i % lanes];
+    for (int s = 0; s < steps; ++s)
+        for (int i = 0; i < n; ++i) {
+            omx_ctx *c = b->ctx[i];
+            const long long before = c->launches;
+            if (!plans) {
+                fused_step<R>(c);
+            } else {
+                const RunPlan &P = (*plans)[i];
+                std::vector<StepParam> amps;
+                for (size_t q = 0; q < c->sources.size(); ++q) amps.push_back(plan_param(c, P, 4 + (int)q));
+                fused_step<R>(c, true, c->fold3 ? &amps[0] : nullptr);
+                if (!c->fold3) do_sources<R>(c, amps);
+                do_inject<R>(c, plan_param(c, P, 0), plan_param(c, P, 1));
+                for (auto &g : c->groups) do_group<R>(c, *g, plan_param(c, P, 2));
+                if (P.has_det) do_sample<R>(c, plan_param(c, P, 3), plan_param(c, P, 0));
+            }
+            k += c->launches - before;
+        }
+    for (int l = 0; l < lanes; ++l) {
+        ck(cudaEventRecord(b->ev_lane[l], b->lane[l]), "event");
+        ck(cudaStreamWaitEvent(b->stream, b->ev_lane[l], 0), "event");
+    }
+    return k;
+}
+
 // One batched step: H of every grid in one launch, the sources, the dispersive cells and the
 // bulk E of every grid in one launch, the per-grid emitter work, the detectors in one launch.
 template <class R> long long batch_step(omx_batch *b, const BatchTables<R> &T, const std::vector<RunPlan> &plans,
@@ -3751,8 +3815,9 @@ template <class R> void batch_run_impl(omx_batch *b, int tt0, int nsteps, int n_
     const int kch = b->kch > 0 ? b->kch : BATCH_DEFAULT_KCH;
     if (b->blocks == 0) b->blocks = batch3_blocks<R>();
     // the fused path alternates the members' buffer sets: step s of this call uses T[s & 1]
-    const bool f3 = b->fused == 1;
-    std::vector<long long> key = {b->fused, kch, b->f3form, b->f3kch, b->f3nsplit, b->blocks};
+    const bool ip = b->fused == 1 && b->f3inplace, f3 = b->fused == 1 && !ip;
+    if (ip) batch_lanes(b);
+    std::vector<long long> key = {b->fused, kch, b->f3form, b->f3kch, b->f3nsplit, b->blocks, b->f3inplace};
     for (size_t i = 0; i < b->ctx.size(); ++i) {
         const omx_ctx *c = b->ctx[i];
         key.insert(key.end(), {(long long)c->epoch, c->cur, (long long)(uintptr_t)c->tab.p, plans[i].W,
@@ -3762,7 +3827,7 @@ template <class R> void batch_run_impl(omx_batch *b, int tt0, int nsteps, int n_
     if (key != b->key) {
         b->drop_graphs();
         b->key.clear();
-        T[0] = batch_tables<R>(b, &plans, kch, 0);
+        T[0] = ip ? BatchTables<R>() : batch_tables<R>(b, &plans, kch, 0);
         T[1] = f3 ? batch_tables<R>(b, &plans, kch, 1) : BatchTables<R>();
         b->key = key;
     }
@@ -3782,7 +3847,8 @@ template <class R> void batch_run_impl(omx_batch *b, int tt0, int nsteps, int n_
                 cudaGraph_t graph;
                 ck(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "capture");
                 long long per = 0;
-                for (int q = 0; q < steps; ++q) per += batch_step<R>(b, T[f3 ? (q & 1) : 0], plans, kch);
+                if (ip) per = batch_inplace_steps<R>(b, &plans, steps);
+                for (int q = 0; !ip && q < steps; ++q) per += batch_step<R>(b, T[f3 ? (q & 1) : 0], plans, kch);
                 ck(cudaStreamEndCapture(b->stream, &graph), "end capture");
                 for (size_t i = 0; i < b->ctx.size(); ++i) b->ctx[i]->cur = cur0[i];
                 cudaGraphExec_t exec = nullptr;
@@ -3803,11 +3869,36 @@ template <class R> void batch_run_impl(omx_batch *b, int tt0, int nsteps, int n_
         const int left = per_graph > 0 ? nsteps % per_graph : nsteps;
         if (left) run_graph(left, k);
     } else if (!prepare_only) {
-        for (int s = 0; s < nsteps; ++s) b->launches += batch_step<R>(b, T[f3 ? (s & 1) : 0], plans, kch);
+        if (ip) b->launches += batch_inplace_steps<R>(b, &plans, nsteps);
+        for (int s = 0; !ip && s < nsteps; ++s) b->launches += batch_step<R>(b, T[f3 ? (s & 1) : 0], plans, kch);
     }
     ck(cudaPeekAtLastError(), "launch");
     if (!prepare_only)
         for (size_t i = 0; i < b->ctx.size(); ++i) b->ctx[i]->rec_count += plans[i].nrec;
+}
+
+// In place or staged for a batch of grids that the fused pass can step: in place when every member
+// would step so by itself.  Measured, us per step, staged in the best of four shapes / in place: twelve
+// grids of 8.4 M cells in all 310 / 261, twelve of 1.3 M 85 / 48, three of 2.6 M 127 / 65, four of
+// 17.7 M 446 / 410, 32 of 31.7 M 906 / 906.
+bool batch_inplace_rule(const omx_batch *b)
+{
+    for (const auto *c : b->ctx) {
+        if (c->step_form != OMX_STEP_DEFAULT || (long long)c->n[0] * c->n[1] * c->n[2] > F3_INPLACE_MOST) return false;
+        for (const auto &g : c->groups)
+            if (g->cl) return false;         // members may share a closure, whose steps run one after the other
+    }
+    return true;
+}
+void batch_set_inplace(omx_batch *b, bool on)
+{
+    b->f3inplace = on;
+    for (auto *c : b->ctx) {
+        c->f3_pin = on ? 1 : 2;       // staged: the batched pass reads one buffer set and writes the other
+        c->march = 0;
+        c->fused_dirty = true;
+        c->epoch++;
+    }
 }
 
 // Tile depth of the batched passes, timed on the zero initial fields (which every pass maps to
@@ -3825,9 +3916,21 @@ template <class R> int batch_autotune_impl(omx_batch *b, int reps)
         cudaEvent_t e0, e1;
         ck(cudaEventCreate(&e0), "event");
         ck(cudaEventCreate(&e1), "event");
-        float best = 0.f;
+        float best = 0.f, inplace = 0.f;
         int pick = 8064;
         bool first = true;
+        const bool may = b->f3inplace;       // the in-place pass is timed beside the staged shapes
+        if (may) {
+            batch_lanes(b);
+            batch_inplace_steps<R>(b, nullptr, 1);
+            ck(cudaEventRecord(e0, b->stream), "event");
+            batch_inplace_steps<R>(b, nullptr, reps);
+            ck(cudaEventRecord(e1, b->stream), "event");
+            ck(cudaEventSynchronize(e1), "batch autotune");
+            ck(cudaEventElapsedTime(&inplace, e0, e1), "batch autotune");
+            b->f3inplace = false;
+            for (auto *c : b->ctx) second_set(c);
+        }
         int dev = 0, optin = 0;
         ck(cudaGetDevice(&dev), "device");
         ck(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "device");
@@ -3862,6 +3965,7 @@ template <class R> int batch_autotune_impl(omx_batch *b, int reps)
         b->f3nsplit = pick / 1000000;
         b->f3form = pick / 1000 % 1000;
         b->f3kch = pick % 1000;
+        if (may) batch_set_inplace(b, inplace <= best);
         return pick;
     }
     cudaEvent_t e0, e1;
@@ -3911,12 +4015,7 @@ void batch_decide(omx_batch *b)
     bool all = b->fp32;
     for (auto *c : b->ctx) all = all && fused_eligible(c);
     b->fused = all ? 1 : 0;
-    if (all)
-        for (auto *c : b->ctx) {
-            c->f3_pin = 2;             // the batched pass reads one buffer set and writes the other
-            c->fused_dirty = true;
-            c->epoch++;
-        }
+    if (all) batch_set_inplace(b, batch_inplace_rule(b));
     if (!all)
         for (auto *c : b->ctx) {
             c->step_form = OMX_STEP_TWO_PASS;
@@ -3995,6 +4094,7 @@ int omx_batch_set_launch_shape(omx_batch *b, int shape)
         b->f3nsplit = shape / 1000000;
         b->f3form = form;
         b->f3kch = kch;
+        if (b->f3inplace) batch_set_inplace(b, false);
     } else {
         req(shape == 4 || shape == 8 || shape == 16 || shape == 32, "batched two-pass shape: tile depth 4, 8, 16 or 32");
         b->kch = shape;
@@ -4048,6 +4148,10 @@ int omx_batch_destroy(omx_batch *b)
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     if (b->ev_join) cudaEventDestroy(b->ev_join);
     if (b->ev_mixed) cudaEventDestroy(b->ev_mixed);
+    for (int l = 0; l < omx_batch::LANES; ++l) {
+        if (b->lane[l]) cudaStreamDestroy(b->lane[l]);
+        if (b->ev_lane[l]) cudaEventDestroy(b->ev_lane[l]);
+    }
     cudaStream_t s = b->stream, a = b->aux;
     delete b;
     if (s) cudaStreamDestroy(s);

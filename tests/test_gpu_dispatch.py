@@ -317,3 +317,52 @@ def test_inplace_and_staged_3d_steps_bit_identical(n, bnd, src, taps_h):
         assert len(o) == len(out[0])
         for a, b in zip(o, out[0]):
             assert np.array_equal(a, b)
+
+
+def test_inplace_batch_equals_solo_and_staged():
+    """A batch of small grids steps in place in one launch per half step: ragged sides, dispersive
+    cells, a folded plane source and radial ones, emitters; equal to solo runs and to the staged
+    batch bit for bit, also when the batch is autotuned or switched between calls."""
+    from test_gpu_parity import fused3_deck
+    from omx import decks
+
+    specs = [((33, 30, 27), (3, 3, 3), "plane"), ((40, 36, 28), (3, 3, 2), "both"), ((29, 41, 26), (1, 3, 3), "plane")]
+
+    def build(spec):
+        d = fused3_deck(*spec[:2], src=spec[2])
+        g = omx.TMxll(3, d["grid_Ndims"], d["npml"], d["boundaries"], d["dt"], d["dr"], precision="fp32")
+        gr = decks.apply_deck(g, d, omx, decks.media_map(d, omx.media_map_from_voxels))
+        for det in d["detectors"]:
+            g.add_detector(det["type"], det["field"], det["idx"])
+        return g, gr
+
+    def state(g, gr):
+        return [g.drain_detectors()[1]] + [g.read_field(f) for f in range(1, 7)] + [q.read()["rho"] for q in gr]
+
+    want = []
+    for sp in specs:
+        g, gr = build(sp)
+        g.run(1, 31, 1, 1)
+        want.append(state(g, gr))
+        g.kill()
+    for mode in ("inplace", "staged", "tuned", "switched"):
+        grids = [build(sp) for sp in specs]
+        b = omx.Batch([g for g, _ in grids])
+        if mode == "tuned":
+            b.autotune(reps=1)
+        if mode == "staged":
+            b.set_launch_shape(8016)
+        b.run(1, 14, 1, 1)
+        if mode == "switched":
+            b.synchronize()
+            b.set_launch_shape(8016)
+        b.run(15, 17, 1, 1)
+        b.synchronize()
+        for (g, gr), w in zip(grids, want):
+            got = state(g, gr)
+            assert np.max(np.abs(w[0])) > 0
+            for x, y in zip(got, w):
+                assert np.array_equal(x, y)
+        b.kill()
+        for g, _ in grids:
+            g.kill()
