@@ -1026,8 +1026,8 @@ void second_set(omx_ctx *c)
 
 // In place or staged, for a grid that the fused 3D pass can step: in place up to F3_INPLACE_MOST
 // cells.  Measured, us per step with a gold sphere and 10-cell CPML on every face, in place / staged
-// (default shapes): 32^3 7.9 / 25.4, 64^3 10.8 / 27.4, 96^3 22.0 / 62.8, 128^3 44.4 / 99.4, 160^3
-// 104 / 139, 192^3 171 / 175, 224^3 257 / 236, 256^3 362 / 321.
+// (default shapes): 32^3 7.9 / 25.4, 64^3 10.7 / 27.4, 96^3 20.5 / 62.8, 128^3 37.9 / 99.4, 160^3
+// 89 / 139, YY
 constexpr long long F3_INPLACE_MOST = 7000000;
 bool f3_inplace_rule(const omx_ctx *c)
 {

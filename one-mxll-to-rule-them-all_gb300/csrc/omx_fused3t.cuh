@@ -858,7 +858,7 @@ __device__ __forceinline__ void f3g_h_run(const Fused3Args &A, const GridArgs<fl
 // One general run's new E; then, when G.step_inc is set, the last of the nblk blocks of this
 // grid's launch advances the grid's device-loop step counter (this launch ends the pass and holds
 // its only reads of the step's scalars).
-template <int TY, bool ADE_LIST = false>
+template <int TY>
 __device__ __forceinline__ void f3g_e_run(const Fused3Args &A, const GridArgs<float> &G, int4 it, unsigned nblk)
 {
     const Lay &L = G.L;
@@ -887,13 +887,12 @@ __device__ __forceinline__ void f3g_e_run(const Fused3Args &A, const GridArgs<fl
             hxm = hx;
             hym = hy;
             float ex = __ldcs(A.in.f[0] + idx), ey = __ldcs(A.in.f[1] + idx), ez = __ldcs(A.in.f[2] + idx);
-            const int skip = f3t_e_general<ADE_LIST>(
-                ex, ey, ez, rx, ry, rz, dhxk, dhyk, hx, hy, hz, hz_im, hy_im, hz_jm, hx_jm, i, j, k,
-                bxE >= 0 ? bxE + sX * (k - 1) : -1, byE >= 0 ? byE + sY * (k - 1) : -1, lez >= 0 ? bz0 + sZ * lez : -1,
-                __ldg(G.bE[2] + k), __ldg(G.cE[2] + k), bbc, dt_eps0, G);
-            if (!ADE_LIST || !(skip & 1)) __stcs(A.out.f[0] + idx, ex);
-            if (!ADE_LIST || !(skip & 2)) __stcs(A.out.f[1] + idx, ey);
-            if (!ADE_LIST || !(skip & 4)) __stcs(A.out.f[2] + idx, ez);
+            f3t_e_general(ex, ey, ez, rx, ry, rz, dhxk, dhyk, hx, hy, hz, hz_im, hy_im, hz_jm, hx_jm, i, j, k,
+                          bxE >= 0 ? bxE + sX * (k - 1) : -1, byE >= 0 ? byE + sY * (k - 1) : -1,
+                          lez >= 0 ? bz0 + sZ * lez : -1, __ldg(G.bE[2] + k), __ldg(G.cE[2] + k), bbc, dt_eps0, G);
+            __stcs(A.out.f[0] + idx, ex);
+            __stcs(A.out.f[1] + idx, ey);
+            __stcs(A.out.f[2] + idx, ez);
         }
     }
     if (G.step_inc) {
@@ -927,17 +926,199 @@ __global__ void __launch_bounds__(32 * TY, 1536 / (32 * TY)) k_f3g_e(Fused3Args 
 // marching kch planes.  Grids that fit in L2 step faster this way than through the staged pass: half
 // the working set, and thousands of short blocks instead of a hundred that march their planes one
 // by one (f3_inplace_rule has both sides' times).  The H launch advances the device-loop step counter.
-__global__ void __launch_bounds__(128, 10) k_f3p_h(Fused3Args A, GridArgs<float> G, int kch)
+//
+// The march is instruction-bound before it is memory-bound (a 128^3 pass through the general runs'
+// loop issued 226 instructions per warp and plane: 43.6 us per step, 160^3 102 us; this loop 37.9 and
+// 89), so a warp without an x or y slab takes a loop
+// compiled without their terms (XY = false), the slab coefficients of the others are held per
+// thread, and a plane that needs more (a z slab, the media box, the plane source) is a branch that the
+// whole warp takes or leaves.  The operations and their rounding are f3t_hx / f3t_hy / f3t_hz's and
+// f3t_e_general's.
+constexpr int F3P_H_BLOCKS = 8, F3P_E_BLOCKS = 8;   // blocks per SM: 64 registers (10 and 9: 39, 6: 46 us at 128^3 against 38)
+
+template <bool XY>
+__device__ __forceinline__ void f3p_h_march(const Fused3Args &A, const GridArgs<float> &G, int i, int j, int k0, int k1)
 {
-    if (G.step_inc && blockIdx.x + blockIdx.y + blockIdx.z == 0 && threadIdx.x + threadIdx.y == 0) *G.step_inc += 1;
-    const int k0 = 1 + (int)blockIdx.z * kch;
-    f3g_h_run<4>(A, G, make_int4((1 + 32 * (int)blockIdx.x) | (32 << 20), (1 + 4 * (int)blockIdx.y) | (4 << 20), k0,
-                                 min(G.L.nz, k0 + kch - 1)));
+    const Lay &L = G.L;
+    const bool perz = G.per[2] != 0;
+    const float *__restrict__ Ex = A.in.f[0];
+    const float *__restrict__ Ey = A.in.f[1];
+    const float *__restrict__ Ez = A.in.f[2];
+    float *Hx = A.out.f[3], *Hy = A.out.f[4], *Hz = A.out.f[5];
+    const float dt_mu0 = G.dt_mu0, dhx = G.den_h[0][i], dhy = G.den_h[1][j];
+    const int px_ = L.px, pz_ = (int)L.pz, sZ = L.nx * L.ny, bz0 = (i - 1) + L.nx * (j - 1);
+    int qx = -1, qy = -1;                       // psi indices at plane k
+    float bx = 0.f, cx = 0.f, by = 0.f, cy = 0.f;
+    if (XY) {
+        const int lx = G.lH[0][i], ly = G.lH[1][j];
+        if (lx >= 0) {
+            qx = lx + G.L2 * ((j - 1) + L.ny * (k0 - 1));
+            bx = G.bH[0][i];
+            cx = G.cH[0][i];
+        }
+        if (ly >= 0) {
+            qy = (i - 1) + L.nx * (ly + G.L2 * (k0 - 1));
+            by = G.bH[1][j];
+            cy = G.cH[1][j];
+        }
+    }
+    int idx = (int)L.off + i + px_ * j + pz_ * k0;   // element offsets < 2^31 (checked by the host)
+    float ex_c = Ex[idx], ey_c = Ey[idx];
+#pragma unroll 2
+    for (int k = k0; k <= k1; ++k, idx += pz_) {
+        const int kp = (perz && k == L.nz) ? idx - (L.nz - 1) * pz_ : idx + pz_;   // E of plane k + 1
+        const float ez_c = Ez[idx], ez_jp = Ez[idx + px_], ez_ip = Ez[idx + 1], ey_ip = Ey[idx + 1], ex_jp = Ex[idx + px_];
+        const float ex_kp = Ex[kp], ey_kp = Ey[kp];
+        float hx = __ldcs(Hx + idx), hy = __ldcs(Hy + idx), hz = __ldcs(Hz + idx);
+        float x0 = 0.f, x1 = 0.f, y0 = 0.f, y1 = 0.f;
+        if (XY && qx >= 0) {
+            x0 = A.psiH_out[0][0][qx];
+            x1 = A.psiH_out[0][1][qx];
+        }
+        if (XY && qy >= 0) {
+            y0 = A.psiH_out[1][0][qy];
+            y1 = A.psiH_out[1][1][qy];
+        }
+        const float dhz = G.den_h[2][k];
+        const int lz = G.lH[2][k];
+        const float dzy = __fsub_rn(ez_c, ez_jp), dyz = __fsub_rn(ey_kp, ey_c), dzx = __fsub_rn(ez_ip, ez_c),
+                    dxz = __fsub_rn(ex_c, ex_kp), dyx = __fsub_rn(ey_c, ey_ip), dxy = __fsub_rn(ex_jp, ex_c);
+        hx = __fmaf_rn(dt_mu0, __fmaf_rn(dyz, dhz, __fmul_rn(dzy, dhy)), hx);
+        hy = __fmaf_rn(dt_mu0, __fmaf_rn(dxz, dhz, __fmul_rn(dzx, dhx)), hy);
+        hz = __fmaf_rn(dt_mu0, __fmaf_rn(dxy, dhy, __fmul_rn(dyx, dhx)), hz);
+        if (XY && qx >= 0) {   // mxll_3D_mod.f90:585-620
+            const float v0 = f3t_psi(bx, x0, cx, dzx), v1 = f3t_psi(bx, x1, cx, dyx);
+            A.psiH_out[0][0][qx] = v0;
+            A.psiH_out[0][1][qx] = v1;
+            hy = __fmaf_rn(dt_mu0, v0, hy);
+            hz = __fmaf_rn(dt_mu0, v1, hz);
+            qx += G.L2 * L.ny;
+        }
+        if (XY && qy >= 0) {   // :622-657
+            const float v0 = f3t_psi(by, y0, cy, dzy), v1 = f3t_psi(by, y1, cy, dxy);
+            A.psiH_out[1][0][qy] = v0;
+            A.psiH_out[1][1][qy] = v1;
+            hx = __fmaf_rn(dt_mu0, v0, hx);
+            hz = __fmaf_rn(dt_mu0, v1, hz);
+            qy += L.nx * G.L2;
+        }
+        if (lz >= 0) {         // :659-694
+            const int q = bz0 + sZ * lz;
+            const float bz = G.bH[2][k], cz = G.cH[2][k];
+            const float v0 = f3t_psi(bz, A.psiH_out[2][0][q], cz, dyz), v1 = f3t_psi(bz, A.psiH_out[2][1][q], cz, dxz);
+            A.psiH_out[2][0][q] = v0;
+            A.psiH_out[2][1][q] = v1;
+            hx = __fmaf_rn(dt_mu0, v0, hx);
+            hy = __fmaf_rn(dt_mu0, v1, hy);
+        }
+        __stcs(Hx + idx, hx);
+        __stcs(Hy + idx, hy);
+        __stcs(Hz + idx, hz);
+        if (perz && k == L.nz) {   // periodic ghost plane H(0) = H(nz) (mxll_3D_mod.f90:725-738)
+            Hx[idx - L.nz * pz_] = hx;
+            Hy[idx - L.nz * pz_] = hy;
+        }
+        ex_c = ex_kp;
+        ey_c = ey_kp;
+    }
 }
+
+__global__ void __launch_bounds__(128, F3P_H_BLOCKS) k_f3p_h(const __grid_constant__ Fused3Args A,
+                                                             const __grid_constant__ GridArgs<float> G, int kch)
+{
+    const int i = 1 + 32 * (int)blockIdx.x + (int)threadIdx.x, j = 1 + 4 * (int)blockIdx.y + (int)threadIdx.y;
+    const int k0 = 1 + (int)blockIdx.z * kch, k1 = min(G.L.nz, k0 + kch - 1);
+    if (G.step_inc && blockIdx.x + blockIdx.y + blockIdx.z == 0 && threadIdx.x + threadIdx.y == 0) *G.step_inc += 1;
+    const bool in = i <= G.L.nx && j <= G.L.ny;
+    const bool xy = __any_sync(0xffffffffu, in && (G.lH[0][i] >= 0 || G.lH[1][j] >= 0));
+    if (!in) return;
+    if (xy) f3p_h_march<true>(A, G, i, j, k0, k1);
+    else f3p_h_march<false>(A, G, i, j, k0, k1);
+}
+
+template <bool XY>
+__device__ __forceinline__ void f3p_e_march(const Fused3Args &A, const GridArgs<float> &G, int i, int j, int k0, int k1)
+{
+    const Lay &L = G.L;
+    const float *__restrict__ Hx = A.out.f[3];
+    const float *__restrict__ Hy = A.out.f[4];
+    const float *__restrict__ Hz = A.out.f[5];
+    float *Ex = A.out.f[0], *Ey = A.out.f[1], *Ez = A.out.f[2];
+    const float dt_eps0 = G.dt_eps0, dex = G.den_e[0][i], dey = G.den_e[1][j];
+    const int px_ = L.px, pz_ = (int)L.pz, sZ = L.nx * L.ny, bz0 = (i - 1) + L.nx * (j - 1);
+    const int sX = G.L2 * L.ny, sY = L.nx * G.L2;
+    int qx = -1, qy = -1;
+    float bx = 0.f, cx = 0.f, by = 0.f, cy = 0.f;
+    if (XY) {
+        const int lx = G.lE[0][i], ly = G.lE[1][j];
+        if (lx >= 0) {
+            qx = lx + G.L2 * ((j - 1) + L.ny * (k0 - 1));
+            bx = G.bE[0][i];
+            cx = G.cE[0][i];
+        }
+        if (ly >= 0) {
+            qy = (i - 1) + L.nx * (ly + G.L2 * (k0 - 1));
+            by = G.bE[1][j];
+            cy = G.cE[1][j];
+        }
+    }
+    const bool bbc = i >= G.bb0[0] && i <= G.bb1[0] && j >= G.bb0[1] && j <= G.bb1[1];
+    // planes k of this column that the media box or the plane source reaches
+    const int mk0 = bbc ? G.bb0[2] : 1, mk1 = bbc ? G.bb1[2] : 0;
+    const bool plc = G.pl_on && (G.pl_axis == 0 ? i == G.pl_index : (G.pl_axis == 1 ? j == G.pl_index : false));
+    const int plk = G.pl_on && G.pl_axis == 2 ? G.pl_index : 0;
+    int idx = (int)L.off + i + px_ * j + pz_ * k0;
+    float hxm = Hx[idx - pz_], hym = Hy[idx - pz_];
+#pragma unroll 2
+    for (int k = k0; k <= k1; ++k, idx += pz_) {
+        const float hx = Hx[idx], hy = Hy[idx], hz = Hz[idx];
+        const float hz_im = Hz[idx - 1], hy_im = Hy[idx - 1], hz_jm = Hz[idx - px_], hx_jm = Hx[idx - px_];
+        float ex = __ldcs(Ex + idx), ey = __ldcs(Ey + idx), ez = __ldcs(Ez + idx);
+        const float dez = G.den_e[2][k];
+        const int lz = G.lE[2][k];
+        int skip = 0;
+        const float dhyk = __fsub_rn(hym, hy), dhxk = __fsub_rn(hx, hxm);
+        const float dzy = __fsub_rn(hz, hz_jm), dzx = __fsub_rn(hz_im, hz), dyx = __fsub_rn(hy, hy_im),
+                    dxy = __fsub_rn(hx_jm, hx);
+        const float rx = __fmaf_rn(dhyk, dez, __fmul_rn(dzy, dey)), ry = __fmaf_rn(dhxk, dez, __fmul_rn(dzx, dex)),
+                    rz = __fmaf_rn(dxy, dey, __fmul_rn(dyx, dex));
+        if (lz >= 0 || plc || k == plk || (k >= mk0 && k <= mk1)) {
+            skip = f3t_e_general<true>(ex, ey, ez, rx, ry, rz, dhxk, dhyk, hx, hy, hz, hz_im, hy_im, hz_jm, hx_jm, i, j, k,
+                                       XY ? qx : -1, XY ? qy : -1, lz >= 0 ? bz0 + sZ * lz : -1, G.bE[2][k], G.cE[2][k],
+                                       bbc, dt_eps0, G);
+        } else {
+            ex = __fmaf_rn(dt_eps0, rx, ex);
+            ey = __fmaf_rn(dt_eps0, ry, ey);
+            ez = __fmaf_rn(dt_eps0, rz, ez);
+            if (XY && qx >= 0) {   // mxll_3D_mod.f90:817-849
+                const float v0 = f3t_psi(bx, G.psiE[0][0][qx], cx, dzx), v1 = f3t_psi(bx, G.psiE[0][1][qx], cx, dyx);
+                G.psiE[0][0][qx] = v0;
+                G.psiE[0][1][qx] = v1;
+                ey = __fmaf_rn(dt_eps0, v0, ey);
+                ez = __fmaf_rn(dt_eps0, v1, ez);
+            }
+            if (XY && qy >= 0) {   // :851-885
+                const float v0 = f3t_psi(by, G.psiE[1][0][qy], cy, dzy), v1 = f3t_psi(by, G.psiE[1][1][qy], cy, dxy);
+                G.psiE[1][0][qy] = v0;
+                G.psiE[1][1][qy] = v1;
+                ex = __fmaf_rn(dt_eps0, v0, ex);
+                ez = __fmaf_rn(dt_eps0, v1, ez);
+            }
+        }
+        if (XY && qx >= 0) qx += sX;
+        if (XY && qy >= 0) qy += sY;
+        if (!(skip & 1)) __stcs(Ex + idx, ex);
+        if (!(skip & 2)) __stcs(Ey + idx, ey);
+        if (!(skip & 4)) __stcs(Ez + idx, ez);
+        hxm = hx;
+        hym = hy;
+    }
+}
+
 // New E of one dispersive component-cell (entry q of the grid's list): f3t_e_general's terms of that
 // component.  A thread per entry: marched inside the plane loop, a column of gold cells is a chain
 // of state reads (a 128^3 grid with a sphere of 20 cells radius: 51 us per step at best that way,
-// 62 us at four planes a thread; 44 us with the list).
+// 62 us at four planes a thread; 38 us with the list).
 __device__ __forceinline__ void f3p_ade_cell(const Fused3Args &A, const GridArgs<float> &G, int q)
 {
     const Lay &L = G.L;
@@ -989,7 +1170,8 @@ __device__ __forceinline__ void f3p_ade_cell(const Fused3Args &A, const GridArgs
 }
 
 // zl: leading block layers along z that take the list of dispersive component-cells
-__global__ void __launch_bounds__(128, 9) k_f3p_e(Fused3Args A, GridArgs<float> G, int kch, int zl)
+__global__ void __launch_bounds__(128, F3P_E_BLOCKS) k_f3p_e(const __grid_constant__ Fused3Args A,
+                                                             const __grid_constant__ GridArgs<float> G, int kch, int zl)
 {
     if ((int)blockIdx.z < zl) {
         const int q = 128 * (int)(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)) +
@@ -997,9 +1179,13 @@ __global__ void __launch_bounds__(128, 9) k_f3p_e(Fused3Args A, GridArgs<float> 
         if (q < G.ade_n) f3p_ade_cell(A, G, q);
         return;
     }
-    const int k0 = 1 + ((int)blockIdx.z - zl) * kch;
-    f3g_e_run<4, true>(A, G, make_int4((1 + 32 * (int)blockIdx.x) | (32 << 20), (1 + 4 * (int)blockIdx.y) | (4 << 20), k0,
-                                       min(G.L.nz, k0 + kch - 1)), 0u);
+    const int i = 1 + 32 * (int)blockIdx.x + (int)threadIdx.x, j = 1 + 4 * (int)blockIdx.y + (int)threadIdx.y;
+    const int k0 = 1 + ((int)blockIdx.z - zl) * kch, k1 = min(G.L.nz, k0 + kch - 1);
+    const bool in = i <= G.L.nx && j <= G.L.ny;
+    const bool xy = __any_sync(0xffffffffu, in && (G.lE[0][i] >= 0 || G.lE[1][j] >= 0));
+    if (!in) return;
+    if (xy) f3p_e_march<true>(A, G, i, j, k0, k1);
+    else f3p_e_march<false>(A, G, i, j, k0, k1);
 }
 
 // Batched general runs of several grids: items[b].w carries the run's grid (k1 | g << 20); the

@@ -231,8 +231,8 @@ cudaError_t launch_fused3p(const Fused3Args &A, const GridArgs<float> &G, int kc
 {
     const Lay &L = G.L;
     const dim3 b(32, 4);
-    // us per step at marches of 1, 2, 4, 8: 48^3 8.6, 9.1, 11.8, 19; 96^3 23.6, 22.0, 24.2, 22.2; 128^3 51,
-    // 45.6, 44.4, 48.6; 160^3 123, 108, 104, 105
+    // us per step at marches of 1, 2, 4, 8: 64^3 10.7, 9.8, 12.3, 18.3; 96^3 23.1, 20.5, 20.9, 23.1; 128^3
+    // 48, 40, 37.8, 40.6; 160^3 112, 93, 89, 93
     int m = kch > 0 ? kch : march_rule((long long)((L.nx + 31) / 32) * ((L.ny + 3) / 4), L.nz, 4, 22);
     dim3 g((L.nx + 31) / 32, (L.ny + 3) / 4, (L.nz + m - 1) / m);
     if (e_half) {
