@@ -299,7 +299,7 @@ int omx_run_prepare(omx_ctx *ctx, int tt0, int nsteps, int n_skip_steps, int t_d
  * FP32 bar; they differ in rounding, and the form may be changed between steps.
  *   OMX_STEP_DEFAULT      one fused pass per step where eligible (2D TMz; 3D with x and y not
  *                         periodic: the planes staged by TMA, the dispersive cells and a single
- *                         plane source inside the pass; 3D grids that fit in L2 take the same
+ *                         plane source inside the pass; 3D grids of up to 18 M cells take the same
  *                         arithmetic in two passes in place), else the two half-step passes
  *   OMX_STEP_TWO_PASS     the two half-step passes everywhere: the arithmetic of batched runs
  *                         (omx_batch_create sets it on its members)

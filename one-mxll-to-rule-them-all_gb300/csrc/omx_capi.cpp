@@ -1027,8 +1027,9 @@ void second_set(omx_ctx *c)
 // In place or staged, for a grid that the fused 3D pass can step: in place up to F3_INPLACE_MOST
 // cells.  Measured, us per step with a gold sphere and 10-cell CPML on every face, in place / staged
 // (default shapes): 32^3 7.9 / 25.4, 64^3 10.7 / 27.4, 96^3 20.5 / 62.8, 128^3 37.9 / 99.4, 160^3
-// 89 / 139, YY
-constexpr long long F3_INPLACE_MOST = 7000000;
+// 89 / 139, 192^3 140 / 173, 224^3 208 / 233, 256^3 293 / 318, 288^3 403 / 419, 320^3 537 / 529, 384^3
+// 879 / 820; with 1e5 emitters, which overlap the in-place step's H pass only, 320 x 288 x 250 482 / 438.
+constexpr long long F3_INPLACE_MOST = 18000000;
 bool f3_inplace_rule(const omx_ctx *c)
 {
     if (c->dims != 3) return false;

@@ -232,8 +232,9 @@ cudaError_t launch_fused3p(const Fused3Args &A, const GridArgs<float> &G, int kc
     const Lay &L = G.L;
     const dim3 b(32, 4);
     // us per step at marches of 1, 2, 4, 8: 64^3 10.7, 9.8, 12.3, 18.3; 96^3 23.1, 20.5, 20.9, 23.1; 128^3
-    // 48, 40, 37.8, 40.6; 160^3 112, 93, 89, 93
-    int m = kch > 0 ? kch : march_rule((long long)((L.nx + 31) / 32) * ((L.ny + 3) / 4), L.nz, 4, 22);
+    // 48, 40, 37.8, 40.6; 160^3 112, 93, 89, 93; of 4, 8, 16: 224^3 208, 208; 256^3 298, 293, 302
+    const long long tiles = (long long)((L.nx + 31) / 32) * ((L.ny + 3) / 4);
+    int m = kch > 0 ? kch : std::max(march_rule(tiles, L.nz, 4, 22), march_rule(tiles, L.nz, 8, 80));
     dim3 g((L.nx + 31) / 32, (L.ny + 3) / 4, (L.nz + m - 1) / m);
     if (e_half) {
         const unsigned layer = g.x * g.y * 128, zl = ((unsigned)G.ade_n + layer - 1) / layer;
