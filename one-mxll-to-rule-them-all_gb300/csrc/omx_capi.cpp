@@ -191,6 +191,7 @@ struct omx_ctx {
     DevBuf<int> inj_c, inj_a, inj_b;
     int inj_n = 0;
     std::vector<int4> inj_host;    // (i, j, k, component) of every emitter-current point
+    DevBuf<int> jp_at, inj_at;     // 1D: J point of each cell (or -1), and whether its E takes the current
     bool j_dirty = false;
     // detectors
     struct Det {
@@ -545,6 +546,15 @@ template <class R> FieldPtrs<R> field_ptrs(omx_ctx *c, int parity = -1)
     return F;
 }
 
+// 1/d as the sum of two doubles for div_dr (0 where it divides): the remainder 1 - h * d is exact
+void reciprocal(double d, double &h, double &l)
+{
+    h = l = 0.0;
+    if (!(d > 0x1p-100 && d < 0x1p100)) return;
+    h = 1.0 / d;
+    l = std::fma(-h, d, 1.0) / d;
+}
+
 template <class R> GridArgs<R> grid_args(omx_ctx *c)
 {
     GridArgs<R> G;
@@ -556,11 +566,11 @@ template <class R> GridArgs<R> grid_args(omx_ctx *c)
     G.dt_mu0 = (R)dt_mu0;
     G.dt_eps0 = (R)dt_eps0;
     G.dr = (R)c->desc.dr;
-    if (std::is_same<R, double>::value && c->desc.dr > 0x1p-100 && c->desc.dr < 0x1p100) {
-        // 1/dr as the sum of two doubles for div_dr: the remainder 1 - rdr_h * dr is exact
-        const double h = 1.0 / c->desc.dr;
+    if (std::is_same<R, double>::value) {
+        double h, l;
+        reciprocal(c->desc.dr, h, l);
         G.rdr_h = (R)h;
-        G.rdr_l = (R)(std::fma(-h, c->desc.dr, 1.0) / c->desc.dr);
+        G.rdr_l = (R)l;
     }
     for (int a = 0; a < 3; ++a) G.per[a] = c->per[a];
     G.npml = c->desc.npml;
@@ -860,6 +870,13 @@ void rebuild_jpoints(omx_ctx *c)
         g->wk.upload(wk);
     }
     rebuild_injection(c);
+    if (c->dims == 1) {
+        std::vector<int> at((size_t)c->n[0] + 2, -1), inj((size_t)c->n[0] + 2, 0);
+        for (int p = 0; p < np; ++p) at[(size_t)(keys[p] % (c->n[0] + 2))] = p;
+        for (const int4 &e : c->inj_host) inj[(size_t)e.x] = 1;
+        c->jp_at.upload(at);
+        c->inj_at.upload(inj);
+    }
     c->j_dirty = false;
 }
 
@@ -1147,9 +1164,15 @@ template <class R> void do_inject(omx_ctx *c, StepParam time, StepParam t_skip)
     }
 }
 
-template <class R> void do_group(omx_ctx *c, GroupRec &g, StepParam move)
+DtArgs dt_args(const omx_ctx *c, double dt)
 {
-    ProfScope ps(c, KC_EMIT);
+    DtArgs D{dt, c->fp32 ? 1.0 / dt : 0.0, 0.0, 0.0};
+    reciprocal(dt, D.rdt_h, D.rdt_l);
+    return D;
+}
+
+EmitArgs emit_args(const omx_ctx *c, const GroupRec &g)
+{
     EmitArgs A;
     A.n = g.d.n_systems;
     A.model = g.d.model;
@@ -1169,8 +1192,30 @@ template <class R> void do_group(omx_ctx *c, GroupRec &g, StepParam move)
     A.dt = g.d.dt;
     A.h2 = 0.5 * g.d.dt;
     A.h6 = g.d.dt / 6.0;
-    A.inv_dt = c->fp32 ? 1.0 / g.d.dt : 0.0;
+    A.over = dt_args(c, g.d.dt);
     A.only_if = nullptr;
+    return A;
+}
+
+ScatArgs scat_args(const omx_ctx *c, const GroupRec &g)
+{
+    ScatArgs S;
+    S.np = (int)c->jkeys.size();
+    if (c->dims == 3) { S.c0 = 0; S.c1 = 2; }
+    else if (c->dims == 1) { S.c0 = 0; S.c1 = 0; }
+    else if (c->desc.mode == OMX_TMZ_2D_MODE) { S.c0 = 2; S.c1 = 2; }
+    else { S.c0 = 0; S.c1 = 1; }
+    S.win = g.win.p;
+    S.wk = g.wk.p;
+    S.dPdt = g.dPdt.p;
+    S.over = dt_args(c, g.d.dt);
+    return S;
+}
+
+template <class R> void do_group(omx_ctx *c, GroupRec &g, StepParam move)
+{
+    ProfScope ps(c, KC_EMIT);
+    EmitArgs A = emit_args(c, g);
     if (g.cl) {
         // network step, spot-check subset, check / fallback; the plain propagator below runs only
         // once the fallback flag is set
@@ -1182,17 +1227,7 @@ template <class R> void do_group(omx_ctx *c, GroupRec &g, StepParam move)
         A.only_if = &g.dep.st->plain_now;    // not on the step the fallback happens
     }
     launch_emit<R>(field_ptrs<R>(c), c->L, A, move, c->stream);
-    ScatArgs S;
-    S.np = (int)c->jkeys.size();
-    if (c->dims == 3) { S.c0 = 0; S.c1 = 2; }
-    else if (c->dims == 1) { S.c0 = 0; S.c1 = 0; }
-    else if (c->desc.mode == OMX_TMZ_2D_MODE) { S.c0 = 2; S.c1 = 2; }
-    else { S.c0 = 0; S.c1 = 1; }
-    S.win = g.win.p;
-    S.wk = g.wk.p;
-    S.dPdt = g.dPdt.p;
-    S.dt = g.d.dt;
-    S.inv_dt = c->fp32 ? 1.0 / g.d.dt : 0.0;
+    const ScatArgs S = scat_args(c, g);
     launch_scatter(jstate(c), S, move, c->stream);
     c->launches += 2;
 }
@@ -1668,6 +1703,72 @@ RunPlan stage_run(omx_ctx *c, int tt0, int nsteps, int n_skip, int t_det_print, 
 
 StepParam plan_param(omx_ctx *c, const RunPlan &plan, int row) { return StepParam{0.0, c->tab.p + row, c->d_step.p, plan.W}; }
 
+// The 1D time loop in one launch (k_run1): what it leaves to the per-launch kernels are closures,
+// Fourier accumulation, H detectors, points outside the cells 1..n, and numbers of sources, groups,
+// emitters or cells that one cluster would be slow on or has no shared memory for (2048 FP64 cells a
+// block).  Measured, us per step in one launch / in launches, FP64 with a Drude film: 200 cells 3.2 /
+// 12.4, with 16 emitters 1500 cells 7.2 / 24.7, 12000 cells 10.6 / 24.9; 6000 cells with 256 emitters
+// 9.2 / 24.7, 512 13.8 / 26.5, 1024 (all through memory) 24.3 / 26.7.
+constexpr int RUN1_CELLS = 16384, RUN1_EMITTERS = 512, RUN1_TAPS = 2048;
+bool run1_ok(const omx_ctx *c, int nsteps, int use_graph)
+{
+    const int n = c->n[0];
+    if (c->dims != 1 || !use_graph || c->prof || nsteps < 2 || c->n_freq > 0 || c->taps_h) return false;
+    if (n > RUN1_CELLS || (int)c->sources.size() > RUN1_SOURCES || (int)c->groups.size() > RUN1_GROUPS) return false;
+    if ((int)c->tap_field.size() > RUN1_TAPS) return false;
+    for (const auto &S : c->sources) {
+        if (S->kind == 0) {
+            if (S->comp != 0) return false;
+            for (const int4 &p : S->cells)
+                if (p.x < 1 || p.x > n) return false;
+        } else if (S->pd.plane_axis != 1 || S->pd.comp != 1 || S->pd.plane_index < 1 || S->pd.plane_index > n) {
+            return false;
+        }
+    }
+    long long ne = 0;
+    for (const auto &g : c->groups) {
+        if (g->cl) return false;
+        ne += g->d.n_systems;
+    }
+    for (const long long key : c->jkeys)
+        if (key % (n + 2) < 1 || key % (n + 2) > n) return false;
+    return ne <= RUN1_EMITTERS;
+}
+
+template <class R> void run1(omx_ctx *c, const RunPlan &plan, int nsteps)
+{
+    Run1Args A;
+    std::memset(&A, 0, sizeof(A));
+    A.W = plan.W;
+    A.n_src = (int)c->sources.size();
+    for (int q = 0; q < A.n_src; ++q) {
+        const SourceRec &S = *c->sources[q];
+        A.src_kind[q] = S.kind;
+        if (S.kind == 0) A.src[q] = src_args(S);
+        else A.plane_e[q] = eindex(c, S.pd.plane_index, 0, 0);
+        A.plane_c[q] = S.c_src;
+    }
+    A.n_grp = (int)c->groups.size();
+    for (int q = 0; q < A.n_grp; ++q) {
+        A.grp[q] = emit_args(c, *c->groups[q]);
+        A.scat[q] = scat_args(c, *c->groups[q]);
+    }
+    A.J = jstate(c);
+    A.jp_at = c->jkeys.empty() ? nullptr : c->jp_at.p;
+    A.inj_at = c->inj_at.p;
+    A.dt_eps0 = c->desc.dt / omx::consts().eps0;
+    A.has_det = plan.has_det;
+    A.det = det_args(c);
+    // a launch of at most 4096 steps (tens of milliseconds) holds its SMs for no longer than other
+    // work may have to wait for
+    for (int s = 0; s < nsteps; s += 4096) {
+        A.tab = c->tab.p + (size_t)s * plan.W;
+        A.nsteps = std::min(4096, nsteps - s);
+        ck(launch_run1<R>(field_ptrs<R>(c), grid_args<R>(c), A, c->stream), "1D time loop");
+        c->launches++;
+    }
+}
+
 // prepare_only: capture and instantiate the step graphs that the same call without it launches,
 // with the device table and the record buffer sized for it, and run nothing (the stepping state
 // and the record count stay as they are).
@@ -1753,6 +1854,13 @@ template <class R> void run_impl(omx_ctx *c, int tt0, int nsteps, int n_skip, in
     join_side(c);
     if (prepare_only) stage_reserve(c, plan);
     else stage_upload(c, plan, false);
+    if (run1_ok(c, nsteps, use_graph)) {
+        if (!prepare_only) {
+            run1<R>(c, plan, nsteps);
+            c->rec_count += nrec;
+        }
+        return;
+    }
     std::vector<StepParam> amps;
     for (int q = 0; q < nsrc; ++q) amps.push_back(P(4 + q));
     auto tail = [&]() {

@@ -184,39 +184,6 @@ __device__ __forceinline__ float f3t_hz(float hz, float ey_c, float ey_ip, float
     return h;
 }
 
-// The ADE of one dispersive component-cell: ade_update's terms in the same order, each product
-// added by an explicitly rounded FMA (so that no tile shape or code path contracts differently),
-// with the pole state read again in the second loop instead of held in register arrays (which
-// would take registers from the whole pass).  st: the cell's state at slot 0 (PD), V: the slot stride, P:
-// poles per cell in the state.
-__device__ __forceinline__ float f3t_ade(float e, float rot, int type, const MedR<float> *mp, float *st, long long V,
-                                         int P)
-{
-    const MedR<float> &m = *mp;
-    const float PD = st[0];
-    if (type == CLS_DRUDE) {
-        const float t = __fmaf_rn(-m.C4, PD, __fmaf_rn(m.C3, rot, __fmul_rn(m.C1, e)));
-        st[0] = __fmaf_rn(m.A1, PD, __fmul_rn(m.A2, __fadd_rn(t, e)));
-        return t;
-    }
-    const float eo = st[V];
-    float t = __fmaf_rn(-m.C4, PD, __fmaf_rn(m.C3, rot, __fmaf_rn(m.C2, eo, __fmul_rn(m.C1, e))));
-    const int np = m.np;
-#pragma unroll 1
-    for (int p = 0; p < np; ++p)
-        t = __fmaf_rn(-m.B2[p], st[(2 + P + p) * V], __fmaf_rn(-m.B1[p], st[(2 + p) * V], t));
-    st[0] = __fmaf_rn(m.A1, PD, __fmul_rn(m.A2, __fadd_rn(t, e)));
-    const float dte = __fsub_rn(t, eo);
-#pragma unroll 1
-    for (int p = 0; p < np; ++p) {
-        const float pl = st[(2 + p) * V], plo = st[(2 + P + p) * V];
-        st[(2 + P + p) * V] = pl;
-        st[(2 + p) * V] = __fmaf_rn(m.al[p], pl, __fmaf_rn(m.be[p], plo, __fmul_rn(m.ga[p], dte)));
-    }
-    st[V] = e;
-    return t;
-}
-
 // E of one component inside the media box: plain classes, or the ADE of a dispersive class
 __device__ __forceinline__ float f3t_media(float e, float rot, int c, int b, const GridArgs<float> &G)
 {

@@ -126,6 +126,13 @@ struct PlaneArgs {
     double c_src;
 };
 
+// division by the emitters' dt (over_dt)
+struct DtArgs {
+    double dt;
+    double inv;               // FP32 fields: 1/dt; 0: the reference's division
+    double rdt_h, rdt_l;      // 1/dt as the sum of two doubles (0: divide)
+};
+
 struct EmitArgs {
     int n, model, npar, nst, dims, mode2d;
     const int *ci, *cj, *ck;
@@ -133,9 +140,7 @@ struct EmitArgs {
     const double *rates;      // (1/T1, 1/T2) per emitter, formed at group creation
     double *rho, *E, *dipole, *dPdt;
     double dt, h2, h6;        // dt, dt/2, dt/6
-    // 0: dPt_dt = (new - old) / dt, the reference's division (FP64 fields); else (new - old) * inv_dt,
-    // 1/dt rounded once (FP32 fields: within an ulp of the quotient, without an FP64 division)
-    double inv_dt;
+    DtArgs over;              // dPt_dt = (new - old) / dt
     const int *only_if;       // optional: run only while *only_if != 0 (the closure's fallback flag)
 };
 
@@ -144,8 +149,7 @@ struct ScatArgs {
     const int *win;
     const double *wk;
     const double *dPdt;
-    double dt;
-    double inv_dt;            // as EmitArgs::inv_dt, for dJ = (J - J_old) / dt
+    DtArgs over;              // dJ = (J - J_old) / dt
 };
 
 struct DetArgs {
@@ -185,6 +189,27 @@ template <class R> void launch_pack(const R *field, const PackArgs &P, long long
 template <class R> void launch_unpack(R *field, const PackArgs &P, long long row0, long long rows, const double *in, void *stream);
 // out[order[r] * w + q] = in[r * w + q]: device rows back into the caller's order
 void launch_scatter_rows(const double *in, const int *order, long long n, int w, double *out, void *stream);
+// the whole time loop of a 1D grid in one launch (omx_run1d.cuh)
+constexpr int RUN1_GROUPS = 4, RUN1_SOURCES = 4;
+struct Run1Args {
+    const double *tab;     // per-step table: time, t_skip, move, slot, source amplitudes
+    int W, nsteps;
+    int n_src;
+    int src_kind[RUN1_SOURCES];            // 0 radial, 1 plane
+    SrcArgs src[RUN1_SOURCES];
+    long long plane_e[RUN1_SOURCES];       // E word of a plane source's cell
+    double plane_c[RUN1_SOURCES];
+    int n_grp;
+    EmitArgs grp[RUN1_GROUPS];
+    ScatArgs scat[RUN1_GROUPS];
+    JState J;
+    const int *jp_at;      // J point of each cell (index 0 .. n + 1), or -1; null without emitters
+    const int *inj_at;     // 1 where the cell's E takes the emitter current
+    double dt_eps0;
+    int has_det;
+    DetArgs det;
+};
+template <class R> cudaError_t launch_run1(const FieldPtrs<R> &F, const GridArgs<R> &G, const Run1Args &A, void *stream);
 // FP32 fused TMz step: reads the in buffers, writes the out buffers (see omx_fused2d.cuh)
 struct Fused2Args {
     const float *ez_in, *hx_in, *hy_in;

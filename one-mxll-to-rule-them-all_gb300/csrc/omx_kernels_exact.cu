@@ -5,6 +5,7 @@
 #include "omx_stencil.cuh"
 #include "omx_sparse.cuh"
 #include "omx_batch.cuh"
+#include "omx_run1d.cuh"
 
 namespace omx {
 
@@ -17,6 +18,14 @@ template <> void launch_e<double>(const FieldPtrs<double> &F, const GridArgs<dou
     launch_e_impl<double, true>(F, G, s);
 }
 
+template <> cudaError_t launch_run1<double>(const FieldPtrs<double> &F, const GridArgs<double> &G, const Run1Args &A, void *s)
+{
+    return launch_run1_impl<double, true>(F, G, A, s);
+}
+template <> cudaError_t launch_run1<float>(const FieldPtrs<float> &F, const GridArgs<float> &G, const Run1Args &A, void *s)
+{
+    return launch_run1_impl<float, false>(F, G, A, s);
+}
 template <> void launch_batch3<double>(int pass, const BatchGrid<double> *g, int n, long long total, int kch,
                                       int blocks, void *s)
 {

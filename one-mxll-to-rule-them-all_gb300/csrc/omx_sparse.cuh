@@ -110,7 +110,7 @@ __global__ void k_emit(FieldPtrs<R> F, Lay L, EmitArgs A, StepParam move_p)
         const double old = A.dipole[3 * n + a];
         const double nw = d * u[a];
         A.dipole[3 * n + a] = nw;
-        A.dPdt[3 * n + a] = A.inv_dt != 0.0 ? (nw - old) * A.inv_dt : (nw - old) / A.dt;
+        A.dPdt[3 * n + a] = over_dt(nw - old, A.over);
         A.E[3 * n + a] = E[a];
     }
 }
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(64) k_emit_lanes(FieldPtrs<R> F, Lay L, EmitAr
         const double old = A.dipole[3 * n + l];
         const double nw = d * u[l];
         A.dipole[3 * n + l] = nw;
-        A.dPdt[3 * n + l] = A.inv_dt != 0.0 ? (nw - old) * A.inv_dt : (nw - old) / A.dt;
+        A.dPdt[3 * n + l] = over_dt(nw - old, A.over);
         A.E[3 * n + l] = E;
     }
 }
@@ -182,7 +182,7 @@ __global__ void k_scatter(JState J, ScatArgs S, StepParam move_p)
         const double jn = (w >= 0) ? S.wk[p] * S.dPdt[3 * w + c] : jo;
         J.Jo[c][p] = jo;
         J.J[c][p] = jn;
-        J.dJ[c][p] = S.inv_dt != 0.0 ? (jn - jo) * S.inv_dt : (jn - jo) / S.dt;
+        J.dJ[c][p] = over_dt(jn - jo, S.over);
     }
 }
 

@@ -20,25 +20,6 @@
 
 namespace omx {
 
-// x / dr of the exact path, correctly rounded, in four FP64 operations: a quotient good to one ulp
-// from 1/dr held as the sum of two doubles (Brisebarre, Muller and Raina, "Accelerating correctly
-// rounded floating-point division when the divisor is known in advance", IEEE TC 53(8), 2004),
-// then Markstein's correction (IBM J. R&D 34(1), 1990): the remainder x - q dr is exact and
-// q + rem * RN(1/dr) rounds to the quotient.  Arguments whose quotient or remainder could leave
-// the normal range (and zeros, infinities, NaN) take the division.  The FP64 pipe bounds the exact
-// path (2 operations per SM and cycle); with a division per CPML term a 128^3 step took 394 us,
-// with this 326 us.
-__device__ __forceinline__ double div_dr(double x, double dr, double rh, double rl)
-{
-    const unsigned e = (unsigned)(__double2hiint(x) & 0x7ff00000) - 0x0c800000u;   // 2^-823 <= |x| < 2^824
-    if (e < 0x66f00000u && rh != 0.0) {
-        const double q = __fma_rn(x, rh, __dmul_rn(x, rl));
-        return __fma_rn(__fma_rn(-q, dr, x), rh, q);
-    }
-    if (x == 0.0) return x;   // dr > 0: the sign of zero stays
-    return x / dr;
-}
-
 template <class R, bool EXACT>
 __device__ __forceinline__ R psi3(R b, R psi, R c, R d, const GridArgs<R> &G)
 {
@@ -91,6 +72,39 @@ __device__ __forceinline__ R ade_update(R e, R rot, const ClsR<R> &cl, int c, lo
     return t;
 }
 
+// The ADE of one dispersive component-cell: ade_update's terms in the same order, each product
+// added by an explicitly rounded FMA (so that no tile shape or code path contracts differently),
+// with the pole state read again in the second loop instead of held in register arrays (which
+// would take registers from the whole pass).  st: the cell's state at slot 0 (PD), V: the slot stride, P:
+// poles per cell in the state.
+__device__ __forceinline__ float f3t_ade(float e, float rot, int type, const MedR<float> *mp, float *st, long long V,
+                                         int P)
+{
+    const MedR<float> &m = *mp;
+    const float PD = st[0];
+    if (type == CLS_DRUDE) {
+        const float t = __fmaf_rn(-m.C4, PD, __fmaf_rn(m.C3, rot, __fmul_rn(m.C1, e)));
+        st[0] = __fmaf_rn(m.A1, PD, __fmul_rn(m.A2, __fadd_rn(t, e)));
+        return t;
+    }
+    const float eo = st[V];
+    float t = __fmaf_rn(-m.C4, PD, __fmaf_rn(m.C3, rot, __fmaf_rn(m.C2, eo, __fmul_rn(m.C1, e))));
+    const int np = m.np;
+#pragma unroll 1
+    for (int p = 0; p < np; ++p)
+        t = __fmaf_rn(-m.B2[p], st[(2 + P + p) * V], __fmaf_rn(-m.B1[p], st[(2 + p) * V], t));
+    st[0] = __fmaf_rn(m.A1, PD, __fmul_rn(m.A2, __fadd_rn(t, e)));
+    const float dte = __fsub_rn(t, eo);
+#pragma unroll 1
+    for (int p = 0; p < np; ++p) {
+        const float pl = st[(2 + p) * V], plo = st[(2 + P + p) * V];
+        st[(2 + P + p) * V] = pl;
+        st[(2 + p) * V] = __fmaf_rn(m.al[p], pl, __fmaf_rn(m.be[p], plo, __fmul_rn(m.ga[p], dte)));
+    }
+    st[V] = e;
+    return t;
+}
+
 // Bulk update of one E component inside the media box.  Vacuum and dielectric classes update
 // here (E + dt_eps0*eps_inv*rotH); dispersive classes were already advanced by k_ade in this
 // half-step and only receive their CPML terms from the bulk pass.
@@ -138,6 +152,11 @@ __global__ void k_ade(FieldPtrs<R> F, GridArgs<R> G)
     const long long idx = L.off + en.x + (long long)L.px * en.y + L.pz * en.z;
     const ClsR<R> cl = G.cls[G.mat[c][b]];
     R *E = F.f[c];
+    if constexpr (sizeof(R) == 4)
+        if (L.dims == 1) {   // the time loop in one launch rounds the same way
+            E[idx] = f3t_ade(E[idx], rot, cl.type, G.med + cl.medium, G.ade + (long long)c * (2 + 2 * G.P) * G.bbV + b, G.bbV, G.P);
+            return;
+        }
     E[idx] = ade_update<R>(E[idx], rot, cl, c, b, G);
 }
 
@@ -511,7 +530,35 @@ __global__ void __launch_bounds__(128) k_e2(FieldPtrs<R> F, GridArgs<R> G, int j
 }
 
 // ===================================================================================== 1D
-// Ex(1:n), Hy(1:n-1) on the single axis (mxll_1D_mod.f90:252-355).
+// Ex(1:n), Hy(1:n-1) on the single axis (mxll_1D_mod.f90:252-355).  The FP32 operations are rounded
+// explicitly: the per-launch kernels and the time loop in one launch (omx_run1d.cuh) are compiled in
+// different units and give the same bits.
+template <class R, bool EXACT> __device__ __forceinline__ R fma1(R a, R b, R c)   // a * b + c
+{
+    if constexpr (EXACT) return a * b + c;
+    else return __fmaf_rn(a, b, c);
+}
+// new Hy(i) from d = Ex(i) - Ex(i+1), and the CPML term, which advances the cell's psi
+template <class R, bool EXACT> __device__ __forceinline__ R h1_bulk(const GridArgs<R> &G, R d, R den, R hy)
+{
+    return fma1<R, EXACT>(G.dt_mu0 * d, den, hy);
+}
+template <class R, bool EXACT>
+__device__ __forceinline__ R h1_absorb(const GridArgs<R> &G, R d, R b, R c, R &psi, R hy)
+{
+    if constexpr (EXACT) psi = psi3<R, true>(b, psi, c, d, G);
+    else psi = __fmaf_rn(b, psi, __fmul_rn(c, d));
+    return fma1<R, EXACT>(G.dt_mu0, psi, hy);
+}
+// CPML term of new Ex(i), d = Hy(i-1) - Hy(i)
+template <class R, bool EXACT>
+__device__ __forceinline__ R e1_absorb(const GridArgs<R> &G, R d, R b, R c, R &psi, R ex)
+{
+    if constexpr (EXACT) psi = psi2<R, true>(b, psi, c, d, G);
+    else psi = __fmaf_rn(b, psi, __fmul_rn(c, d));
+    return fma1<R, EXACT>(G.dt_eps0, psi, ex);
+}
+
 template <class R, bool EXACT>
 __global__ void k_h1(FieldPtrs<R> F, GridArgs<R> G)
 {
@@ -519,45 +566,34 @@ __global__ void k_h1(FieldPtrs<R> F, GridArgs<R> G)
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     if (G.step_inc && i == 1) *G.step_inc += 1;   // device-loop step counter
     if (i > L.nx - 1) return;
-    R *__restrict__ Ex = F.f[0];
-    R *__restrict__ Hy = F.f[4];
     const long long idx = L.off + i;
-    const R d = Ex[idx] - Ex[idx + 1];
-    R hy = Hy[idx] + G.dt_mu0 * d * G.den_h[0][i];
+    const R d = F.f[0][idx] - F.f[0][idx + 1];
+    R hy = h1_bulk<R, EXACT>(G, d, G.den_h[0][i], F.f[4][idx]);
     const int l = G.lH[0][i];
-    if (l >= 0) {
-        const R v = psi3<R, EXACT>(G.bH[0][i], G.psiH[0][0][l], G.cH[0][i], d, G);
-        G.psiH[0][0][l] = v;
-        hy = hy + G.dt_mu0 * v;
-    }
-    Hy[idx] = hy;
+    if (l >= 0) hy = h1_absorb<R, EXACT>(G, d, G.bH[0][i], G.cH[0][i], G.psiH[0][0][l], hy);
+    F.f[4][idx] = hy;
 }
 
+// after k_ade
 template <class R, bool EXACT>
 __global__ void k_e1(FieldPtrs<R> F, GridArgs<R> G)
 {
     const Lay L = G.L;
     const int i = 2 + blockIdx.x * blockDim.x + threadIdx.x;
     if (i > L.nx - 1) return;
-    R *__restrict__ Ex = F.f[0];
-    R *__restrict__ Hy = F.f[4];
     const long long idx = L.off + i;
-    const R d = Hy[idx - 1] - Hy[idx];
+    const R d = F.f[4][idx - 1] - F.f[4][idx];
     const R r = d * G.den_e[0][i];
-    R ex = Ex[idx];
+    R ex = F.f[0][idx];
     if (i >= G.bb0[0] && i <= G.bb1[0]) {
-        const long long b = i - G.bb0[0];
-        ex = plain_update<R>(ex, r, G.mat[0][b], G);
+        const ClsR<R> cl = G.cls[G.mat[0][i - G.bb0[0]]];
+        if (cl.type == CLS_PLAIN) ex = fma1<R, EXACT>(cl.coef, r, ex);
     } else {
-        ex = ex + G.dt_eps0 * r;
+        ex = fma1<R, EXACT>(G.dt_eps0, r, ex);
     }
     const int l = G.lE[0][i];
-    if (l >= 0) {
-        const R v = psi2<R, EXACT>(G.bE[0][i], G.psiE[0][0][l], G.cE[0][i], d, G);
-        G.psiE[0][0][l] = v;
-        ex = ex + G.dt_eps0 * v;
-    }
-    Ex[idx] = ex;
+    if (l >= 0) ex = e1_absorb<R, EXACT>(G, d, G.bE[0][i], G.cE[0][i], G.psiE[0][0][l], ex);
+    F.f[0][idx] = ex;
 }
 
 // ===================================================================================== launchers

@@ -366,3 +366,51 @@ def test_inplace_batch_equals_solo_and_staged():
         b.kill()
         for g, _ in grids:
             g.kill()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("n,bnd,skip", [
+    (64, 3, 1), (71, 1, 2),
+    (3072, 3, 1),                            # eight blocks of 384 cell threads: one cell each
+    (3073, 3, 2), (3079, 1, 1), (6151, 3, 1),
+])
+def test_one_launch_1d_loop(n, bnd, skip, precision):
+    """The 1D time loop in one launch against one launch per phase, bit for bit: a dielectric, a
+    Drude and a Drude-Lorentz layer, two groups that share cells (one inside a layer), three sources
+    on one cell or side by side, samples, several calls."""
+    ev, fs = omx.UNITS["ev_to_au"], omx.UNITS["fs_to_au"]
+    dr = 18.9
+    dt = omx.units.yee_dt(dr)
+    q = n // 8
+    m = np.zeros(n, np.int32)
+    m[4 * q:4 * q + 5], m[5 * q:5 * q + 4], m[6 * q:6 * q + 3] = 1, 2, 3
+    out = []
+    for graph in (True, False):
+        g = omx.TMxll(1, (n,), 5, (bnd, 1, 1), dt, dr, precision=precision)
+        g.set_media([omx.medium_dielectric(4.0), omx.medium_drude(9.17 * ev, 0.02 * ev, 1.0, dt),
+                     omx.medium_dl_custom(5.9, 9.0, 0.07, [2.7, 3.9], [1.0, 0.6], [0.3, 0.5], dt)], m)
+        g.add_plane_source(1, 1, 3 * q, 1e-2, 2.0 * ev, 1.0 * fs, 2.0 * fs, 0.0, 1e30)
+        g.add_source("x", 1e-2, 2.5 * ev, 1.0 * fs, 2.0 * fs, [(3 * q - n // 2) * dr], 4 * dr, 0.0, 1e30)
+        g.add_plane_source(1, 1, 3 * q + 1, 1e-2, 3.0 * ev, 1.0 * fs, 2.0 * fs, 0.0, 0.5 * fs)
+        groups = []
+        r = np.random.default_rng(n + 1)
+        for model, ne in ((1, 9), (2, 5)):
+            cells = (3 * q + 2 + r.integers(0, 2 * q, ne))[:, None].astype(np.int32)
+            cells[:2, 0] = 3 * q, 5 * q + 2
+            par = [np.full((ne, model), 2.5 * ev), np.full((ne, model), 2.0), np.full((ne, 1), 4e4),
+                   np.full((ne, 1), 4e3), r.uniform(0.2, 1.0, (ne, 3))]
+            groups.append(g.add_q_group(omx.Q_MATERIAL, model, cells, np.concatenate(par, 1), 1e-4, skip * dt))
+        for p in (2, 3 * q, 5 * q + 1, n - 1):
+            g.add_detector(omx.POINT, "Ex", [[p]])
+        f = np.zeros([h - b + 1 for b, h in zip(*g.field_bounds(1))], order="F")
+        a0 = 1 - g.field_bounds(1)[0][0]
+        f[a0 + 1:a0 + n - 1] = (1e-3 * np.random.default_rng(n).standard_normal(n - 2)).reshape((n - 2,) + f.shape[1:])
+        g.write_field(1, f)
+        for tt, k in ((1, 2), (3, 1), (4, 33)):
+            g.run(tt, k, skip, 3, use_graph=graph)
+        out.append([np.concatenate([v.ravel() for v in g.drain_detectors()])] + [g.read_field(x) for x in (1, 5)] +
+                   [v for gr in groups for v in gr.read().values()])
+        g.kill()
+    assert all(np.max(np.abs(v)) > 0 for v in out[0][:3]) and np.max(np.abs(out[0][-1])) > 0
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
