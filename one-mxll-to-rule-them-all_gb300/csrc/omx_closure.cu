@@ -55,7 +55,7 @@ constexpr int GEMM_MAX_DEV = 64;
 // (small training GEMMs keep every SM busy).  A CTA holds two
 // accumulators of TMEM_COLS columns; its shared memory is padded so that no more CTAs share an SM
 // than its 512 TMEM columns hold (an allocation beyond them would wait for a CTA to finish).
-template <int BN, int STAGES>
+template <int BN, int STAGES, int CELL>
 static cudaError_t gemm_launch_s(const CUtensorMap &ta, const CUtensorMap &tb, int K, const GemmEpi &E, cudaStream_t s)
 {
     using S = GemmSmem<BN, STAGES>;
@@ -67,7 +67,7 @@ static cudaError_t gemm_launch_s(const CUtensorMap &ta, const CUtensorMap &tb, i
     const int per_sm = 512 / (2 * (int)S::TMEM_COLS);
     const int bytes = std::max(S::BYTES, 233472 / (per_sm + 1) + 1024);
     if (!attr[di]) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<BN, STAGES, CELL>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms[di], cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return e;
         attr[di] = 1;
@@ -77,17 +77,37 @@ static cudaError_t gemm_launch_s(const CUtensorMap &ta, const CUtensorMap &tb, i
     const int mt = (E.M + 127) / 128, tiles = mt * ((E.N + BN - 1) / BN);
     const int cap = std::max(1, 2 * sms[di] / std::max(1, splits));
     GemmEpi Ep = E;
+    // a launch that fills the device has nothing to gain from the next one's early start (20000 rows,
+    // 32 steps: 2.38 ms chained, 1.99 ms not)
+    Ep.chained = E.chained && tiles <= sms[di];
     Ep.row_major_tiles = mt >= 2 * cap ? 1 : 0;
     const int px = Ep.row_major_tiles ? cap : std::min(tiles, cap);
     const dim3 grid((unsigned)px, 1, (unsigned)splits);
-    k_gemm_tc<BN, STAGES><<<grid, GEMM_THREADS, bytes, s>>>(ta, tb, K, Ep);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = (size_t)bytes;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = Ep.chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, STAGES, CELL>, ta, tb, K, Ep);
 }
 template <int BN>
 static cudaError_t gemm_launch(const CUtensorMap &ta, const CUtensorMap &tb, int K, const GemmEpi &E, cudaStream_t s)
 {
     const int nk = (E.kpz > 0 ? E.kpz : (K + 63) / 64);
-    return nk <= 4 ? gemm_launch_s<BN, 2>(ta, tb, K, E, s) : gemm_launch_s<BN, 4>(ta, tb, K, E, s);
+    if constexpr (BN == 32) {   // recurrent steps alone: every K block in flight at once
+        return E.gru_h ? gemm_launch_s<BN, 4, EPI_GRU>(ta, tb, K, E, s) : gemm_launch_s<BN, 4, EPI_BWD>(ta, tb, K, E, s);
+    } else {
+        if constexpr (BN >= 64) {
+            if (E.gru_h) return gemm_launch_s<BN, 2, EPI_GRU>(ta, tb, K, E, s);
+            if (E.bwd_dG) return gemm_launch_s<BN, 4, EPI_BWD>(ta, tb, K, E, s);
+        }
+        return nk <= 4 ? gemm_launch_s<BN, 2, EPI_PLAIN>(ta, tb, K, E, s) : gemm_launch_s<BN, 4, EPI_PLAIN>(ta, tb, K, E, s);
+    }
 }
 
 // D = act(alpha * A * B^T + bias) on device buffers; A [M x K] (lda), B [N x K] (ldb) in BF16.
@@ -104,7 +124,15 @@ bool gemm_bf16(const uint16_t *A, int lda, const uint16_t *B, int ldb, int K, co
         err = "gemm: rows must be 16-byte aligned";
         return false;
     }
-    const int BN = E.N <= 16 ? 16 : (E.N <= 64 ? 64 : 128);
+    // Few row tiles of a recurrent step: narrower column tiles, down to one 16-column chunk per epilogue
+    // warp, while the tiles stay within one per SM.  A step is latency alone: for 256 rows, both
+    // directions took 36 us in six launches (input, 128-column GEMM, cell) and take 12 us in two
+    // (gradient of 129 steps 5.7 -> 2.3 ms); a forward pass of 20000 rows, 32 steps 3.4 -> 1.9 ms.
+    int BN = E.N <= 16 ? 16 : (E.N <= 64 ? 64 : 128);
+    if (E.gru_h || E.bwd_dG) {
+        const long long mt = (E.M + 127) / 128;
+        while (BN > 32 && mt * (E.N / (BN / 2)) <= 152) BN /= 2;
+    }
     CUtensorMap ta, tb;
     if (!tmap_bf16(&ta, A, (unsigned long long)E.M, (unsigned long long)K, (unsigned long long)lda, 128) ||
         !tmap_bf16(&tb, B, (unsigned long long)E.N, (unsigned long long)K, (unsigned long long)ldb, (unsigned)BN)) {
@@ -113,6 +141,7 @@ bool gemm_bf16(const uint16_t *A, int lda, const uint16_t *B, int ldb, int K, co
     }
     cudaError_t e;
     if (BN == 16) e = gemm_launch<16>(ta, tb, K, E, s);
+    else if (BN == 32) e = gemm_launch<32>(ta, tb, K, E, s);
     else if (BN == 64) e = gemm_launch<64>(ta, tb, K, E, s);
     else e = gemm_launch<128>(ta, tb, K, E, s);
     if (e != cudaSuccess) {
@@ -215,7 +244,6 @@ __device__ __forceinline__ bool cl_wg_masked(int row, int col)
 {
     return (row >= 2 * CL_H && row < 3 * CL_H && col >= CL_W) || (row >= 3 * CL_H && col < CL_W);
 }
-__device__ __forceinline__ float cl_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // FP32 master -> BF16 weights (row-major and transposed), masked Wg, padded read-out row
 // row of the gate weights in the deployment order: tile b of 128 rows holds hidden units
@@ -262,40 +290,17 @@ __global__ void k_cl_refresh(const float *__restrict__ p, uint16_t *wg, uint16_t
     if (n < CL_OUT) b4pad[n] = n == 0 ? p[CL_OFF_B4] : 0.f;
 }
 
-// XH row of step t: window e[b, t .. t+W-1] (row stride lde) and the previous hidden state
-__global__ void k_cl_build_xh(const float *__restrict__ e, long long lde, int t, const float *__restrict__ hprev,
-                              uint16_t *__restrict__ xh, int B)
+// window columns of the XH rows of every step (step t of sequence b: e[b, t .. t+W-1], row stride lde;
+// rows t*B + b), and the zero hidden state of step 0; the GRU epilogue writes the other hidden columns
+__global__ void k_cl_build_xh(const float *__restrict__ e, long long lde, uint16_t *__restrict__ xh, int B, long long TB)
 {
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (q >= (long long)B * CL_XH) return;
-    const int b = (int)(q / CL_XH), c = (int)(q % CL_XH);
-    const float v = c < CL_W ? e[b * lde + t + c] : (hprev ? hprev[(long long)b * CL_H + (c - CL_W)] : 0.f);
-    xh[q] = f32_to_bf16_rn(v);
-}
-
-// GRU cell: gates G [B x 512] (pre-activations, biases included) -> h_t (FP32 and BF16); the
-// activations r, z, n and the nh pre-activation are kept for the backward pass when cache != null
-__global__ void k_cl_gru_fwd(const float *__restrict__ G, const float *hprev, float *h, uint16_t *__restrict__ hb,
-                             float *__restrict__ cache, int B, const int *skip)
-{
-    const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (q >= (long long)B * CL_H || (skip && *skip)) return;
-    const int b = (int)(q / CL_H), j = (int)(q % CL_H);
-    const float *g = G + (long long)b * CL_G;
-    const float r = cl_sigmoid(g[j]), z = cl_sigmoid(g[CL_H + j]);
-    const float nh = g[3 * CL_H + j];
-    const float n = tanhf(g[2 * CL_H + j] + r * nh);
-    const float hp = hprev ? hprev[q] : 0.f;
-    const float hn = (1.0f - z) * n + z * hp;
-    h[q] = hn;
-    hb[q] = f32_to_bf16_rn(hn);
-    if (cache) {
-        float *c = cache + (long long)b * 4 * CL_H;
-        c[j] = r;
-        c[CL_H + j] = z;
-        c[2 * CL_H + j] = n;
-        c[3 * CL_H + j] = nh;
+    if (q < TB * CL_W) {
+        const long long row = q / CL_W;
+        const int c = (int)(q % CL_W);
+        xh[row * CL_XH + c] = f32_to_bf16_rn(e[(row % B) * lde + row / B + c]);
     }
+    if (q < (long long)B * CL_H) xh[q / CL_H * CL_XH + CL_W + q % CL_H] = 0;
 }
 
 // loss and its gradient: y = Y[:, 0] (rows t*B + b), target [T][B]; steps t < skip do not count
@@ -318,39 +323,20 @@ __global__ void k_cl_loss(const float *__restrict__ Y, const float *__restrict__
     if ((threadIdx.x & 31) == 0 && part != 0.0) atomicAdd(loss, part);
 }
 
-// GRU backward of step t: dh = dHm_t + dh_next -> dG_t (BF16, gate pre-activation gradients)
-// and the direct part of dh_prev (dh * z)
-__global__ void k_cl_gru_bwd(const float *__restrict__ dHm, const float *__restrict__ dh_next,
-                             const float *__restrict__ cache, const float *__restrict__ hprev,
-                             uint16_t *__restrict__ dG, float *__restrict__ dh_direct, int B)
-{
-    const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (q >= (long long)B * CL_H) return;
-    const int b = (int)(q / CL_H), j = (int)(q % CL_H);
-    const float *c = cache + (long long)b * 4 * CL_H;
-    const float r = c[j], z = c[CL_H + j], n = c[2 * CL_H + j], nh = c[3 * CL_H + j];
-    const float hp = hprev ? hprev[q] : 0.f;
-    const float dh = dHm[q] + (dh_next ? dh_next[q] : 0.f);
-    const float dn = dh * (1.0f - z);
-    const float dz = dh * (hp - n) * z * (1.0f - z);
-    const float dpn = dn * (1.0f - n * n);
-    const float dr = dpn * nh * r * (1.0f - r);
-    uint16_t *g = dG + (long long)b * CL_G;
-    g[j] = f32_to_bf16_rn(dr);
-    g[CL_H + j] = f32_to_bf16_rn(dz);
-    g[2 * CL_H + j] = f32_to_bf16_rn(dpn);
-    g[3 * CL_H + j] = f32_to_bf16_rn(dpn * r);
-    dh_direct[q] = dh * z;
-}
-
-// dh_prev = dXH[:, W:] + dh_direct
-__global__ void k_cl_dh_prev(const float *__restrict__ dXH, const float *__restrict__ dh_direct, float *__restrict__ out,
+// GRU backward of the last step (the others are the epilogue of the GEMM before them): dh = dHm
+__global__ void k_cl_gru_bwd(const float *__restrict__ dHm, const float *__restrict__ cache,
+                             const float *__restrict__ hprev, uint16_t *__restrict__ dG, float *__restrict__ dh_direct,
                              int B)
 {
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (q >= (long long)B * CL_H) return;
     const int b = (int)(q / CL_H), j = (int)(q % CL_H);
-    out[q] = dXH[(long long)b * CL_XH + CL_W + j] + dh_direct[q];
+    const float *c = cache + (long long)b * 4 * CL_H;
+    const GruGrad w = gru_grad(dHm[q], c[j], c[CL_H + j], c[2 * CL_H + j], c[3 * CL_H + j], hprev ? hprev[q] : 0.f);
+    uint16_t *g = dG + (long long)b * CL_G;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) g[k * CL_H + j] = f32_to_bf16_rn(w.g[k]);
+    dh_direct[q] = w.dhd;
 }
 
 // BF16 transpose [R x C] -> [C x R] (32 x 32 tiles through shared memory)
@@ -376,7 +362,14 @@ __global__ void k_cl_rowsum(const uint16_t *__restrict__ src, int rows, long lon
     const int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
     if (row >= rows) return;
     float s = 0.f;
-    for (long long k = lane; k < n; k += 32) s += __bfloat162float(__ushort_as_bfloat16(src[row * ld + k]));
+    const uint16_t *a = src + row * ld;
+    for (long long k = lane; k < n; k += 32 * 64) {     // 64 loads in flight, added in order
+        uint16_t v[64];
+#pragma unroll
+        for (int q = 0; q < 64; ++q) v[q] = k + 32 * q < n ? a[k + 32 * q] : (uint16_t)0;
+#pragma unroll
+        for (int q = 0; q < 64; ++q) s += __bfloat162float(__ushort_as_bfloat16(v[q]));
+    }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (lane == 0) out[row] = s;
 }
@@ -442,7 +435,7 @@ struct omx_closure {
     omx::DBuf<float> p, g, m, v, b4pad, bgp;
     omx::DBuf<uint16_t> wg, wgT, w1, w1T, w2, w2T, w3, w3T, w4, w4T, wgp;   // wgp, bgp: deployment gate order
     // training / batch work buffers (grown on demand)
-    omx::DBuf<float> e, tgt, G, H, cache, A1, A2, A3, Y, dHm, dXH, dh, dhd, part;
+    omx::DBuf<float> e, tgt, G, H, cache, A1, A2, A3, Y, dHm, dhd, part;
     omx::DBuf<uint16_t> XH, Hb, A1b, A2b, A3b, dY, dZ1, dZ2, dZ3, dG, T1, T2;
     omx::DBuf<double> loss;
     omx::DBuf<int> err;
@@ -492,30 +485,34 @@ static bool cl_forward(omx_closure *c, int B, int T, bool keep, std::string &err
 {
     const long long TB = (long long)T * B;
     CL_NEED(c->XH, (size_t)TB * CL_XH);
-    CL_NEED(c->G, (size_t)B * CL_G);
-    CL_NEED(c->H, (size_t)TB * CL_H);
+    CL_NEED(c->H, (size_t)(keep ? TB : B) * CL_H);
     CL_NEED(c->Hb, (size_t)TB * CL_H);
-    CL_NEED(c->cache, (size_t)(keep ? TB : B) * 4 * CL_H);
-    CL_NEED(c->A1, (size_t)TB * CL_F);
-    CL_NEED(c->A2, (size_t)TB * CL_F);
-    CL_NEED(c->A3, (size_t)TB * CL_F);
+    if (keep) {
+        CL_NEED(c->cache, (size_t)TB * 4 * CL_H);
+        CL_NEED(c->A1, (size_t)TB * CL_F);
+        CL_NEED(c->A2, (size_t)TB * CL_F);
+        CL_NEED(c->A3, (size_t)TB * CL_F);
+    }
     CL_NEED(c->A1b, (size_t)TB * CL_F);
     CL_NEED(c->A2b, (size_t)TB * CL_F);
     CL_NEED(c->A3b, (size_t)TB * CL_F);
     CL_NEED(c->Y, (size_t)TB * CL_OUT);
     const long long lde = T + CL_W - 1;
+    k_cl_build_xh<<<cl_blocks(std::max(TB * CL_W, (long long)B * CL_H)), 256, 0, c->stream>>>(c->e.p, lde, c->XH.p, B, TB);
     for (int t = 0; t < T; ++t) {
-        const float *hprev = t > 0 ? c->H.p + (long long)(t - 1) * B * CL_H : nullptr;
-        uint16_t *xh = c->XH.p + (long long)t * B * CL_XH;
-        k_cl_build_xh<<<cl_blocks((long long)B * CL_XH), 256, 0, c->stream>>>(c->e.p, lde, t, hprev, xh, B);
+        // gates, GRU cell and the next step's input in one launch; h stays in place when no backward
+        // pass reads it
+        const long long at = keep ? (long long)t * B : 0, was = keep ? at - B : 0;
         GemmEpi E = cl_epi(c, B, CL_G);
-        E.d_f32 = c->G.p;
-        E.ld_f32 = CL_G;
-        E.bias = c->p.p + CL_OFF_BG;
-        if (!gemm_bf16(xh, CL_XH, c->wg.p, CL_XH, CL_XH, E, c->stream, err)) return false;
-        k_cl_gru_fwd<<<cl_blocks((long long)B * CL_H), 256, 0, c->stream>>>(
-            c->G.p, hprev, c->H.p + (long long)t * B * CL_H, c->Hb.p + (long long)t * B * CL_H,
-            c->cache.p + (keep ? (long long)t * B * 4 * CL_H : 0), B, nullptr);
+        E.bias = c->bgp.p;
+        E.gru_h = c->H.p + at * CL_H;
+        E.gru_hp = t > 0 ? c->H.p + was * CL_H : nullptr;
+        E.gru_hb = c->Hb.p + (long long)t * B * CL_H;
+        E.gru_xh = t < T - 1 ? c->XH.p + (long long)(t + 1) * B * CL_XH : nullptr;
+        E.gru_round_h = 1;
+        E.chained = 1;
+        E.gru_cache = keep ? c->cache.p + at * 4 * CL_H : nullptr;
+        if (!gemm_bf16(c->XH.p + (long long)t * B * CL_XH, CL_XH, c->wgp.p, CL_XH, CL_XH, E, c->stream, err)) return false;
     }
     // MLP on all T*B rows at once
     struct Layer {
@@ -527,10 +524,10 @@ static bool cl_forward(omx_closure *c, int B, int T, bool keep, std::string &err
         uint16_t *outb;
     } L[3] = {{c->Hb.p, CL_H, c->w1.p, CL_OFF_B1, c->A1.p, c->A1b.p},
               {c->A1b.p, CL_F, c->w2.p, CL_OFF_B2, c->A2.p, c->A2b.p},
-              {c->A2b.p, CL_F, c->w3.p, CL_OFF_B3, c->A3.p, c->A3b.p}};
+              {c->A2b.p, CL_F, c->w3.p, CL_OFF_B3, c->A3.p, c->A3b.p}};   // FP32 for the backward pass
     for (auto &l : L) {
         GemmEpi E = cl_epi(c, (int)TB, CL_F);
-        E.d_f32 = l.out;
+        E.d_f32 = keep ? l.out : nullptr;
         E.ld_f32 = CL_F;
         E.d_bf16 = l.outb;
         E.ld_bf16 = CL_F;
@@ -548,9 +545,10 @@ static bool cl_forward(omx_closure *c, int B, int T, bool keep, std::string &err
 }
 
 // dW [N x K] = sum over rows of dZ[:, n] * X[:, k]: one long-K GEMM over the T*B rows (both
-// operands transposed first), split over K and reduced in a fixed order
+// operands transposed first), split over K and reduced in a fixed order; the bias gradient, sums of
+// the first nbias columns of dZ, from the same transpose (one warp per column, fixed order)
 static bool cl_weight_grad(omx_closure *c, const uint16_t *dZ, int N, const uint16_t *X, int K, long long TB, float *out,
-                           int wg_mask, std::string &err)
+                           float *bias, int nbias, int wg_mask, std::string &err)
 {
     const int ldT = (int)((TB + 7) / 8 * 8);
     CL_NEED(c->T1, (size_t)N * ldT);
@@ -570,19 +568,7 @@ static bool cl_weight_grad(omx_closure *c, const uint16_t *dZ, int N, const uint
     if (!gemm_bf16(c->T1.p, ldT, c->T2.p, ldT, (int)TB, E, c->stream, err)) return false;
     k_cl_reduce<<<cl_blocks((long long)N * K), 256, 0, c->stream>>>(c->part.p, splits, (long long)N * K, out, wg_mask,
                                                                    K);
-    CL_CK(cudaGetLastError());
-    return true;
-}
-
-// bias gradient: sums of the first N columns of a BF16 [TB x ld] matrix (through its
-// transpose, one warp per column, fixed order)
-static bool cl_bias_grad(omx_closure *c, const uint16_t *dZ, int N, int ld, long long TB, float *out, std::string &err)
-{
-    const int ldT = (int)((TB + 7) / 8 * 8);
-    CL_NEED(c->T1, (size_t)N * ldT);
-    k_cl_transpose<<<dim3((N + 31) / 32, (unsigned)((TB + 31) / 32)), dim3(32, 8), 0, c->stream>>>(dZ, (int)TB, N, ld,
-                                                                                                 c->T1.p, ldT);
-    k_cl_rowsum<<<(N + 7) / 8, 256, 0, c->stream>>>(c->T1.p, N, TB, ldT, out);
+    k_cl_rowsum<<<(nbias + 7) / 8, 256, 0, c->stream>>>(c->T1.p, nbias, TB, ldT, bias);
     CL_CK(cudaGetLastError());
     return true;
 }
@@ -598,8 +584,6 @@ static bool cl_gradient(omx_closure *c, int B, int T, int skip, std::string &err
     CL_NEED(c->dZ3, (size_t)TB * CL_F);
     CL_NEED(c->dHm, (size_t)TB * CL_H);
     CL_NEED(c->dG, (size_t)TB * CL_G);
-    CL_NEED(c->dXH, (size_t)B * CL_XH);
-    CL_NEED(c->dh, (size_t)B * CL_H);
     CL_NEED(c->dhd, (size_t)B * CL_H);
     CL_CK(cudaMemsetAsync(c->loss.p, 0, sizeof(double), c->stream));
     k_cl_loss<<<cl_blocks(TB), 256, 0, c->stream>>>(c->Y.p, c->tgt.p, B, T, skip, c->dY.p, c->loss.p);
@@ -629,34 +613,33 @@ static bool cl_gradient(omx_closure *c, int B, int T, int skip, std::string &err
     // weight and bias gradients of the MLP
     CL_NEED(c->part, (size_t)CL_OUT * CL_F);
     float *g = c->g.p;
-    if (!cl_weight_grad(c, c->dZ3.p, CL_F, c->A2b.p, CL_F, TB, g + CL_OFF_W3, 0, err)) return false;
-    if (!cl_weight_grad(c, c->dZ2.p, CL_F, c->A1b.p, CL_F, TB, g + CL_OFF_W2, 0, err)) return false;
-    if (!cl_weight_grad(c, c->dZ1.p, CL_F, c->Hb.p, CL_H, TB, g + CL_OFF_W1, 0, err)) return false;
-    if (!cl_bias_grad(c, c->dZ3.p, CL_F, CL_F, TB, g + CL_OFF_B3, err)) return false;
-    if (!cl_bias_grad(c, c->dZ2.p, CL_F, CL_F, TB, g + CL_OFF_B2, err)) return false;
-    if (!cl_bias_grad(c, c->dZ1.p, CL_F, CL_F, TB, g + CL_OFF_B1, err)) return false;
+    if (!cl_weight_grad(c, c->dZ3.p, CL_F, c->A2b.p, CL_F, TB, g + CL_OFF_W3, g + CL_OFF_B3, CL_F, 0, err)) return false;
+    if (!cl_weight_grad(c, c->dZ2.p, CL_F, c->A1b.p, CL_F, TB, g + CL_OFF_W2, g + CL_OFF_B2, CL_F, 0, err)) return false;
+    if (!cl_weight_grad(c, c->dZ1.p, CL_F, c->Hb.p, CL_H, TB, g + CL_OFF_W1, g + CL_OFF_B1, CL_F, 0, err)) return false;
     // read-out row: dw4 = dY[:, 0]^T A3, db4 = sum dY[:, 0] (via a 16 x 256 product and row 0)
-    CL_NEED(c->G, (size_t)B * CL_G > (size_t)CL_OUT * CL_F ? (size_t)B * CL_G : (size_t)CL_OUT * CL_F);
-    if (!cl_weight_grad(c, c->dY.p, CL_OUT, c->A3b.p, CL_F, TB, c->G.p, 0, err)) return false;
+    CL_NEED(c->G, (size_t)CL_OUT * CL_F);
+    if (!cl_weight_grad(c, c->dY.p, CL_OUT, c->A3b.p, CL_F, TB, c->G.p, g + CL_OFF_B4, 1, 0, err)) return false;
     CL_CK(cudaMemcpyAsync(g + CL_OFF_W4, c->G.p, sizeof(float) * CL_F, cudaMemcpyDeviceToDevice, c->stream));
-    if (!cl_bias_grad(c, c->dY.p, 1, CL_OUT, TB, g + CL_OFF_B4, err)) return false;
-    // GRU, backward through time
-    for (int t = T - 1; t >= 0; --t) {
-        const float *hprev = t > 0 ? c->H.p + (long long)(t - 1) * B * CL_H : nullptr;
+    // GRU, backward through time: the product of step t's gate gradients with the hidden columns of
+    // the gate weights, and step t - 1's cell in its epilogue
+    auto hprev = [&](int t) { return t > 0 ? c->H.p + (long long)(t - 1) * B * CL_H : nullptr; };
+    {
+        const long long at = (long long)(T - 1) * B;
         k_cl_gru_bwd<<<cl_blocks((long long)B * CL_H), 256, 0, c->stream>>>(
-            c->dHm.p + (long long)t * B * CL_H, t < T - 1 ? c->dh.p : nullptr, c->cache.p + (long long)t * B * 4 * CL_H,
-            hprev, c->dG.p + (long long)t * B * CL_G, c->dhd.p, B);
-        if (t > 0) {
-            GemmEpi E = cl_epi(c, B, CL_XH);
-            E.d_f32 = c->dXH.p;
-            E.ld_f32 = CL_XH;
-            if (!gemm_bf16(c->dG.p + (long long)t * B * CL_G, CL_G, c->wgT.p, CL_G, CL_G, E, c->stream, err))
-                return false;
-            k_cl_dh_prev<<<cl_blocks((long long)B * CL_H), 256, 0, c->stream>>>(c->dXH.p, c->dhd.p, c->dh.p, B);
-        }
+            c->dHm.p + at * CL_H, c->cache.p + at * 4 * CL_H, hprev(T - 1), c->dG.p + at * CL_G, c->dhd.p, B);
     }
-    if (!cl_weight_grad(c, c->dG.p, CL_G, c->XH.p, CL_XH, TB, g + CL_OFF_WG, 1, err)) return false;
-    if (!cl_bias_grad(c, c->dG.p, CL_G, CL_G, TB, g + CL_OFF_BG, err)) return false;
+    for (int t = T - 1; t > 0; --t) {
+        const long long at = (long long)(t - 1) * B;
+        GemmEpi E = cl_epi(c, B, CL_H);
+        E.bwd_dG = c->dG.p + at * CL_G;
+        E.bwd_dHm = c->dHm.p + at * CL_H;
+        E.bwd_cache = c->cache.p + at * 4 * CL_H;
+        E.bwd_hp = hprev(t - 1);
+        E.bwd_dhd = c->dhd.p;
+        E.chained = 1;
+        if (!gemm_bf16(c->dG.p + (at + B) * CL_G, CL_G, c->wgT.p + CL_W * CL_G, CL_G, CL_G, E, c->stream, err)) return false;
+    }
+    if (!cl_weight_grad(c, c->dG.p, CL_G, c->XH.p, CL_XH, TB, g + CL_OFF_WG, g + CL_OFF_BG, CL_G, 1, err)) return false;
     CL_CK(cudaGetLastError());
     return true;
 }
@@ -737,6 +720,7 @@ bool closure_infer(omx_closure *c, const ClDeploy &D, const EmitArgs &A, cudaStr
     GemmEpi E = cl_epi(c, n, CL_G);
     E.bias = c->bgp.p;
     E.gru_h = D.hst;
+    E.gru_hp = D.hst;
     E.gru_hb = D.hb;
     E.skip = skip;
     E.err = D.err;

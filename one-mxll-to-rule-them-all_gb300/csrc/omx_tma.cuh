@@ -60,6 +60,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     return true;
 }
 
+// programmatic dependent launch: let the next launch of the stream start; wait until the launch before
+// has completed and its writes are visible
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // an L2 policy that marks the lines a load brings in as the first to evict (data read once)
 __device__ __forceinline__ uint64_t l2_policy_evict_first()
 {
