@@ -1852,8 +1852,12 @@ template <class R> void run_impl(omx_ctx *c, int tt0, int nsteps, int n_skip, in
         return;
     }
     join_side(c);
-    if (prepare_only) stage_reserve(c, plan);
-    else stage_upload(c, plan, false);
+    if (prepare_only) {
+        stage_reserve(c, plan);
+        c->run_step = c->d_step.p;   // as stage_upload leaves it: the captured steps advance the counter
+    } else {
+        stage_upload(c, plan, false);
+    }
     if (run1_ok(c, nsteps, use_graph)) {
         if (!prepare_only) {
             run1<R>(c, plan, nsteps);

@@ -440,3 +440,29 @@ def test_closure_step_tiles():
         assert abs(l2 - loss) <= 1e-9 * abs(loss)
         assert np.max(np.abs(g2 - g)) <= 1e-3 * np.max(np.abs(g))
     cl.kill()
+
+
+@pytest.mark.parametrize("dims,n,precision,shape", [
+    (1, (200,), "fp64", None), (2, (70, 60), "fp32", None), (2, (70, 60), "fp64", None),
+    (3, (30, 26, 28), "fp32", None), (3, (30, 26, 28), "fp32", 8016), (3, (30, 26, 28), "fp64", None),
+])
+def test_prepared_run_equals_run(dims, n, precision, shape):
+    """A run whose step graphs were captured beforehand steps through its table as any other."""
+    dt = omx.units.yee_dt(37.8)
+    out = []
+    for prepared in (False, True):
+        g = omx.TMxll(dims, n, 4, (3,) * 3, dt, 37.8, mode=omx.TMZ, precision=precision)
+        comp = 3 if dims == 2 else 1
+        g.add_plane_source(comp, dims, n[dims - 1] // 2, 1e-2, 0.1, 8 * dt, 6 * dt, 0.0, 1e30)
+        g.add_detector(omx.POINT, "Ez" if dims == 2 else "Ex", [[m // 2 for m in n]])
+        if shape:
+            g.set_launch_shape(shape)
+        g.run(1, 3, 1, 1)
+        if prepared:
+            g.prepare_run(4, 20, 1, 1)
+        g.run(4, 20, 1, 1)
+        out.append(list(g.drain_detectors()) + [g.read_field(comp)])
+        g.kill()
+    assert np.max(np.abs(out[0][1])) > 0
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
