@@ -618,7 +618,8 @@ def cfg5_decks(count, side_min=64, side_max=256):
 
 
 def batch_shape_text(shape):
-    """(the fused batched pass, its tile) from omx_batch_autotune's choice."""
+    """(the batched pass, its tile) from omx_batch_autotune's choice; grids that each step in place keep
+    that form, side by side, where it timed faster than the staged shape the tuner returns."""
     if shape < 1000:
         return "the two half-step passes of every grid (k_batch3)", "tile depth %d" % shape
     form = shape // 1000 % 1000
@@ -720,7 +721,8 @@ def measure_cfg5(args, dist, K, W, cpu_seconds):
                        "cells": cells, "sides": sides, "precision": "fp32",
                        "parallelism": f"replicas x{dist.world}" if dist.world > 1 else "single GPU",
                        "l2": "working set %.1f GB > 126 MB L2, no flush" % (cells * 6 * 4 / 1e9),
-                       "loop": "omx_batch_run: %s, the steps captured in CUDA graphs; shape from "
+                       "loop": "omx_batch_run: each grid in place on one of the batch's streams where that timed "
+                               "faster, else %s; the steps captured in CUDA graphs; shape from "
                                "omx_batch_autotune: %s" % batch_shape_text(shape),
                        "timing": "wall clock around omx_batch_run + omx_batch_synchronize"},
             "one_at_a_time": {"value": solo_value, "unit": "Gcell-updates/s",
@@ -729,7 +731,7 @@ def measure_cfg5(args, dist, K, W, cpu_seconds):
                               "batch_speedup": value / solo_value,
                               "detector_traces_bit_identical": same,
                               "arithmetic": "one fused pass per grid and step, as the batch"},
-            "roofline": {"bound": "hbm", "kernel": batch_shape_text(shape)[0],
+            "roofline": {"bound": "hbm", "kernel": "k_f3p_h / k_f3p_e side by side, or " + batch_shape_text(shape)[0],
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": None, "peak_source": peak_kind,
                          "algorithmic_bytes_per_step": alg,

@@ -127,11 +127,15 @@ bool gemm_bf16(const uint16_t *A, int lda, const uint16_t *B, int ldb, int K, co
     // Few row tiles of a recurrent step: narrower column tiles, down to one 16-column chunk per epilogue
     // warp, while the tiles stay within one per SM.  A step is latency alone: for 256 rows, both
     // directions took 36 us in six launches (input, 128-column GEMM, cell) and take 12 us in two
-    // (gradient of 129 steps 5.7 -> 2.3 ms); a forward pass of 20000 rows, 32 steps 3.4 -> 1.9 ms.
+    // (gradient of 129 steps 5.7 -> 2.3 ms); a forward pass of 20000 rows, 32 steps 3.4 -> 1.8 ms.
     int BN = E.N <= 16 ? 16 : (E.N <= 64 ? 64 : 128);
     if (E.gru_h || E.bwd_dG) {
         const long long mt = (E.M + 127) / 128;
         while (BN > 32 && mt * (E.N / (BN / 2)) <= 152) BN /= 2;
+        // past that, 32 again up to 32768 rows: the last round of tiles over the SMs is a quarter as
+        // long (forward, 40 steps, columns 128 / 64 / 32: 2000 rows 0.60 / 0.47 / 0.52 ms, 6000 0.95 /
+        // 0.87 / 0.84, 20000 2.31 / 2.21 / 2.13, 32000 3.32 / 3.31 / 3.12)
+        if (E.gru_h && BN == 128 && mt <= 256) BN = 32;
     }
     CUtensorMap ta, tb;
     if (!tmap_bf16(&ta, A, (unsigned long long)E.M, (unsigned long long)K, (unsigned long long)lda, 128) ||

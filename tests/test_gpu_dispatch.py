@@ -430,7 +430,7 @@ def test_closure_step_tiles():
     e = rng.standard_normal((8, T + 31)).astype(np.float32)
     y = cl.forward(e, T)
     assert np.max(np.abs(y)) > 0
-    for copies in (2, 144, 145, 304, 305):       # the last and first rows of each forward tile width
+    for copies in (2, 144, 145, 304, 305, 4097): # the last and first rows of each forward tile width
         yy = cl.forward(np.tile(e, (copies, 1)), T).reshape(T, copies, 8)
         assert np.array_equal(yy, np.broadcast_to(np.asarray(y).reshape(T, 1, 8), yy.shape))
     tgt = rng.standard_normal((T, 8)).astype(np.float32)
