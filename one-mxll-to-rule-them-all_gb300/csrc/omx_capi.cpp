@@ -1706,9 +1706,9 @@ StepParam plan_param(omx_ctx *c, const RunPlan &plan, int row) { return StepPara
 // The 1D time loop in one launch (k_run1): what it leaves to the per-launch kernels are closures,
 // Fourier accumulation, H detectors, points outside the cells 1..n, and numbers of sources, groups,
 // emitters or cells that one cluster would be slow on or has no shared memory for (2048 FP64 cells a
-// block).  Measured, us per step in one launch / in launches, FP64 with a Drude film: 200 cells 3.2 /
-// 12.4, with 16 emitters 1500 cells 7.2 / 24.7, 12000 cells 10.6 / 24.9; 6000 cells with 256 emitters
-// 9.2 / 24.7, 512 13.8 / 26.5, 1024 (all through memory) 24.3 / 26.7.
+// block).  Measured, us per step in one launch / in launches, FP64 with a Drude film: 200 cells 3.1 /
+// 12.4, with 16 emitters 1500 cells 6.5 / 24.7, 12000 cells 8.6 / 24.9; 6000 cells with 256 emitters
+// 8.6 / 24.7, 512 12.9 / 26.5, 1024 (all through memory) 24.3 / 26.7.
 constexpr int RUN1_CELLS = 16384, RUN1_EMITTERS = 512, RUN1_TAPS = 2048;
 bool run1_ok(const omx_ctx *c, int nsteps, int use_graph)
 {

@@ -2,7 +2,7 @@
 // stepping (H, sources, ADE and E with CPML, emitter current, emitters, detectors) with cluster
 // barriers between the phases, instead of eight launches a step that each wait for the one before.
 // A 1D step is latency alone (1500 FP64 cells, a Drude film, 16 emitters and 16 detectors: 24.7 us
-// in launches of a few microseconds each, 7.2 us here); what is left is the FP64 chain of an emitter
+// in launches of a few microseconds each, 6.5 us here); what is left is the FP64 chain of an emitter
 // and of a cell (64 cycles an instruction) and two barriers.
 //
 // Block r owns a contiguous piece of the cells and holds their fields, coefficients and psi in shared
@@ -25,41 +25,68 @@ constexpr int RUN1_CLUSTER = 8, RUN1_THREADS = 512, RUN1_SIDE = 128, RUN1_ROWS =
 
 template <class R> __device__ __forceinline__ R ld_cg(const R *p) { return __ldcg(p); }
 
+// A lane's part of an emitter: constants, state word and dipole component
+struct Run1Emitter {
+    double pr[4], u[3], ul, g1, g2, x, dipole;
+    long long cell;
+    int n;
+    bool live;
+};
+template <int LANES> __device__ __forceinline__ Run1Emitter run1_load(const Lay &L, const EmitArgs &A, int n0, int l)
+{
+    constexpr int NST = LANES == 8 ? 8 : 3;
+    Run1Emitter e;
+    e.live = n0 < A.n;
+    e.n = e.live ? n0 : A.n - 1;          // lanes past the end follow the last emitter, without writes
+    const double *pr = A.par + (long long)e.n * A.npar;
+    const double *u = pr + (A.npar - 3);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) e.pr[q] = LANES == 8 || q < 2 ? pr[q] : 0.0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) e.u[q] = u[q];
+    e.ul = u[min(l, 2)];
+    e.g1 = A.rates[2 * e.n];
+    e.g2 = A.rates[2 * e.n + 1];
+    e.x = A.rho[(long long)e.n * NST + min(l, NST - 1)];
+    e.dipole = A.dipole[3 * e.n + min(l, 2)];
+    e.cell = L.off + A.ci[e.n];
+    return e;
+}
 template <class R, int LANES>
-__device__ __forceinline__ void run1_emit(const R *Ex, const Lay &L, const EmitArgs &A, int t, int nt)
+__device__ __forceinline__ void run1_step(const R *Ex, const EmitArgs &A, int l, Run1Emitter &e)
 {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int NST = LANES == 8 ? 8 : 3;
-    const int l = t % LANES, per = nt / LANES;
-    for (int base = 0; base < A.n; base += per) {
-        const int n0 = base + t / LANES;
-        const bool live = n0 < A.n;
-        const int n = live ? n0 : A.n - 1;
-        const double E = l == 0 ? (double)ld_cg(Ex + (L.off + A.ci[n])) : 0.0;
-        const double *pr = A.par + (long long)n * A.npar;
-        const double *u = pr + (A.npar - 3);
-        const double E0 = __shfl_sync(FULL, E, 0, LANES);
-        const double E_u = u[0] * E0 + u[1] * 0.0 + u[2] * 0.0;
-        const int w = min(l, NST - 1);
-        double *st = A.rho + (long long)n * NST;
-        const EmitLane q = emit_lane<LANES>(w, pr, E_u, A.rates[2 * n], A.rates[2 * n + 1]);
-        const double x = rk4_lane<LANES>(q, w, st[w], A.dt, A.h2, A.h6);
+    const double E = (double)ld_cg(Ex + e.cell);
+    const double E_u = e.u[0] * E + e.u[1] * 0.0 + e.u[2] * 0.0;
+    const int w = min(l, NST - 1), n = e.n;
+    const EmitLane q = emit_lane<LANES>(w, e.pr, E_u, e.g1, e.g2);
+    e.x = rk4_lane<LANES>(q, w, e.x, A.dt, A.h2, A.h6);
+    if (e.live && l < NST) A.rho[(long long)n * NST + l] = e.x;
+    double d;
+    if (LANES == 4) {
+        d = 2.0 * e.pr[1] * __shfl_sync(FULL, e.x, 1, LANES);
+    } else {
+        const double x2 = __shfl_sync(FULL, e.x, 2, LANES), x4 = __shfl_sync(FULL, e.x, 4, LANES);
+        d = 2.0 * e.pr[2] * x2 + 2.0 * e.pr[3] * x4;
+    }
+    const double nw = d * e.ul;
+    if (e.live && l < 3) {
+        A.dipole[3 * n + l] = nw;
+        __stcg(A.dPdt + 3 * n + l, over_dt(nw - e.dipole, A.over));
+        A.E[3 * n + l] = l == 0 ? E : 0.0;
+    }
+    e.dipole = nw;
+}
+// the emitters of one group from `from` on, LANES lanes each
+template <class R, int LANES>
+__device__ __forceinline__ void run1_emit(const R *Ex, const Lay &L, const EmitArgs &A, int t, int nt, int from)
+{
+    const int l = t % LANES;
+    for (int base = from; base < A.n; base += nt / LANES) {
+        Run1Emitter e = run1_load<LANES>(L, A, base + t / LANES, l);
         __syncwarp();                       // every lane has read its word
-        if (live && l < NST) st[l] = x;
-        double d;
-        if (LANES == 4) {
-            d = 2.0 * pr[1] * __shfl_sync(FULL, x, 1, LANES);
-        } else {
-            const double x2 = __shfl_sync(FULL, x, 2, LANES), x4 = __shfl_sync(FULL, x, 4, LANES);
-            d = 2.0 * pr[2] * x2 + 2.0 * pr[3] * x4;
-        }
-        if (live && l < 3) {
-            const double old = A.dipole[3 * n + l];
-            const double nw = d * u[l];
-            A.dipole[3 * n + l] = nw;
-            __stcg(A.dPdt + 3 * n + l, over_dt(nw - old, A.over));
-            A.E[3 * n + l] = l == 0 ? E : 0.0;
-        }
+        run1_step<R, LANES>(Ex, A, l, e);
     }
 }
 
@@ -136,12 +163,28 @@ __global__ void __launch_bounds__(RUN1_THREADS) k_run1(const __grid_constant__ F
         jpt[x] = j;
     }
 
+    // the first group's first emitters stay in registers (read again each step: 7.2 us); warps past them
+    // hold none
+    Run1Emitter mine{};
+    bool held = false;
+    if (side && A.n_grp > 0) {
+        const EmitArgs &G0 = A.grp[0];
+        const int lanes = G0.model == 1 ? 4 : 8;
+        held = st / 32 * 32 / lanes < G0.n;
+        if (held) mine = lanes == 4 ? run1_load<4>(L, G0, st / 4, st % 4) : run1_load<8>(L, G0, st / 8, st % 8);
+    }
+
     // emitters and samples of the step whose table row is given; side threads
     auto side_work = [&](const double *row) {
         if (row[2] != 0.0)
             for (int g = 0; g < A.n_grp; ++g) {
-                if (A.grp[g].model == 1) run1_emit<R, 4>(F.f[0], L, A.grp[g], st, nst);
-                else run1_emit<R, 8>(F.f[0], L, A.grp[g], st, nst);
+                if (A.grp[g].model == 1) {
+                    if (held && g == 0) run1_step<R, 4>(F.f[0], A.grp[0], st % 4, mine);
+                    run1_emit<R, 4>(F.f[0], L, A.grp[g], st, nst, g == 0 ? nst / 4 : 0);
+                } else {
+                    if (held && g == 0) run1_step<R, 8>(F.f[0], A.grp[0], st % 8, mine);
+                    run1_emit<R, 8>(F.f[0], L, A.grp[g], st, nst, g == 0 ? nst / 8 : 0);
+                }
             }
         const int slot = A.has_det ? (int)row[3] : -1;
         if (slot >= 0) {
