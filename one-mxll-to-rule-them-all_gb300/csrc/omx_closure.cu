@@ -127,7 +127,7 @@ bool gemm_bf16(const uint16_t *A, int lda, const uint16_t *B, int ldb, int K, co
     // Few row tiles of a recurrent step: narrower column tiles, down to one 16-column chunk per epilogue
     // warp, while the tiles stay within one per SM.  A step is latency alone: for 256 rows, both
     // directions took 36 us in six launches (input, 128-column GEMM, cell) and take 12 us in two
-    // (gradient of 129 steps 5.7 -> 2.3 ms); a forward pass of 20000 rows, 32 steps 3.4 -> 1.8 ms.
+    // (gradient of 129 steps 5.7 -> 2.2 ms); a forward pass of 20000 rows, 32 steps 3.4 -> 1.8 ms.
     int BN = E.N <= 16 ? 16 : (E.N <= 64 ? 64 : 128);
     if (E.gru_h || E.bwd_dG) {
         const long long mt = (E.M + 127) / 128;
@@ -343,39 +343,66 @@ __global__ void k_cl_gru_bwd(const float *__restrict__ dHm, const float *__restr
     dh_direct[q] = w.dhd;
 }
 
-// BF16 transpose [R x C] -> [C x R] (32 x 32 tiles through shared memory)
+// BF16 transpose [R x C] -> [C x R] (64 x 64 tiles through shared memory, two elements per access; R, C,
+// lds and ldd even, rows 4-byte aligned).  33024 x 256: 12 us (32 x 32 tiles, one element per access: 17)
 __global__ void k_cl_transpose(const uint16_t *__restrict__ src, int R, int C, int lds, uint16_t *__restrict__ dst,
                                int ldd)
 {
-    __shared__ uint16_t tile[32][33];
-    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int r = r0 + k, c = c0 + threadIdx.x;
-        tile[k][threadIdx.x] = (r < R && c < C) ? src[(long long)r * lds + c] : (uint16_t)0;
+    __shared__ __align__(4) uint16_t tile[64][66];
+    const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64, x = 2 * threadIdx.x;
+#pragma unroll
+    for (int k = threadIdx.y; k < 64; k += 8) {
+        const int r = r0 + k, c = c0 + x;
+        *reinterpret_cast<uint32_t *>(&tile[k][x]) =
+            (r < R && c < C) ? *reinterpret_cast<const uint32_t *>(src + (long long)r * lds + c) : 0u;
     }
     __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int c = c0 + k, r = r0 + threadIdx.x;
-        if (c < C && r < R) dst[(long long)c * ldd + r] = tile[threadIdx.x][k];
+#pragma unroll
+    for (int k = threadIdx.y; k < 64; k += 8) {
+        const int c = c0 + k, r = r0 + x;
+        if (c < C && r < R)
+            *reinterpret_cast<uint32_t *>(dst + (long long)c * ldd + r) =
+                (uint32_t)tile[x][k] | ((uint32_t)tile[x + 1][k] << 16);
     }
 }
 
-// out[i] = sum over the row i of a BF16 [rows x n] matrix (one warp per row, fixed order)
-__global__ void k_cl_rowsum(const uint16_t *__restrict__ src, int rows, long long n, long long ld, float *__restrict__ out)
+// out[i] = sum over the row i of a BF16 [rows x n] matrix, rows 16-byte aligned, ld a multiple of 8 and
+// at least n: one block per row stages ROWSUM_CHUNK elements at a time, one warp adds them in a fixed
+// order (lane l the elements l, l + 32, ...).  256 rows of 33024: 16 us (a warp per row straight from
+// memory 59: one load's latency per element of a lane; with 64 in flight 39)
+constexpr int ROWSUM_CHUNK = 8192;
+__global__ void __launch_bounds__(256) k_cl_rowsum(const uint16_t *__restrict__ src, long long n, long long ld,
+                                                   float *__restrict__ out)
 {
-    const int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
-    if (row >= rows) return;
+    __shared__ __align__(16) uint16_t buf[ROWSUM_CHUNK];
+    const uint16_t *row = src + blockIdx.x * ld;
     float s = 0.f;
-    const uint16_t *a = src + row * ld;
-    for (long long k = lane; k < n; k += 32 * 64) {     // 64 loads in flight, added in order
-        uint16_t v[64];
+    for (long long k0 = 0; k0 < n; k0 += ROWSUM_CHUNK) {
+        __syncthreads();
 #pragma unroll
-        for (int q = 0; q < 64; ++q) v[q] = k + 32 * q < n ? a[k + 32 * q] : (uint16_t)0;
+        for (int q = 0; q < ROWSUM_CHUNK / (8 * 256); ++q) {
+            const int at = 8 * (q * 256 + (int)threadIdx.x);
+            if (k0 + at + 8 <= n) {
+                *reinterpret_cast<uint4 *>(buf + at) = *reinterpret_cast<const uint4 *>(row + k0 + at);
+            } else {
+                for (int e = 0; e < 8; ++e) buf[at + e] = k0 + at + e < n ? row[k0 + at + e] : (uint16_t)0;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const int m = (int)min((long long)ROWSUM_CHUNK, (n - k0 + 1023) / 1024 * 1024);
+            for (int k = (int)threadIdx.x; k < m; k += 1024) {
+                float v[32];
 #pragma unroll
-        for (int q = 0; q < 64; ++q) s += __bfloat162float(__ushort_as_bfloat16(v[q]));
+                for (int q = 0; q < 32; ++q) v[q] = __bfloat162float(__ushort_as_bfloat16(buf[k + 32 * q]));
+#pragma unroll
+                for (int q = 0; q < 32; ++q) s += v[q];
+            }
+        }
     }
+    if (threadIdx.x >= 32) return;
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) out[row] = s;
+    if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
 
 // out = sum of `splits` partial [n] arrays (fixed order), optionally masked like Wg
@@ -550,7 +577,7 @@ static bool cl_forward(omx_closure *c, int B, int T, bool keep, std::string &err
 
 // dW [N x K] = sum over rows of dZ[:, n] * X[:, k]: one long-K GEMM over the T*B rows (both
 // operands transposed first), split over K and reduced in a fixed order; the bias gradient, sums of
-// the first nbias columns of dZ, from the same transpose (one warp per column, fixed order)
+// the first nbias columns of dZ, from the same transpose (one block per column, fixed order)
 static bool cl_weight_grad(omx_closure *c, const uint16_t *dZ, int N, const uint16_t *X, int K, long long TB, float *out,
                            float *bias, int nbias, int wg_mask, std::string &err)
 {
@@ -558,8 +585,8 @@ static bool cl_weight_grad(omx_closure *c, const uint16_t *dZ, int N, const uint
     CL_NEED(c->T1, (size_t)N * ldT);
     CL_NEED(c->T2, (size_t)K * ldT);
     const dim3 tb(32, 8);
-    k_cl_transpose<<<dim3((N + 31) / 32, (unsigned)((TB + 31) / 32)), tb, 0, c->stream>>>(dZ, (int)TB, N, N, c->T1.p, ldT);
-    k_cl_transpose<<<dim3((K + 31) / 32, (unsigned)((TB + 31) / 32)), tb, 0, c->stream>>>(X, (int)TB, K, K, c->T2.p, ldT);
+    k_cl_transpose<<<dim3((N + 63) / 64, (unsigned)((TB + 63) / 64)), tb, 0, c->stream>>>(dZ, (int)TB, N, N, c->T1.p, ldT);
+    k_cl_transpose<<<dim3((K + 63) / 64, (unsigned)((TB + 63) / 64)), tb, 0, c->stream>>>(X, (int)TB, K, K, c->T2.p, ldT);
     const int nk = (int)((TB + 63) / 64);
     const int kpz = nk < 32 ? nk : (nk + 31) / 32;      // about 32 splits
     const int splits = (nk + kpz - 1) / kpz;
@@ -572,7 +599,7 @@ static bool cl_weight_grad(omx_closure *c, const uint16_t *dZ, int N, const uint
     if (!gemm_bf16(c->T1.p, ldT, c->T2.p, ldT, (int)TB, E, c->stream, err)) return false;
     k_cl_reduce<<<cl_blocks((long long)N * K), 256, 0, c->stream>>>(c->part.p, splits, (long long)N * K, out, wg_mask,
                                                                    K);
-    k_cl_rowsum<<<(nbias + 7) / 8, 256, 0, c->stream>>>(c->T1.p, nbias, TB, ldT, bias);
+    k_cl_rowsum<<<nbias, 256, 0, c->stream>>>(c->T1.p, TB, ldT, bias);
     CL_CK(cudaGetLastError());
     return true;
 }
