@@ -298,16 +298,18 @@ struct omx_ctx {
     DevBuf<float> ff2[6];
     DevBuf<float> psiH2[3][2];
     int cur = 0;
-    bool fused_ok = false;
+    bool fused_any = false;     // the fused pass can step this grid, whatever its own step form (fused_possible)
+    bool fused_ok = false;      // and the step form takes it
     bool fused_dirty = true;    // media or sources changed since the last eligibility check
     bool post_ok = false;       // the work after the fused pass goes in one launch (post_eligible)
     bool plane_fold = false;    // the 3D bulk E pass adds the plane source (plane_fold_eligible)
     bool fold3 = false;         // the fused 3D pass adds the single plane source (fold3_of)
     // the fused 3D step runs in place (k_f3p_h / k_f3p_e) instead of through the staged pass: the rule's
-    // choice (prepare), or pinned by a launch shape (0: the rule, 1: in place, 2: staged; a batch needs
-    // the staged pass's buffers)
+    // choice (prepare), or pinned by a launch shape (0: the rule, 1: in place, 2: staged).  A batch steps
+    // its members in a form of its own and leaves these alone.
     bool f3_inplace = false;
     int f3_pin = 0;
+    int f3_step = 0;            // form of the last 3D step, by itself or in a batch (0: none yet, 1: in place, 2: staged)
     bool taps_h = false;        // some detector samples an H component
     bool side_wait = false;     // graph capture: the in-place step waits for ev_join where it must
     F3tMaps f3maps[2][2];       // tensor maps of the fused 3D pass: [in set][tile rows 8 / 16]
@@ -959,9 +961,9 @@ bool fold3_of(const omx_ctx *c)
     return c->dims == 3 && c->sources.size() == 1 && c->sources[0]->kind == 1;
 }
 
-bool fused_eligible(const omx_ctx *c)
+bool fused_possible(const omx_ctx *c)
 {
-    if (!c->fp32 || c->step_form == OMX_STEP_TWO_PASS) return false;
+    if (!c->fp32) return false;
     if (c->dims == 2) {
         if (c->desc.mode != OMX_TMZ_2D_MODE || c->n[0] % 4 != 0) return false;
         const int npml = c->desc.npml;
@@ -994,6 +996,8 @@ bool fused_eligible(const omx_ctx *c)
     }
     return true;
 }
+
+bool fused_eligible(const omx_ctx *c) { return c->step_form != OMX_STEP_TWO_PASS && fused_possible(c); }
 
 // The dispersive cells, the sources and the emitter current after a fused pass can share one
 // launch when they write disjoint E words: at most one source, a plane (the plane holds no
@@ -1029,16 +1033,22 @@ bool plane_fold_eligible(const omx_ctx *c)
 
 void f3t_plan(omx_ctx *c);
 
-// the other buffer set of a pass that reads one set and writes the other
+// the other buffer set of a pass that reads one set and writes the other; a call that follows one that
+// ran out of memory allocates what is still missing
 void second_set(omx_ctx *c)
 {
-    if (c->ff2[2].p) return;
+    bool made = false;
+    auto need = [&](DevBuf<float> &b, size_t n) {
+        if (b.p) return;
+        b.alloc(n);
+        made = true;
+    };
     for (int q = 0; q < 6; ++q)
-        if (c->field_used[q]) c->ff2[q].alloc(c->felems);
+        if (c->field_used[q]) need(c->ff2[q], c->felems);
     for (int a = 0; a < 3; ++a)
         for (int q = 0; q < 2; ++q)
-            if (c->psif[a][1][q].p) c->psiH2[a][q].alloc(c->psif[a][1][q].n);
-    c->epoch++;
+            if (c->psif[a][1][q].p) need(c->psiH2[a][q], c->psif[a][1][q].n);
+    if (made) c->epoch++;
 }
 
 // In place or staged, for a grid that the fused 3D pass can step: in place up to F3_INPLACE_MOST
@@ -1063,8 +1073,10 @@ void prepare(omx_ctx *c)
     if (c->det_dirty) rebuild_detectors(c);
     c->started = true;
     if (c->fused_dirty) {
-        c->fused_ok = fused_eligible(c);
+        c->fused_any = fused_possible(c);
+        c->fused_ok = c->fused_any && c->step_form != OMX_STEP_TWO_PASS;
         c->f3_inplace = c->fused_ok && f3_inplace_rule(c);
+        c->f3_step = 0;
         c->fused_dirty = false;
     }
     c->taps_h = false;
@@ -1072,7 +1084,7 @@ void prepare(omx_ctx *c)
     if (recheck) {
         c->post_ok = post_eligible(c);
         c->plane_fold = plane_fold_eligible(c);
-        c->fold3 = c->fused_ok && fold3_of(c);
+        c->fold3 = c->fused_any && fold3_of(c);
     }
     if (c->fused_ok && c->fp32 && c->dims == 3 && !c->f3_inplace) f3t_plan(c);
     if (c->fused_ok && !c->f3_inplace) second_set(c);
@@ -1385,41 +1397,53 @@ void f3t_plan(omx_ctx *c)
 // plane source when fold3 holds (`plane`: its amplitude).  The caller adds the other sources and
 // the emitter current to the new set.
 void join_side_kernels(omx_ctx *c);
+
+// One FP32 3D step in place (k_f3p_h / k_f3p_e), march planes per thread (0: the default by size).
+template <class R> void inplace_step(omx_ctx *c, int march, const StepParam *plane);
+template <> void inplace_step<double>(omx_ctx *, int, const StepParam *) {}
+template <> void inplace_step<float>(omx_ctx *c, int march, const StepParam *plane)
+{
+    ProfScope ps(c, KC_E);
+    GridArgs<float> G = grid_args<float>(c);
+    // H overwrites what the previous step's side work may sample, E what its emitters gather
+    auto wait_side = [&]() {
+        if (c->side_wait) ck(cudaStreamWaitEvent(c->stream, c->ev_join, 0), "wait");
+        else join_side_kernels(c);
+    };
+    Fused3Args A;
+    A.in = A.out = field_ptrs<float>(c);
+    for (int a = 0; a < 3; ++a)
+        for (int q = 0; q < 2; ++q) A.psiH_out[a][q] = G.psiH[a][q];
+    if (c->taps_h) wait_side();
+    ck(launch_fused3p(A, G, march, false, c->stream), "3D launch");
+    if (!c->taps_h) wait_side();
+    G.step_inc = nullptr;
+    if (c->fold3 && plane) {
+        const SourceRec &S = *c->sources[0];
+        G.pl_on = 1;
+        G.pl_comp = S.pd.comp - 1;
+        G.pl_axis = S.pd.plane_axis - 1;
+        G.pl_index = S.pd.plane_index;
+        G.pl_c_src = S.c_src;
+        G.pl_amp = *plane;
+    }
+    ck(launch_fused3p(A, G, march, true, c->stream), "3D launch");
+    c->launches += 2;
+    c->f3_step = 1;
+}
+
 template <class R> void fused_step(omx_ctx *c, bool ade = true, const StepParam *plane = nullptr);
 template <> void fused_step<double>(omx_ctx *, bool, const StepParam *) {}
 template <> void fused_step<float>(omx_ctx *c, bool ade, const StepParam *plane)
 {
+    if (c->dims == 3 && c->f3_inplace) {
+        inplace_step<float>(c, c->march, plane);
+        return;
+    }
     ProfScope ps(c, KC_E);
     const int in = c->cur, out = 1 - c->cur;
     const FieldPtrs<float> Fin = field_ptrs<float>(c, in), Fout = field_ptrs<float>(c, out);
     GridArgs<float> G = grid_args<float>(c);
-    if (c->dims == 3 && c->f3_inplace) {
-        // H overwrites what the previous step's side work may sample, E what its emitters gather
-        auto wait_side = [&]() {
-            if (c->side_wait) ck(cudaStreamWaitEvent(c->stream, c->ev_join, 0), "wait");
-            else join_side_kernels(c);
-        };
-        Fused3Args A;
-        A.in = A.out = Fin;
-        for (int a = 0; a < 3; ++a)
-            for (int q = 0; q < 2; ++q) A.psiH_out[a][q] = G.psiH[a][q];
-        if (c->taps_h) wait_side();
-        ck(launch_fused3p(A, G, c->march, false, c->stream), "3D launch");
-        if (!c->taps_h) wait_side();
-        G.step_inc = nullptr;
-        if (c->fold3 && plane) {
-            const SourceRec &S = *c->sources[0];
-            G.pl_on = 1;
-            G.pl_comp = S.pd.comp - 1;
-            G.pl_axis = S.pd.plane_axis - 1;
-            G.pl_index = S.pd.plane_index;
-            G.pl_c_src = S.c_src;
-            G.pl_amp = *plane;
-        }
-        ck(launch_fused3p(A, G, c->march, true, c->stream), "3D launch");
-        c->launches += 2;
-        return;
-    }
     if (c->dims == 3) {
         Fused3Args A;
         A.in = Fin;
@@ -1471,6 +1495,7 @@ template <> void fused_step<float>(omx_ctx *c, bool ade, const StepParam *plane)
         }
         c->launches += (ng > 0 ? 2 : 0) + (nl > 0 ? 1 : 0);
         c->cur = out;
+        c->f3_step = 2;
         return;
     }
     Fused2Args A;
@@ -2040,6 +2065,7 @@ void apply_shape(omx_ctx *c, int v)
         c->march = v;
     }
     c->f3_inplace = fused && f3_inplace_rule(c);
+    c->f3_step = 0;
 }
 
 constexpr int AUTOTUNE_STEPS = 4;   // steps timed back to back per candidate and round
@@ -3450,9 +3476,10 @@ struct omx_batch {
     // H on `aux` beside their lean runs, then their E), the others in one k_fused3_batch launch
     // (on `aux` after that H)
     int f3nsplit = 0;
-    // small grids (batch_inplace_rule): each member steps in place by itself, its launches on one of
-    // the lanes, so that the grids fill the GPU together
-    bool f3inplace = false;
+    // small grids (batch_inplace_rule) step in place, each member's launches on one of the lanes, so that
+    // the grids fill the GPU together; staged: a launch shape was set, or the tuner found the staged
+    // pass faster
+    bool staged = false;
     static constexpr int LANES = 12;
     cudaStream_t lane[LANES] = {};
     cudaEvent_t ev_lane[LANES] = {};
@@ -3483,6 +3510,20 @@ namespace {
 
 constexpr int BATCH_DEFAULT_KCH = 16;
 
+// building tables and capturing steps leave the members' buffer sets as they are
+struct KeepCur {
+    omx_batch *b;
+    std::vector<int> cur0;
+    explicit KeepCur(omx_batch *bb) : b(bb)
+    {
+        for (auto *c : b->ctx) cur0.push_back(c->cur);
+    }
+    ~KeepCur()
+    {
+        for (size_t i = 0; i < cur0.size(); ++i) b->ctx[i]->cur = cur0[i];
+    }
+};
+
 template <class T> size_t pad16(size_t n) { return (n * sizeof(T) + 15) / 16 * 16; }
 
 // Tables of one batched step.  Two-pass path: q = 0.  Fused path: the step of parity q, whose
@@ -3493,16 +3534,8 @@ BatchTables<R> batch_tables(omx_batch *b, const std::vector<RunPlan> *plans, int
 {
     const int n = (int)b->ctx.size();
     const bool f3 = b->fused == 1;
-    std::vector<int> cur0;
-    for (auto *c : b->ctx) cur0.push_back(c->cur);
-    struct RestoreCur {
-        omx_batch *b;
-        const std::vector<int> &cur0;
-        ~RestoreCur()
-        {
-            for (size_t i = 0; i < b->ctx.size(); ++i) b->ctx[i]->cur = cur0[i];
-        }
-    } restore{b, cur0};
+    const KeepCur keep(b);
+    const std::vector<int> &cur0 = keep.cur0;
     if (f3)
         for (int i = 0; i < n; ++i) b->ctx[i]->cur = cur0[i] ^ q ^ 1;
     BatchTables<R> T;
@@ -3776,7 +3809,9 @@ void batch_lanes(omx_batch *b)
 
 // `steps` steps of every member in place: member i's own launches (H, E, sources, emitter work,
 // detectors, as its omx_run issues them) on lane i mod LANES, forked from the batch's stream and
-// joined to it at the end; no member waits for another.  plans null: the field passes alone.
+// joined to it at the end; no member waits for another.  plans null: the field passes alone.  The
+// form is the batch's: a member's own step form and launch shape do not count, and no buffer set is
+// switched.
 template <class R> long long batch_inplace_steps(omx_batch *b, const std::vector<RunPlan> *plans, int steps)
 {
     // four lanes when the members are large (fewer buffer sets share L2), else every lane.  us per
@@ -3789,25 +3824,38 @@ template <class R> long long batch_inplace_steps(omx_batch *b, const std::vector
     long long k = 0;
     ck(cudaEventRecord(b->ev_fork, b->stream), "event");
     for (int l = 0; l < lanes; ++l) ck(cudaStreamWaitEvent(b->lane[l], b->ev_fork, 0), "event");
-    struct Route {
+    struct Route {   // joins the lanes when a launch fails, too
         omx_batch *b;
+        int lanes;
+        bool joined = false;
+        void join()
+        {
+            joined = true;
+            for (int l = 0; l < lanes; ++l) {
+                ck(cudaEventRecord(b->ev_lane[l], b->lane[l]), "event");
+                ck(cudaStreamWaitEvent(b->stream, b->ev_lane[l], 0), "event");
+            }
+        }
         ~Route()
         {
             for (auto *c : b->ctx) c->stream = b->stream;
+            for (int l = 0; l < lanes && !joined; ++l)
+                if (cudaEventRecord(b->ev_lane[l], b->lane[l]) == cudaSuccess)
+                    cudaStreamWaitEvent(b->stream, b->ev_lane[l], 0);
         }
-    } route{b};
+    } route{b, lanes};
     for (int i = 0; i < n; ++i) b->ctx[i]->stream = b->lane[i % lanes];
     for (int s = 0; s < steps; ++s)
         for (int i = 0; i < n; ++i) {
             omx_ctx *c = b->ctx[i];
             const long long before = c->launches;
             if (!plans) {
-                fused_step<R>(c);
+                inplace_step<R>(c, 0, nullptr);
             } else {
                 const RunPlan &P = (*plans)[i];
                 std::vector<StepParam> amps;
                 for (size_t q = 0; q < c->sources.size(); ++q) amps.push_back(plan_param(c, P, 4 + (int)q));
-                fused_step<R>(c, true, c->fold3 ? &amps[0] : nullptr);
+                inplace_step<R>(c, 0, c->fold3 ? &amps[0] : nullptr);
                 if (!c->fold3) do_sources<R>(c, amps);
                 do_inject<R>(c, plan_param(c, P, 0), plan_param(c, P, 1));
                 for (auto &g : c->groups) do_group<R>(c, *g, plan_param(c, P, 2));
@@ -3815,10 +3863,7 @@ template <class R> long long batch_inplace_steps(omx_batch *b, const std::vector
             }
             k += c->launches - before;
         }
-    for (int l = 0; l < lanes; ++l) {
-        ck(cudaEventRecord(b->ev_lane[l], b->lane[l]), "event");
-        ck(cudaStreamWaitEvent(b->stream, b->ev_lane[l], 0), "event");
-    }
+    route.join();
     return k;
 }
 
@@ -3907,12 +3952,80 @@ template <class R> long long batch_step(omx_batch *b, const BatchTables<R> &T, c
     return k;
 }
 
+// In place or staged for a batch of grids that the fused pass can step: in place when every member
+// would step so by itself.  Measured, us per step, staged in the best of four shapes / in place: twelve
+// grids of 8.4 M cells in all 310 / 261, twelve of 1.3 M 85 / 48, three of 2.6 M 127 / 65, four of
+// 17.7 M 446 / 410, 32 of 31.7 M 906 / 906.
+bool batch_inplace_rule(const omx_batch *b)
+{
+    for (const auto *c : b->ctx) {
+        if (c->step_form != OMX_STEP_DEFAULT || (long long)c->n[0] * c->n[1] * c->n[2] > F3_INPLACE_MOST) return false;
+        for (const auto &g : c->groups)
+            if (g->cl) return false;         // members may share a closure, whose steps run one after the other
+    }
+    return true;
+}
+
+void batch_two_pass(omx_batch *b)
+{
+    b->fused = 0;
+    for (auto *c : b->ctx) {
+        c->step_form = OMX_STEP_TWO_PASS;
+        c->fused_dirty = true;
+        c->fused_ok = false;
+        c->epoch++;
+    }
+}
+
+// Prepare every member, and choose the form of the batch's next steps from the members as they are now
+// (their step forms, shapes, sources and buffer sets may have changed since the last run, by hand or
+// in another batch).  True: in place.  A member that the fused pass can no longer step takes the
+// batch to the two half-step passes for good; the staged pass has every member's second buffer set.
+bool batch_settle(omx_batch *b)
+{
+    for (auto *c : b->ctx) prepare(c);
+    if (b->fused != 1) return false;
+    bool any = true;
+    for (const auto *c : b->ctx) any = any && c->fused_any;
+    if (!any) {
+        batch_two_pass(b);
+        for (auto *c : b->ctx) prepare(c);
+        return false;
+    }
+    if (!b->staged && batch_inplace_rule(b)) return true;
+    for (auto *c : b->ctx) second_set(c);
+    return false;
+}
+
+// a capture on a stream, ended (and its graph dropped) when an error leaves it
+struct Capture {
+    cudaStream_t s;
+    bool open = true;
+    explicit Capture(cudaStream_t st) : s(st)
+    {
+        ck(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "capture");
+    }
+    ~Capture()
+    {
+        cudaGraph_t g = nullptr;
+        if (open && cudaStreamEndCapture(s, &g) == cudaSuccess && g) cudaGraphDestroy(g);
+    }
+    cudaGraph_t end()
+    {
+        cudaGraph_t g = nullptr;
+        open = false;
+        ck(cudaStreamEndCapture(s, &g), "end capture");
+        return g;
+    }
+};
+
 // prepare_only: build the tables and capture the step graphs that the same call without it
 // launches, and run nothing (the members' stepping state and records are unchanged).
 template <class R> void batch_run_impl(omx_batch *b, int tt0, int nsteps, int n_skip, int t_det_print, int use_graph,
                                        bool prepare_only = false)
 {
     BatchStreams streams(b);
+    const bool ip = batch_settle(b);
     std::vector<RunPlan> plans;
     for (auto *c : b->ctx) {
         const double t_skip0 = c->t_skip;
@@ -3928,9 +4041,9 @@ template <class R> void batch_run_impl(omx_batch *b, int tt0, int nsteps, int n_
     const int kch = b->kch > 0 ? b->kch : BATCH_DEFAULT_KCH;
     if (b->blocks == 0) b->blocks = batch3_blocks<R>();
     // the fused path alternates the members' buffer sets: step s of this call uses T[s & 1]
-    const bool ip = b->fused == 1 && b->f3inplace, f3 = b->fused == 1 && !ip;
+    const bool f3 = b->fused == 1 && !ip;
     if (ip) batch_lanes(b);
-    std::vector<long long> key = {b->fused, kch, b->f3form, b->f3kch, b->f3nsplit, b->blocks, b->f3inplace};
+    std::vector<long long> key = {b->fused, kch, b->f3form, b->f3kch, b->f3nsplit, b->blocks, ip};
     for (size_t i = 0; i < b->ctx.size(); ++i) {
         const omx_ctx *c = b->ctx[i];
         key.insert(key.end(), {(long long)c->epoch, c->cur, (long long)(uintptr_t)c->tab.p, plans[i].W,
@@ -3955,15 +4068,12 @@ template <class R> void batch_run_impl(omx_batch *b, int tt0, int nsteps, int n_
             for (auto &g : b->graphs)
                 if (g.steps == steps) hit = &g;
             if (!hit) {
-                std::vector<int> cur0;
-                for (auto *c : b->ctx) cur0.push_back(c->cur);
-                cudaGraph_t graph;
-                ck(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "capture");
+                KeepCur keep(b);
+                Capture capture(b->stream);
                 long long per = 0;
                 if (ip) per = batch_inplace_steps<R>(b, &plans, steps);
                 for (int q = 0; !ip && q < steps; ++q) per += batch_step<R>(b, T[f3 ? (q & 1) : 0], plans, kch);
-                ck(cudaStreamEndCapture(b->stream, &graph), "end capture");
-                for (size_t i = 0; i < b->ctx.size(); ++i) b->ctx[i]->cur = cur0[i];
+                cudaGraph_t graph = capture.end();
                 cudaGraphExec_t exec = nullptr;
                 const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
                 cudaGraphDestroy(graph);
@@ -3987,31 +4097,10 @@ template <class R> void batch_run_impl(omx_batch *b, int tt0, int nsteps, int n_
     }
     ck(cudaPeekAtLastError(), "launch");
     if (!prepare_only)
-        for (size_t i = 0; i < b->ctx.size(); ++i) b->ctx[i]->rec_count += plans[i].nrec;
-}
-
-// In place or staged for a batch of grids that the fused pass can step: in place when every member
-// would step so by itself.  Measured, us per step, staged in the best of four shapes / in place: twelve
-// grids of 8.4 M cells in all 310 / 261, twelve of 1.3 M 85 / 48, three of 2.6 M 127 / 65, four of
-// 17.7 M 446 / 410, 32 of 31.7 M 906 / 906.
-bool batch_inplace_rule(const omx_batch *b)
-{
-    for (const auto *c : b->ctx) {
-        if (c->step_form != OMX_STEP_DEFAULT || (long long)c->n[0] * c->n[1] * c->n[2] > F3_INPLACE_MOST) return false;
-        for (const auto &g : c->groups)
-            if (g->cl) return false;         // members may share a closure, whose steps run one after the other
-    }
-    return true;
-}
-void batch_set_inplace(omx_batch *b, bool on)
-{
-    b->f3inplace = on;
-    for (auto *c : b->ctx) {
-        c->f3_pin = on ? 1 : 2;       // staged: the batched pass reads one buffer set and writes the other
-        c->march = 0;
-        c->fused_dirty = true;
-        c->epoch++;
-    }
+        for (size_t i = 0; i < b->ctx.size(); ++i) {
+            b->ctx[i]->rec_count += plans[i].nrec;
+            if (b->fused == 1) b->ctx[i]->f3_step = ip ? 1 : 2;
+        }
 }
 
 // Tile depth of the batched passes, timed on the zero initial fields (which every pass maps to
@@ -4032,7 +4121,7 @@ template <class R> int batch_autotune_impl(omx_batch *b, int reps)
         float best = 0.f, inplace = 0.f;
         int pick = 8064;
         bool first = true;
-        const bool may = b->f3inplace;       // the in-place pass is timed beside the staged shapes
+        const bool may = batch_inplace_rule(b);   // the in-place pass is timed beside the staged shapes
         if (may) {
             batch_lanes(b);
             batch_inplace_steps<R>(b, nullptr, 1);
@@ -4041,9 +4130,8 @@ template <class R> int batch_autotune_impl(omx_batch *b, int reps)
             ck(cudaEventRecord(e1, b->stream), "event");
             ck(cudaEventSynchronize(e1), "batch autotune");
             ck(cudaEventElapsedTime(&inplace, e0, e1), "batch autotune");
-            b->f3inplace = false;
-            for (auto *c : b->ctx) second_set(c);
         }
+        for (auto *c : b->ctx) second_set(c);
         int dev = 0, optin = 0;
         ck(cudaGetDevice(&dev), "device");
         ck(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "device");
@@ -4078,7 +4166,7 @@ template <class R> int batch_autotune_impl(omx_batch *b, int reps)
         b->f3nsplit = pick / 1000000;
         b->f3form = pick / 1000 % 1000;
         b->f3kch = pick % 1000;
-        if (may) batch_set_inplace(b, inplace <= best);
+        b->staged = !may || inplace > best;
         return pick;
     }
     cudaEvent_t e0, e1;
@@ -4119,23 +4207,15 @@ template <class R> int batch_autotune_impl(omx_batch *b, int reps)
 }
 
 // The batch's arithmetic, fixed at its first autotune or run: when every member steps with one
-// fused FP32 pass, the batched fused pass (one launch, or split by plane form for the largest
-// grids); otherwise the two half-step passes (k_batch3), which every member then keeps when used
-// on its own.
+// fused FP32 pass, that pass, in place or batched (batch_settle); otherwise the two half-step passes
+// (k_batch3), which every member then keeps when used on its own.
 void batch_decide(omx_batch *b)
 {
     if (b->fused >= 0) return;
     bool all = b->fp32;
     for (auto *c : b->ctx) all = all && fused_eligible(c);
-    b->fused = all ? 1 : 0;
-    if (all) batch_set_inplace(b, batch_inplace_rule(b));
-    if (!all)
-        for (auto *c : b->ctx) {
-            c->step_form = OMX_STEP_TWO_PASS;
-            c->fused_dirty = true;
-            c->fused_ok = false;
-            c->epoch++;
-        }
+    if (all) b->fused = 1;
+    else batch_two_pass(b);
 }
 
 }  // namespace
@@ -4178,10 +4258,8 @@ int omx_batch_autotune(omx_batch *b, int reps, int *choice)
         req(!c->started && !c->fields_written,
             "omx_batch_autotune times the passes on the initial zero fields: call it after the grids are "
             "configured and before their first step or field write", OMX_ERR_STATE);
-    for (auto *c : b->ctx) {
-        prepare(c);
-        c->epoch++;
-    }
+    batch_settle(b);
+    for (auto *c : b->ctx) c->epoch++;
     b->drop_graphs();
     b->key.clear();
     const int pick = b->fp32 ? batch_autotune_impl<float>(b, reps) : batch_autotune_impl<double>(b, reps);
@@ -4207,7 +4285,7 @@ int omx_batch_set_launch_shape(omx_batch *b, int shape)
         b->f3nsplit = shape / 1000000;
         b->f3form = form;
         b->f3kch = kch;
-        if (b->f3inplace) batch_set_inplace(b, false);
+        b->staged = true;
     } else {
         req(shape == 4 || shape == 8 || shape == 16 || shape == 32, "batched two-pass shape: tile depth 4, 8, 16 or 32");
         b->kch = shape;
@@ -4363,7 +4441,7 @@ int omx_algorithmic_bytes(const omx_ctx *c, int kc, double *bytes)
         ade_bytes = (double)drude * 2.0 * w + (double)dl * (2.0 + 2.0 + 4.0 * c->P) * w;
     }
     const bool fused = c->fused_ok;   // FP32 fused (2D TMz, 3D): one pass per step (class KC_E)
-    if (fused && c->f3_inplace) {     // both half-step passes counted as one launch of class KC_E
+    if (fused && (c->f3_step ? c->f3_step == 1 : c->f3_inplace)) {     // both half-step passes counted as one launch of class KC_E
         b = kc != KC_E ? 0.0 : cells * w * 3.0 * (ncomp_e + ncomp_h) + (psi_cells_h + psi_cells_e) * 2.0 * w +
                                    (double)c->bbV * ncomp_e + ade_bytes;
     } else if (kc == KC_H) {

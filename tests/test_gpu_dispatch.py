@@ -466,3 +466,96 @@ def test_prepared_run_equals_run(dims, n, precision, shape):
     assert np.max(np.abs(out[0][1])) > 0
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+# what happens to member 0 between two odd-length runs of the batch: a staged shape or the two-pass form of
+# its own, runs in a second (staged) batch, a source on dispersive cells (two half-step passes from
+# then on, for every member)
+@pytest.mark.parametrize("use_graph", [True, False])
+@pytest.mark.parametrize("change", ["shape", "two_pass", "single_pass", "second", "source"])
+def test_inplace_batch_after_its_members_change(change, use_graph):
+    """A batch steps in its own form whatever happens to its members between runs: every member
+    equals its solo run bit for bit, and a member's own form is its own afterwards."""
+    from test_gpu_parity import fused3_deck
+    from omx import decks
+
+    specs = [((33, 30, 27), (3, 3, 3)), ((40, 36, 28), (3, 3, 2)), ((29, 41, 26), (1, 3, 3))]
+
+    def build(spec):
+        d = fused3_deck(*spec, src="both")
+        g = omx.TMxll(3, d["grid_Ndims"], d["npml"], d["boundaries"], d["dt"], d["dr"], precision="fp32")
+        gr = decks.apply_deck(g, d, omx, decks.media_map(d, omx.media_map_from_voxels))
+        for det in d["detectors"]:
+            g.add_detector(det["type"], det["field"], det["idx"])
+        return g, gr
+
+    def state(g, gr):
+        return [g.drain_detectors()[1]] + [g.read_field(f) for f in range(1, 7)] + [q.read()["rho"] for q in gr]
+
+    def add_source(g):
+        fs = omx.UNITS["fs_to_au"]
+        g.add_plane_source(1, 3, 27 // 2, 1.0, 0.08, 1.0 * fs, 1.0 * fs, 0.0, 1e30)
+
+    want = []
+    for q, sp in enumerate(specs):
+        g, gr = build(sp)
+        g.run(1, 13, 1, 1)
+        if change == "source":
+            add_source(g) if q == 0 else g.set_step_form(omx.STEP_TWO_PASS)
+        if change == "second" and q == 0:
+            g.run(14, 5, 1, 1)
+        g.run(19, 7, 1, 1)
+        want.append(state(g, gr))
+        g.kill()
+    grids = [build(sp) for sp in specs]
+    b = omx.Batch([g for g, _ in grids])
+    b.run(1, 13, 1, 1, use_graph=use_graph)
+    m = grids[0][0]
+    if change == "shape":
+        m.set_launch_shape(8064)
+    elif change == "two_pass":
+        m.set_step_form(omx.STEP_TWO_PASS)
+    elif change == "single_pass":
+        m.set_step_form(omx.STEP_SINGLE_PASS)
+    elif change == "source":
+        add_source(m)
+    else:
+        b2 = omx.Batch([m])
+        b2.set_launch_shape(8016)
+        b2.run(14, 5, 1, 1, use_graph=use_graph)
+        b2.synchronize()
+        b2.kill()
+    b.run(19, 7, 1, 1, use_graph=use_graph)
+    b.synchronize()
+    for (g, gr), w in zip(grids, want):
+        got = state(g, gr)
+        assert np.max(np.abs(w[0])) > 0
+        for x, y in zip(got, w):
+            assert np.array_equal(x, y)
+    b.kill()
+    for g, _ in grids:
+        g.kill()
+
+
+@pytest.mark.parametrize("staged", [False, True])
+def test_batch_leaves_its_members_own_shape(staged):
+    """A member that ran in a batch launches what a grid that did not launches afterwards."""
+    def launches(batch):
+        dt = omx.units.yee_dt(37.8)
+        g = omx.TMxll(3, (30, 26, 28), 4, (3,) * 3, dt, 37.8, precision="fp32")
+        if batch:
+            b = omx.Batch([g])
+            if staged:
+                b.set_launch_shape(8016)
+            b.run(1, 4)
+            b.synchronize()
+            b.kill()
+        else:
+            g.run(1, 4)
+        n = g.launch_count()
+        g.run(5, 6, use_graph=False)
+        n = g.launch_count() - n, g.algorithmic_bytes(omx.KC_E)
+        g.kill()
+        return n
+
+    assert launches(True) == launches(False)
