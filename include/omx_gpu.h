@@ -301,9 +301,10 @@ int omx_run_prepare(omx_ctx *ctx, int tt0, int nsteps, int n_skip_steps, int t_d
  *                         periodic: the planes staged by TMA, the dispersive cells and a single
  *                         plane source inside the pass; 3D grids of up to 18 M cells take the same
  *                         arithmetic in two passes in place), else the two half-step passes
- *   OMX_STEP_TWO_PASS     the two half-step passes everywhere: the arithmetic of batched runs
- *                         (omx_batch_create sets it on its members)
- *   OMX_STEP_SINGLE_PASS  the same results as OMX_STEP_DEFAULT, 3D always in the staged pass */
+ *   OMX_STEP_TWO_PASS     the two half-step passes everywhere: the arithmetic of batches with a
+ *                         member that the fused pass cannot step (such a batch sets it on its members)
+ *   OMX_STEP_SINGLE_PASS  the same results as OMX_STEP_DEFAULT, 3D always in the staged pass, whatever
+ *                         shape or batch selected the passes in place before */
 #define OMX_STEP_DEFAULT 0
 #define OMX_STEP_TWO_PASS 1
 #define OMX_STEP_SINGLE_PASS 2
@@ -327,7 +328,7 @@ int omx_autotune(omx_ctx *ctx, int reps, int *choice);
 /* Sets the launch shape directly (a value omx_autotune reported, e.g. for a grid of the same shape
  * tuned earlier); no counterpart in the reference.  Every shape of one step form gives the same
  * results bit for bit; on a 3D FP32 grid that the fused pass can step a shape below 1000 selects
- * the two passes in place. */
+ * the two passes in place (for OMX_STEP_DEFAULT). */
 int omx_set_launch_shape(omx_ctx *ctx, int shape);
 
 /* ---- batched multi-grid runs (no counterpart in the reference: it runs one grid per process) -

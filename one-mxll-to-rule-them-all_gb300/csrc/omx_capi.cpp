@@ -1059,9 +1059,8 @@ void second_set(omx_ctx *c)
 constexpr long long F3_INPLACE_MOST = 18000000;
 bool f3_inplace_rule(const omx_ctx *c)
 {
-    if (c->dims != 3) return false;
+    if (c->dims != 3 || c->step_form != OMX_STEP_DEFAULT) return false;
     if (c->f3_pin) return c->f3_pin == 1;
-    if (c->step_form != OMX_STEP_DEFAULT) return false;
     return (long long)c->n[0] * c->n[1] * c->n[2] <= F3_INPLACE_MOST;
 }
 
@@ -1368,7 +1367,8 @@ void f3t_runs(const omx_ctx *c, int ty, int kch, std::vector<int4> &gen, std::ve
 void f3t_plan(omx_ctx *c)
 {
     const int ty = f3t_rows(c->fused_form);
-    const int kch = c->march > 0 ? std::min(c->march, F3T_KMAX) : 64;
+    // (a march chosen for the pass in place is no number of planes per block)
+    const int kch = c->march > 0 && c->f3_pin != 1 ? std::min(c->march, F3T_KMAX) : 64;
     const bool pl = c->fold3 && !c->sources.empty();
     const long long key = ((long long)ty * 1000 + kch) * 2 + (pl ? 1 : 0);
     auto hit = c->f3plans.find(key);

@@ -559,3 +559,30 @@ def test_batch_leaves_its_members_own_shape(staged):
         return n
 
     assert launches(True) == launches(False)
+
+
+@pytest.mark.parametrize("before", ["nothing", "shape", "autotune", "batch"])
+def test_single_pass_form_is_the_staged_pass(before):
+    """OMX_STEP_SINGLE_PASS steps 3D grids in the staged pass also after the passes in place were
+    selected by a shape, by the tuner or by a batch; the default form returns to them."""
+    dt = omx.units.yee_dt(37.8)
+    g = omx.TMxll(3, (30, 26, 28), 4, (3,) * 3, dt, 37.8, precision="fp32")
+    if before == "shape":
+        g.set_launch_shape(4)
+    elif before == "autotune":
+        g.autotune(reps=1)
+        g.set_launch_shape(2)                # whatever the tuner's pick
+    elif before == "batch":
+        b = omx.Batch([g])
+        b.run(1, 2)
+        b.synchronize()
+        b.kill()
+    words = {}
+    for form in (omx.STEP_DEFAULT, omx.STEP_SINGLE_PASS, omx.STEP_DEFAULT):
+        g.set_step_form(form)
+        g.run(3, 3)
+        words.setdefault(form, set()).add(g.algorithmic_bytes(omx.KC_E))
+    g.kill()
+    # 18 words a cell and step in place, 12 staged, beside the same CPML words
+    (inplace,), (staged,) = words[omx.STEP_DEFAULT], words[omx.STEP_SINGLE_PASS]
+    assert inplace - staged == 6 * 4 * 30 * 26 * 28
