@@ -1056,10 +1056,12 @@ void second_set(omx_ctx *c)
 // (default shapes): 32^3 7.9 / 25.4, 64^3 10.7 / 27.4, 96^3 20.5 / 62.8, 128^3 37.9 / 99.4, 160^3
 // 89 / 139, 192^3 140 / 173, 224^3 208 / 233, 256^3 293 / 318, 288^3 403 / 419, 320^3 537 / 529, 384^3
 // 879 / 820; with 1e5 emitters, which overlap the in-place step's H pass only, 320 x 288 x 250 482 / 438.
+// Its launches hold the rows of at most 65535 blocks of four; the staged pass takes any number.
 constexpr long long F3_INPLACE_MOST = 18000000;
+bool f3_inplace_fits(const omx_ctx *c) { return c->n[1] <= 4 * 65535; }
 bool f3_inplace_rule(const omx_ctx *c)
 {
-    if (c->dims != 3 || c->step_form != OMX_STEP_DEFAULT) return false;
+    if (c->dims != 3 || c->step_form != OMX_STEP_DEFAULT || !f3_inplace_fits(c)) return false;
     if (c->f3_pin) return c->f3_pin == 1;
     return (long long)c->n[0] * c->n[1] * c->n[2] <= F3_INPLACE_MOST;
 }
@@ -3959,7 +3961,9 @@ template <class R> long long batch_step(omx_batch *b, const BatchTables<R> &T, c
 bool batch_inplace_rule(const omx_batch *b)
 {
     for (const auto *c : b->ctx) {
-        if (c->step_form != OMX_STEP_DEFAULT || (long long)c->n[0] * c->n[1] * c->n[2] > F3_INPLACE_MOST) return false;
+        if (c->step_form != OMX_STEP_DEFAULT || (long long)c->n[0] * c->n[1] * c->n[2] > F3_INPLACE_MOST ||
+            !f3_inplace_fits(c))
+            return false;
         for (const auto &g : c->groups)
             if (g->cl) return false;         // members may share a closure, whose steps run one after the other
     }

@@ -1136,14 +1136,15 @@ __device__ __forceinline__ void f3p_ade_cell(const Fused3Args &A, const GridArgs
     A.out.f[c][idx] = e;
 }
 
-// zl: leading block layers along z that take the list of dispersive component-cells
+// zl: leading block layers along z that take the list of dispersive component-cells, by strides
 __global__ void __launch_bounds__(128, F3P_E_BLOCKS) k_f3p_e(const __grid_constant__ Fused3Args A,
                                                              const __grid_constant__ GridArgs<float> G, int kch, int zl)
 {
     if ((int)blockIdx.z < zl) {
-        const int q = 128 * (int)(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)) +
-                      (int)(threadIdx.x + 32 * threadIdx.y);
-        if (q < G.ade_n) f3p_ade_cell(A, G, q);
+        const unsigned q0 = 128 * (blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)) + threadIdx.x +
+                            32 * threadIdx.y;
+        for (unsigned q = q0; q < (unsigned)G.ade_n; q += 128 * gridDim.x * gridDim.y * (unsigned)zl)
+            f3p_ade_cell(A, G, (int)q);
         return;
     }
     const int i = 1 + 32 * (int)blockIdx.x + (int)threadIdx.x, j = 1 + 4 * (int)blockIdx.y + (int)threadIdx.y;

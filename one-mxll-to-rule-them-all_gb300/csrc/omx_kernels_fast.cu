@@ -227,21 +227,29 @@ cudaError_t launch_fused3t_general(const Fused3Args &A, const GridArgs<float> &G
     return cudaGetLastError();
 }
 
-cudaError_t launch_fused3p(const Fused3Args &A, const GridArgs<float> &G, int kch, bool e_half, void *sv)
+// Block layers along z of a pass in place: `list` leading ones for the dispersive component-cells, then
+// one for every m planes.  A launch takes 65535 layers; the list takes at most half of them (its
+// threads stride over the entries: a long thin grid of dispersive cells has more), and the march is
+// lengthened until the planes fit beside it.
+struct F3pLayers { int m; unsigned list, planes; };
+static F3pLayers f3p_layers(const Lay &L, int ade_n, int kch)
 {
-    const Lay &L = G.L;
-    const dim3 b(32, 4);
+    constexpr unsigned MOST = 65535;
     // us per step at marches of 1, 2, 4, 8: 64^3 10.7, 9.8, 12.3, 18.3; 96^3 23.1, 20.5, 20.9, 23.1; 128^3
     // 48, 40, 37.8, 40.6; 160^3 112, 93, 89, 93; of 4, 8, 16: 224^3 208, 208; 256^3 298, 293, 302
     const long long tiles = (long long)((L.nx + 31) / 32) * ((L.ny + 3) / 4);
     int m = kch > 0 ? kch : std::max(march_rule(tiles, L.nz, 4, 22), march_rule(tiles, L.nz, 8, 80));
-    dim3 g((L.nx + 31) / 32, (L.ny + 3) / 4, (L.nz + m - 1) / m);
-    if (e_half) {
-        const unsigned layer = g.x * g.y * 128, zl = ((unsigned)G.ade_n + layer - 1) / layer;
-        for (; g.z + zl > 65535; m *= 2) g.z = (L.nz + 2 * m - 1) / (2 * m);
-        g.z += zl;
-        k_f3p_e<<<g, b, 0, (cudaStream_t)sv>>>(A, G, m, (int)zl);
-    } else k_f3p_h<<<g, b, 0, (cudaStream_t)sv>>>(A, G, m);
+    const unsigned list = (unsigned)std::min<long long>((ade_n + tiles * 128 - 1) / (tiles * 128), MOST / 2);
+    while ((unsigned)((L.nz - 1) / m) + 1 + list > MOST) m *= 2;
+    return {m, list, (unsigned)((L.nz - 1) / m) + 1};
+}
+
+cudaError_t launch_fused3p(const Fused3Args &A, const GridArgs<float> &G, int kch, bool e_half, void *sv)
+{
+    const F3pLayers z = f3p_layers(G.L, e_half ? G.ade_n : 0, kch);
+    const dim3 b(32, 4), g((G.L.nx + 31) / 32, (G.L.ny + 3) / 4, z.list + z.planes);
+    if (e_half) k_f3p_e<<<g, b, 0, (cudaStream_t)sv>>>(A, G, z.m, (int)z.list);
+    else k_f3p_h<<<g, b, 0, (cudaStream_t)sv>>>(A, G, z.m);
     return cudaGetLastError();
 }
 

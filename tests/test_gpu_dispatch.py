@@ -586,3 +586,36 @@ def test_single_pass_form_is_the_staged_pass(before):
     # 18 words a cell and step in place, 12 staged, beside the same CPML words
     (inplace,), (staged,) = words[omx.STEP_DEFAULT], words[omx.STEP_SINGLE_PASS]
     assert inplace - staged == 6 * 4 * 30 * 26 * 28
+
+
+# a pass in place launches at most 65535 blocks along y and along z: (32, 4, 21846) and (30, 3, 21850) all
+# dispersive have a list of more block layers than that (three entries a cell, 128 a block),
+# (32, 4, 20000) one that leaves few layers to the planes, (3, 262145, 3) has too many rows
+@pytest.mark.parametrize("n,media", [
+    ((32, 4, 21846), "all"), ((30, 3, 21850), "all"), ((32, 4, 20000), "all"), ((4, 4, 70001), "none"),
+    ((3, 262140, 3), "some"), ((3, 262145, 3), "some"),
+])
+def test_inplace_launches_of_long_thin_grids(n, media):
+    """Launch limits of the 3D pass in place: fields as from the staged pass, bit for bit, at the default
+    march and (where the rows fit) one plane a thread."""
+    dr = 37.8
+    dt = omx.units.yee_dt(dr)
+    out = []
+    for form, shape in ((omx.STEP_SINGLE_PASS, None), (omx.STEP_DEFAULT, None), (omx.STEP_DEFAULT, 1)):
+        g = omx.TMxll(3, n, 4, (1, 1, 1), dt, dr, precision="fp32")
+        if media != "none":
+            m = np.zeros(n + (3,), np.int32, order="F")    # a medium per component
+            m[tuple(slice(None) if media == "all" else slice(1, max(2, q // 2)) for q in n)] = 1
+            g.set_media([omx.medium_drude(0.33, 0.01, 1.5, dt)], m)
+        a = int(np.argmax(n))
+        g.add_plane_source(3 if a != 2 else 1, a + 1, n[a] // 2, 1e-2, 0.1, 2 * dt, 3 * dt, 0.0, 1e30)
+        g.set_step_form(form)
+        if shape:
+            g.set_launch_shape(shape)
+        g.run(1, 6)
+        out.append([g.read_field(f) for f in range(1, 7)])
+        g.kill()
+    assert max(np.max(np.abs(f)) for f in out[0]) > 0
+    for o in out[1:]:
+        for a, b in zip(o, out[0]):
+            assert np.array_equal(a, b)
