@@ -955,7 +955,8 @@ DetArgs det_args(omx_ctx *c)
 // dispersive cell.  The 3D pass (k_fused3_tma) updates the dispersive cells inside the pass,
 // before their CPML terms, as the reference does, and adds a single plane source to E_old before
 // the update (fold3); other sources follow the pass and must avoid dispersive cells.  x and y
-// must not be periodic (its staged halo holds the PEC ghosts there).
+// must not be periodic (its staged halo holds the PEC ghosts there); larger fields than the kernels' 31-bit
+// offsets reach step in two passes.
 bool fold3_of(const omx_ctx *c)
 {
     return c->dims == 3 && c->sources.size() == 1 && c->sources[0]->kind == 1;
@@ -975,6 +976,8 @@ bool fused_possible(const omx_ctx *c)
         }
     } else if (c->dims == 3) {
         if (c->per[0] || c->per[1]) return false;
+        // the fused kernels hold element offsets in 31 bits and a run's corner along x and y in 20
+        if (c->felems > 0x7fffffffu || c->n[0] >= 1 << 20 || c->n[1] >= 1 << 20) return false;
     } else {
         return false;
     }
@@ -3692,6 +3695,7 @@ BatchTables<R> batch_tables(omx_batch *b, const std::vector<RunPlan> *plans, int
                     item += (long long)e.tx * e.ty * e.tz;
                 } else {
                     // the grid's runs for the split pass, tagged with its place in the table
+                    req(c->n[2] < 1 << 20, "the batched pass split by plane form takes grids of fewer than 2^20 planes");
                     std::vector<int4> g0, l0;
                     f3t_runs(c, TY, e.kch, g0, l0);
                     for (int4 &r : g0) r.w |= gi << 20;

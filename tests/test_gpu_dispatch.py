@@ -619,3 +619,31 @@ def test_inplace_launches_of_long_thin_grids(n, media):
     for o in out[1:]:
         for a, b in zip(o, out[0]):
             assert np.array_equal(a, b)
+
+
+def test_fields_beyond_31_bit_offsets_step_in_two_passes():
+    """A 3D grid whose fields have more words than the fused pass's 31-bit offsets reach takes the two
+    half-step passes: a source beyond the limit radiates as in a small grid, bit for bit."""
+    dr = 37.8
+    dt = omx.units.yee_dt(dr)
+    out = []
+    for n, z in (((1300, 1300, 1280), 1262), ((64, 64, 64), 32)):
+        g = omx.TMxll(3, n, 4, (1, 1, 1), dt, dr, precision="fp32")
+        if n[0] > 64:
+            for staged in (8064, 8016):
+                with pytest.raises(omx.OMXError):
+                    g.set_launch_shape(staged)
+            g.set_launch_shape(4)            # planes per thread of the two passes
+        else:
+            g.set_step_form(omx.STEP_TWO_PASS)
+        off = z - n[2] // 2
+        g.add_source("z", 1e-2, 0.1, 2 * dt, 3 * dt, (0.0, 0.0, (off + 0.5) * dr if off else 0.0), 1.5 * dr, 0.0, 1e30)
+        c = (n[0] // 2, n[1] // 2, z)
+        for f in ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz"):
+            g.add_detector(omx.POINT, f, [[c[0] + a, c[1] + b, c[2] + k] for a, b, k in ((0, 0, 0), (2, 1, -2), (-3, 2, 3))])
+        g.run(1, 9, 1, 1)
+        out.append(g.drain_detectors()[1])
+        g.kill()
+    reached = np.max(np.abs(out[1]), axis=0).reshape(6, 3)
+    assert np.all(reached[:, 1:] > 0)        # on the source's axis the transverse components vanish
+    assert np.array_equal(*out)
