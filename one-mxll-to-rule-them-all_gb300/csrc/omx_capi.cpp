@@ -13,14 +13,10 @@
 #include <map>
 #include <memory>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <tuple>
 #include <type_traits>
 #include <unordered_map>
 #include <vector>
-
-#include <unistd.h>
 
 #include "../../include/omx_gpu.h"
 #include "omx_host.h"
@@ -2173,31 +2169,6 @@ double *host_stage(omx_ctx *c, size_t need)
     return c->host_stage.p;
 }
 
-// Touch the pages of a large output from a few threads: fresh pages of the caller are cleared by
-// the kernel on first touch, which one thread does at a sixth of the copy's rate (134 MB: 5.2 ms with
-// one thread, 1.7 ms with four; the copy itself 0.8 ms).  Every byte is overwritten by the copy.
-void touch_pages(void *p, size_t bytes)
-{
-    if (bytes < ((size_t)8 << 20)) return;
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE), parts = 4;
-    auto touch = [=](size_t a, size_t b) {
-        for (size_t q = a; q < b; q += page) static_cast<volatile char *>(p)[q] = 0;
-    };
-    std::vector<std::thread> th;
-    size_t done = 0;
-    try {
-        for (size_t t = 0; t + 1 < parts; ++t) {
-            const size_t a = bytes / parts * t / page * page, b = bytes / parts * (t + 1) / page * page;
-            th.emplace_back(touch, a, b);
-            done = b;
-        }
-    } catch (const std::system_error &) {
-        // no more threads: this one touches the rest
-    }
-    touch(done, bytes);
-    for (auto &t : th) t.join();
-}
-
 PackArgs pack_args(const omx_ctx *c, int field, long long &rows)
 {
     int lo[3], hi[3];
@@ -2220,10 +2191,14 @@ template <class R> void read_field_impl(omx_ctx *c, int field, double *host)
 {
     long long rows;
     const PackArgs P = pack_args(c, field, rows);
-    touch_pages(host, (size_t)rows * P.ni * sizeof(double));
+    // beside steps that still run, or once they are done; a read that fails leaves the caller's values alone
+    const size_t bytes = (size_t)rows * P.ni * sizeof(double);
+    const bool busy = cudaStreamQuery(c->stream) == cudaErrorNotReady;
+    if (busy) omx::touch_pages(host, bytes, true);
     sync_checked(c, "sync");
     const long long per = std::max<long long>(1, (long long)HOST_STAGE / P.ni);
     double *buf = host_stage(c, (size_t)std::min(per, rows) * P.ni);
+    if (!busy) omx::touch_pages(host, bytes, false);
     const R *f = field_ptrs<R>(c).f[field_code_to_index(field)];
     for (long long r = 0; r < rows; r += per) {
         const long long m = std::min(per, rows - r);

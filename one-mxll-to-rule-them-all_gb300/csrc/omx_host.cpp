@@ -1,8 +1,18 @@
 // omx_host.cpp -- set-up arithmetic of the reference restated in C++ (see omx_host.h).
 #include "omx_host.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <system_error>
+#include <thread>
+
+#include <sys/mman.h>
+#include <unistd.h>
+
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
 
 namespace omx {
 
@@ -365,6 +375,29 @@ std::vector<double> qgroup_kernel(int dims, int n_ker)
                 ker[(size_t)q] = w;
             }
     return ker;
+}
+
+void touch_pages(void *p, size_t bytes, bool keep)
+{
+    if (bytes < ((size_t)8 << 20)) return;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), parts = 4;
+    const uintptr_t lo = (uintptr_t)p / page * page, hi = (uintptr_t)p + bytes;
+    auto touch = [=](uintptr_t part) {   // the last part ends within its last page
+        const uintptr_t a = lo + (hi - lo) / parts * part / page * page;
+        const uintptr_t b = part + 1 == parts ? hi : lo + (hi - lo) / parts * (part + 1) / page * page;
+        if (keep) madvise((void *)a, b - a, MADV_POPULATE_WRITE);
+        else for (uintptr_t q = std::max(a, (uintptr_t)p); q < b; q = (q / page + 1) * page) *(volatile char *)q = 0;
+    };
+    std::vector<std::thread> th;
+    th.reserve(parts);
+    uintptr_t part = 1;
+    try {
+        for (; part < parts; ++part) th.emplace_back(touch, part);
+    } catch (const std::system_error &) {
+        for (; part < parts; ++part) touch(part);   // no more threads: this one takes the rest
+    }
+    touch(0);
+    for (auto &t : th) t.join();
 }
 
 }  // namespace omx

@@ -112,3 +112,16 @@ def test_deck_media_maps_match(omx, orc):
         assert a.max() >= 1
         for det in d["detectors"]:
             assert det["idx"].shape == (1, d["dimensions"])
+
+
+@pytest.mark.parametrize("nbytes", [(8 << 20) - 1, 8 << 20, (9 << 20) + 4097])
+def test_touching_an_output_keeps_its_values(omx, nbytes):
+    """A read touches the pages of its output while the steps before it still run: the caller's values
+    stay until the copies overwrite them, so that a read that fails leaves them alone."""
+    touch = getattr(omx.lib(), "_ZN3omx11touch_pagesEPvmb")
+    touch.argtypes, touch.restype = [C.c_void_p, C.c_size_t, C.c_bool], None
+    a = np.full(nbytes + 3, 171, np.uint8)
+    touch(a[1:].ctypes.data, nbytes, True)
+    assert np.all(a == 171)
+    touch(a[1:].ctypes.data, nbytes, False)      # once nothing can fail: within the output alone
+    assert np.all(a[:1] == 171) and np.all(a[1 + nbytes:] == 171)
