@@ -355,7 +355,9 @@ int omx_batch_create(omx_ctx *const *ctxs, int n, omx_batch **out);
  * s x 1000000 + (ring depth x 100 + tile rows) x 1000 + planes per block: the s largest grids step
  * with the pass split by plane form, the others in one launch over their tiles (s = 0: every grid
  * in that launch); ring depth 0 for the default of 4 planes.  Grids that step side by side in place
- * keep doing so when that is faster than every shape; *choice is the fastest shape then too. */
+ * keep doing so when that is faster than every shape, both timed in graphs; *choice, the fastest
+ * shape, then stands for their form: omx_batch_set_launch_shape(*choice) on this batch keeps it.
+ * Other batches of the same grids take the form in place by themselves when no shape is set. */
 int omx_batch_autotune(omx_batch *batch, int reps, int *choice);
 /* No counterpart in the reference: sets the launch shape of the batched passes, encoded as
  * omx_batch_autotune's choice (a fused shape when every member steps with the fused FP32 pass,

@@ -3458,8 +3458,10 @@ struct omx_batch {
     int f3nsplit = 0;
     // small grids (batch_inplace_rule) step in place, each member's launches on one of the lanes, so that
     // the grids fill the GPU together; staged: a launch shape was set, or the tuner found the staged
-    // pass faster
+    // pass faster; tuned: the staged shape that the tuner reported when it kept the members in place (0:
+    // none), which stands for that choice
     bool staged = false;
+    int tuned = 0;
     static constexpr int LANES = 12;
     cudaStream_t lane[LANES] = {};
     cudaEvent_t ev_lane[LANES] = {};
@@ -4101,19 +4103,10 @@ template <class R> int batch_autotune_impl(omx_batch *b, int reps)
         cudaEvent_t e0, e1;
         ck(cudaEventCreate(&e0), "event");
         ck(cudaEventCreate(&e1), "event");
-        float best = 0.f, inplace = 0.f;
+        float best = 0.f;
         int pick = 8064;
         bool first = true;
-        const bool may = batch_inplace_rule(b);   // the in-place pass is timed beside the staged shapes
-        if (may) {
-            batch_lanes(b);
-            batch_inplace_steps<R>(b, nullptr, 1);
-            ck(cudaEventRecord(e0, b->stream), "event");
-            batch_inplace_steps<R>(b, nullptr, reps);
-            ck(cudaEventRecord(e1, b->stream), "event");
-            ck(cudaEventSynchronize(e1), "batch autotune");
-            ck(cudaEventElapsedTime(&inplace, e0, e1), "batch autotune");
-        }
+        const bool may = batch_inplace_rule(b);   // the members in place compete with the best staged shape
         for (auto *c : b->ctx) second_set(c);
         int dev = 0, optin = 0;
         ck(cudaGetDevice(&dev), "device");
@@ -4144,12 +4137,48 @@ template <class R> int batch_autotune_impl(omx_batch *b, int reps)
                             first = false;
                         }
                     }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
         b->f3nsplit = pick / 1000000;
         b->f3form = pick / 1000 % 1000;
         b->f3kch = pick % 1000;
-        b->staged = !may || inplace > best;
+        if (may) {
+            // both from graphs of the length that runs replay: two launches per member and step are
+            // bound by the host when they are issued one by one
+            const int steps = std::min(reps, 8), times = (reps + steps - 1) / steps;
+            auto replayed = [&](const std::function<void()> &passes) {
+                passes();
+                cudaGraphExec_t exec = nullptr;
+                {
+                    Capture capture(b->stream);
+                    passes();
+                    cudaGraph_t graph = capture.end();
+                    const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
+                    cudaGraphDestroy(graph);
+                    ck(e, "instantiate");
+                }
+                cudaError_t e = cudaGraphLaunch(exec, b->stream);
+                cudaEventRecord(e0, b->stream);
+                for (int r = 0; r < times && e == cudaSuccess; ++r) e = cudaGraphLaunch(exec, b->stream);
+                cudaEventRecord(e1, b->stream);
+                float ms = 0.f;
+                if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+                if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+                cudaGraphExecDestroy(exec);
+                ck(e, "batch autotune");
+                return ms;
+            };
+            batch_lanes(b);
+            const float inplace = replayed([&]() { batch_inplace_steps<R>(b, nullptr, steps); });
+            const BatchTables<R> T = batch_tables<R>(b, nullptr, b->f3kch, 0);
+            const float staged = replayed([&]() {
+                for (int r = 0; r < steps; ++r) batch_fused_pass(b, T, b->f3form);
+            });
+            b->staged = staged < inplace;
+        } else {
+            b->staged = true;
+        }
+        b->tuned = b->staged ? 0 : pick;
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
         return pick;
     }
     cudaEvent_t e0, e1;
@@ -4268,7 +4297,7 @@ int omx_batch_set_launch_shape(omx_batch *b, int shape)
         b->f3nsplit = shape / 1000000;
         b->f3form = form;
         b->f3kch = kch;
-        b->staged = true;
+        b->staged = shape != b->tuned;
     } else {
         req(shape == 4 || shape == 8 || shape == 16 || shape == 32, "batched two-pass shape: tile depth 4, 8, 16 or 32");
         b->kch = shape;

@@ -647,3 +647,37 @@ def test_fields_beyond_31_bit_offsets_step_in_two_passes():
     reached = np.max(np.abs(out[1]), axis=0).reshape(6, 3)
     assert np.all(reached[:, 1:] > 0)        # on the source's axis the transverse components vanish
     assert np.array_equal(*out)
+
+
+def test_batch_tuners_choice_keeps_its_form():
+    """omx_batch_set_launch_shape(omx_batch_autotune's choice) keeps the form that the tuner kept; another
+    shape selects the staged pass.  Results as from an untuned batch, bit for bit."""
+    dt = omx.units.yee_dt(37.8)
+
+    def build():
+        grids = [omx.TMxll(3, n, 4, (3,) * 3, dt, 37.8, precision="fp32") for n in ((30, 26, 28), (24, 33, 29))]
+        for g in grids:
+            g.add_plane_source(1, 3, 14, 1e-2, 0.1, 4 * dt, 5 * dt, 0.0, 1e30)
+        return grids, omx.Batch(grids)
+
+    grids, b = build()
+    choice = b.autotune(reps=20)
+    form = []
+    for tt, shape in ((1, None), (6, choice), (11, 8016 if choice != 8016 else 8032), (16, choice)):
+        if shape:
+            b.set_launch_shape(shape)
+        b.run(tt, 5)
+        b.synchronize()
+        form.append([g.algorithmic_bytes(omx.KC_E) for g in grids])
+    assert form[0] == form[1] == form[3]
+    cells = np.array([30 * 26 * 28, 24 * 33 * 29])
+    assert np.all((np.array(form[0]) - form[2] == 24 * cells) | (np.array(form[0]) == form[2]))
+    plain, b2 = build()
+    b2.run(1, 20)
+    b2.synchronize()
+    for g, q in zip(grids, plain):
+        for f in range(1, 7):
+            assert np.array_equal(g.read_field(f), q.read_field(f))
+    assert np.max(np.abs(plain[0].read_field(1))) > 0
+    for x in (b, b2, *grids, *plain):
+        x.kill()
