@@ -340,8 +340,8 @@ int omx_set_launch_shape(omx_ctx *ctx, int shape);
  * runs' new E, the other grids' one launch on that second stream too), one
  * launch per round of the other sources, the per-grid emitter work and one launch for the
  * detectors of every grid; a batch of grids that all step in place by themselves runs them side by
- * side on a few streams instead, each grid's launches as its own omx_run issues them.  Otherwise each step runs ONE persistent launch for the H pass of
- * every grid (its blocks walk a list of all grids' tiles), one launch per round of radial sources
+ * side on a few streams instead, each grid's launches as its own omx_run issues them, unless they
+ * are many and small.  Otherwise each step runs ONE persistent launch for the H pass of every grid (its blocks walk a list of all grids' tiles), one launch per round of radial sources
  * (round r: source r of every grid), the dispersive cells, ONE launch for the bulk E pass of every
  * grid, the per-grid emitter work and the detectors.  use_graph != 0 captures that step once and
  * replays it.  Every grid computes exactly what omx_run computes for it alone (same arithmetic,

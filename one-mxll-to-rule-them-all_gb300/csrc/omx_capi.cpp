@@ -3790,6 +3790,14 @@ void batch_lanes(omx_batch *b)
     }
 }
 
+constexpr long long BATCH_LARGE_MEMBER = 400000;   // cells
+long long batch_mean_cells(const omx_batch *b)
+{
+    long long cells = 0;
+    for (const auto *c : b->ctx) cells += (long long)c->n[0] * c->n[1] * c->n[2];
+    return cells / (long long)b->ctx.size();
+}
+
 // `steps` steps of every member in place: member i's own launches (H, E, sources, emitter work,
 // detectors, as its omx_run issues them) on lane i mod LANES, forked from the batch's stream and
 // joined to it at the end; no member waits for another.  plans null: the field passes alone.  The
@@ -3801,9 +3809,7 @@ template <class R> long long batch_inplace_steps(omx_batch *b, const std::vector
     // step with 1, 2, 3, 4, 12 lanes: twelve grids of 0.70 M cells 338, 270, 260, 261, 274; 32 of 0.99 M
     // 1126, 901, 897, 906, 935; twelve of 0.11 M 114, 73, 59, 53, 48; sixteen of 0.03 M 129, 79, 64, 50, 37
     const int n = (int)b->ctx.size();
-    long long cells = 0;
-    for (const auto *c : b->ctx) cells += (long long)c->n[0] * c->n[1] * c->n[2];
-    const int lanes = std::min(n, cells / n >= 400000 ? 4 : omx_batch::LANES);
+    const int lanes = std::min(n, batch_mean_cells(b) >= BATCH_LARGE_MEMBER ? 4 : omx_batch::LANES);
     long long k = 0;
     ck(cudaEventRecord(b->ev_fork, b->stream), "event");
     for (int l = 0; l < lanes; ++l) ck(cudaStreamWaitEvent(b->lane[l], b->ev_fork, 0), "event");
@@ -3936,11 +3942,16 @@ template <class R> long long batch_step(omx_batch *b, const BatchTables<R> &T, c
 }
 
 // In place or staged for a batch of grids that the fused pass can step: in place when every member
-// would step so by itself.  Measured, us per step, staged in the best of four shapes / in place: twelve
-// grids of 8.4 M cells in all 310 / 261, twelve of 1.3 M 85 / 48, three of 2.6 M 127 / 65, four of
-// 17.7 M 446 / 410, 32 of 31.7 M 906 / 906.
+// would step so by itself, unless there are many of them and small: a member's four or five launches a
+// step take the GPU about 2.5 us to start, the staged batch's few serve every member.  Measured, us per
+// step, staged in the best of four shapes / in place: twelve grids of 8.4 M cells in all 310 / 261, twelve
+// of 1.3 M 85 / 48, three of 2.6 M 127 / 65, four of 17.7 M 446 / 410, 32 of 31.7 M 906 / 906; 32, 48, 64
+// and 128 grids of 32^3 112 / 67, 126 / 107, 133 / 160, 245 / 318, of 56^3 299 / 286, 418 / 428, 456 /
+// 575, 876 / 1141, of 80^3 (32, 48, 64) 657 / 576, 932 / 858, 1202 / 1144.
+constexpr size_t BATCH_INPLACE_SMALL = 48;
 bool batch_inplace_rule(const omx_batch *b)
 {
+    if (b->ctx.size() > BATCH_INPLACE_SMALL && batch_mean_cells(b) < BATCH_LARGE_MEMBER) return false;
     for (const auto *c : b->ctx) {
         if (c->step_form != OMX_STEP_DEFAULT || (long long)c->n[0] * c->n[1] * c->n[2] > F3_INPLACE_MOST ||
             !f3_inplace_fits(c))

@@ -681,3 +681,30 @@ def test_batch_tuners_choice_keeps_its_form():
     assert np.max(np.abs(plain[0].read_field(1))) > 0
     for x in (b, b2, *grids, *plain):
         x.kill()
+
+
+@pytest.mark.parametrize("n,count,inplace", [(20, 48, True), (20, 49, False), (74, 49, True)])
+def test_batch_form_by_number_and_size_of_members(n, count, inplace):
+    """Many small grids step in the staged batch, few or larger ones in place; members equal solo runs."""
+    dt = omx.units.yee_dt(37.8)
+
+    def build(k):
+        g = omx.TMxll(3, (n, n, n), 4, (3,) * 3, dt, 37.8, precision="fp32")
+        g.add_plane_source(1, 3, n // 2, 1e-2 * (1 + k), 0.1, 4 * dt, 5 * dt, 0.0, 1e30)
+        return g
+
+    grids = [build(k) for k in range(count)]
+    b = omx.Batch(grids)
+    b.run(1, 9)
+    b.synchronize()
+    solo = build(count - 1)
+    solo.set_step_form(omx.STEP_SINGLE_PASS)
+    solo.run(1, 9)
+    staged = solo.algorithmic_bytes(omx.KC_E)
+    for g in (grids[0], grids[-1]):
+        assert g.algorithmic_bytes(omx.KC_E) - staged == (24 * n ** 3 if inplace else 0)
+    for f in range(1, 7):
+        assert np.array_equal(grids[-1].read_field(f), solo.read_field(f))
+    assert np.max(np.abs(solo.read_field(1))) > 0
+    for x in (b, solo, *grids):
+        x.kill()
