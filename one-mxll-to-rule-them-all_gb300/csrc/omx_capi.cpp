@@ -2100,10 +2100,14 @@ template <class R> int autotune_impl(omx_ctx *c, int reps)
     } else if (c->dims == 3) {
         cand = {1, 2, 4, 8, 16, 32};
     } else if (c->dims == 2) {
-        cand = {8, 16, 32, 64};
+        // the marches that the rule by size chooses from (1..8) and longer ones
+        cand = {1, 2, 4, 8, 16, 32, 64};
     } else {
         return 0;
     }
+    if (!fused)   // a launch takes 65535 blocks along the marched axis
+        cand.erase(std::remove_if(cand.begin(), cand.end(), [&](int m) { return (c->n[c->dims - 1] - 1) / m >= 65535; }),
+                   cand.end());
     auto select = [&](int v) { apply_shape(c, v); };
     auto once = [&]() {
         if (fused) {

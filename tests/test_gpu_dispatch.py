@@ -708,3 +708,25 @@ def test_batch_form_by_number_and_size_of_members(n, count, inplace):
     assert np.max(np.abs(solo.read_field(1))) > 0
     for x in (b, solo, *grids):
         x.kill()
+
+
+# (8, 70001): more rows than a launch takes blocks along y
+@pytest.mark.parametrize("n,precision,mode", [((243, 161), "fp32", 2), ((243, 161), "fp64", 1), ((8, 70001), "fp32", 2)])
+def test_tuner_of_unfused_2d_grids(n, precision, mode):
+    """The tuner looks at the short marches that the rule by size takes on small grids (a march of 8 rows
+    takes such a grid twice as long); the tuned grid gives the untuned one's bits."""
+    dt = omx.units.yee_dt(37.8)
+    out = []
+    for tuned in (False, True):
+        g = omx.TMxll(2, n, 3, (2, 3, 1), dt, 37.8, mode=mode, precision=precision)
+        comp = 3 if mode == 1 else 1
+        g.add_plane_source(comp, 2, n[1] // 2, 1e-2, 0.1, 4 * dt, 5 * dt, 0.0, 1e30)
+        if tuned:
+            choice = g.autotune(reps=10)
+            assert choice <= 4 if n[1] < 65536 else choice >= 2
+        g.run(1, 12)
+        out.append([g.read_field(f) for f in ((3, 4, 5) if mode == 1 else (1, 2, 6))])
+        g.kill()
+    assert np.max(np.abs(out[0][0])) > 0
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
