@@ -1734,19 +1734,23 @@ StepParam plan_param(omx_ctx *c, const RunPlan &plan, int row) { return StepPara
 // emitters or cells that one cluster would be slow on or has no shared memory for (2048 FP64 cells a
 // block).  Measured, us per step in one launch / in launches, FP64 with a Drude film: 200 cells 3.1 /
 // 12.4, with 16 emitters 1500 cells 6.5 / 24.7, 12000 cells 8.6 / 24.9; 6000 cells with 256 emitters
-// 8.6 / 24.7, 512 12.9 / 26.5, 1024 (all through memory) 24.3 / 26.7.
-constexpr int RUN1_CELLS = 16384, RUN1_EMITTERS = 512, RUN1_TAPS = 2048;
+// 8.6 / 24.7, 512 12.9 / 26.5, 1024 (all through memory) 24.3 / 26.7; 12000 cells with one source of 4001
+// points 8.9 / 10.3, four of 1025 11.9 / 14.4, four of 4001 20.3 / 14.5.
+constexpr int RUN1_CELLS = 16384, RUN1_EMITTERS = 512, RUN1_TAPS = 2048, RUN1_POINTS = 8192;
 bool run1_ok(const omx_ctx *c, int nsteps, int use_graph)
 {
     const int n = c->n[0];
     if (c->dims != 1 || !use_graph || c->prof || nsteps < 2 || c->n_freq > 0 || c->taps_h) return false;
     if (n > RUN1_CELLS || (int)c->sources.size() > RUN1_SOURCES || (int)c->groups.size() > RUN1_GROUPS) return false;
     if ((int)c->tap_field.size() > RUN1_TAPS) return false;
+    size_t points = 0;
     for (const auto &S : c->sources) {
         if (S->kind == 0) {
-            if (S->comp != 0) return false;
-            for (const int4 &p : S->cells)
-                if (p.x < 1 || p.x > n) return false;
+            if (S->comp != 0 || (points += S->cells.size()) > RUN1_POINTS) return false;
+            for (size_t q = 0; q < S->cells.size(); ++q) {
+                const int x = S->cells[q].x;
+                if (x < 1 || x > n || x != S->cells[0].x + (int)q) return false;
+            }
         } else if (S->pd.plane_axis != 1 || S->pd.comp != 1 || S->pd.plane_index < 1 || S->pd.plane_index > n) {
             return false;
         }
@@ -1770,8 +1774,12 @@ template <class R> void run1(omx_ctx *c, const RunPlan &plan, int nsteps)
     for (int q = 0; q < A.n_src; ++q) {
         const SourceRec &S = *c->sources[q];
         A.src_kind[q] = S.kind;
-        if (S.kind == 0) A.src[q] = src_args(S);
-        else A.plane_e[q] = eindex(c, S.pd.plane_index, 0, 0);
+        if (S.kind == 0) {
+            A.src[q] = src_args(S);
+            A.src_first[q] = S.cells[0].x;
+        } else {
+            A.plane_e[q] = eindex(c, S.pd.plane_index, 0, 0);
+        }
         A.plane_c[q] = S.c_src;
     }
     A.n_grp = (int)c->groups.size();

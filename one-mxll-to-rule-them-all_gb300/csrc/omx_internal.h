@@ -197,6 +197,7 @@ struct Run1Args {
     int n_src;
     int src_kind[RUN1_SOURCES];            // 0 radial, 1 plane
     SrcArgs src[RUN1_SOURCES];
+    int src_first[RUN1_SOURCES];           // first cell of a radial source, whose points are cells in a row
     long long plane_e[RUN1_SOURCES];       // E word of a plane source's cell
     double plane_c[RUN1_SOURCES];
     int n_grp;

@@ -730,3 +730,39 @@ def test_tuner_of_unfused_2d_grids(n, precision, mode):
     assert np.max(np.abs(out[0][0])) > 0
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+# radial sources of one point, of a piece of the cells or less, over several pieces, from the first cell to
+# the last, and of more points than the loop in one launch takes
+@pytest.mark.parametrize("n,radii", [(200, (0, 30)), (1500, (16, 256, 400)), (6151, (2000, 16, 700, 1)),
+                                     (401, (200,)), (6151, (1400, 1400, 1400))])
+def test_one_launch_1d_loop_wide_sources(n, radii):
+    """Radial 1D sources of any width in the loop in one launch: the bits of one launch per phase, and
+    no slower than those (a thread looks at its own cells, not at every point)."""
+    import time
+
+    dr = 37.8
+    dt = omx.units.yee_dt(dr)
+    out, took = [], []
+    for graph in (True, False):
+        g = omx.TMxll(1, (n,), 5, (3, 1, 1), dt, dr, precision="fp64")
+        for q, r in enumerate(radii):
+            at = 0 if r >= n // 2 - 1 else (q - 1) * (n // 2 - r - 1) // 2
+            g.add_source("x", 1e-2 * (q + 1), 0.1 + 0.03 * q, 5 * dt, 6 * dt, [(at + (0.5 if at >= 0 else -0.5)) * dr],
+                         (r + 0.5) * dr, 0.0, 1e30)
+        g.add_detector(omx.POINT, "Ex", [[n // 2]])
+        g.run(1, 40, 1, 3, use_graph=graph)
+        out.append([g.drain_detectors()[1]] + [g.read_field(f) for f in (1, 5)])
+        t = []
+        for k in range(5):
+            g.synchronize()
+            t0 = time.perf_counter()
+            g.run(41 + 100 * k, 100, use_graph=graph)
+            g.synchronize()
+            t.append(time.perf_counter() - t0)
+        took.append(min(t))
+        g.kill()
+    assert all(np.max(np.abs(v)) > 0 for v in out[0])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+    assert took[0] < took[1]
