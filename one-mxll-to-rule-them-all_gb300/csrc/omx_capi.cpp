@@ -1054,15 +1054,29 @@ void second_set(omx_ctx *c)
 // cells.  Measured, us per step with a gold sphere and 10-cell CPML on every face, in place / staged
 // (default shapes): 32^3 7.9 / 25.4, 64^3 10.7 / 27.4, 96^3 20.5 / 62.8, 128^3 37.9 / 99.4, 160^3
 // 89 / 139, 192^3 140 / 173, 224^3 208 / 233, 256^3 293 / 318, 288^3 403 / 419, 320^3 537 / 529, 384^3
-// 879 / 820; with 1e5 emitters, which overlap the in-place step's H pass only, 320 x 288 x 250 482 / 438.
+// 879 / 820; with 1e5 emitters 320 x 288 x 250 482 / 438.
+// Emitters overlap the in-place step's H pass only, the whole staged pass: the more of them and the
+// larger the grid (the less there is to gain), the sooner the staged pass wins, by F3_INPLACE_WORK on
+// emitters x cells^2.  Three-level emitters in an empty grid with 8-cell CPML, 3e4 / 1e5 / 3e5 of them:
+// 96^3 in place 58 / 118 / 260, staged 80 / 121 / 259; 128^3 88 / 146 / 298, 104 / 142 / 280; 160^3 135 /
+// 187 / 340, 146 / 171 / 317; 200^3 208 / 267 / 420, 202 / 231 / 377; 256^3 347 / 393 / 548, 317 / 355 / 503
+// (3000: 310, 306).
 // Its launches hold the rows of at most 65535 blocks of four; the staged pass takes any number.
 constexpr long long F3_INPLACE_MOST = 18000000;
+constexpr double F3_INPLACE_WORK = 7e17;
+bool f3_inplace_emitters(const omx_ctx *c)
+{
+    double ne = 0.0;
+    for (const auto &g : c->groups) ne += g->d.n_systems;
+    const double cells = (double)c->n[0] * c->n[1] * c->n[2];
+    return ne * cells * cells <= F3_INPLACE_WORK;
+}
 bool f3_inplace_fits(const omx_ctx *c) { return c->n[1] <= 4 * 65535; }
 bool f3_inplace_rule(const omx_ctx *c)
 {
     if (c->dims != 3 || c->step_form != OMX_STEP_DEFAULT || !f3_inplace_fits(c)) return false;
     if (c->f3_pin) return c->f3_pin == 1;
-    return (long long)c->n[0] * c->n[1] * c->n[2] <= F3_INPLACE_MOST;
+    return (long long)c->n[0] * c->n[1] * c->n[2] <= F3_INPLACE_MOST && f3_inplace_emitters(c);
 }
 
 void prepare(omx_ctx *c)
@@ -2088,7 +2102,9 @@ template <class R> int autotune_impl(omx_ctx *c, int reps)
     // 3D FP32 with the fused pass eligible: the two half-step passes in place compete too (shapes
     // below 1000: planes marched per thread); where their one buffer set fits in L2 (small grids)
     // they can beat the staged pass, whose ping-pong sets take twice the room
-    const bool both = fused && c->dims == 3 && c->step_form == OMX_STEP_DEFAULT;
+    // (the zero-field timing leaves the emitters out: where they decide, the passes in place do not)
+    const bool both = fused && c->dims == 3 && c->step_form == OMX_STEP_DEFAULT && f3_inplace_fits(c) &&
+                      f3_inplace_emitters(c);
     if (fused) second_set(c);
     std::vector<int> cand;
     if (fused && c->dims == 3) {

@@ -766,3 +766,31 @@ def test_one_launch_1d_loop_wide_sources(n, radii):
     for a, b in zip(*out):
         assert np.array_equal(a, b)
     assert took[0] < took[1]
+
+
+@pytest.mark.parametrize("emitters,tuned,inplace", [(41723, False, True), (41724, False, False), (41724, True, False)])
+def test_3d_form_by_emitters(emitters, tuned, inplace):
+    """Emitters overlap less of the step in place: past emitters x cells^2 = 7e17 a grid takes the staged
+    pass, tuned or not; both forms give the same bits."""
+    n, dr = (160, 160, 160), 37.8
+    ev, dt = omx.UNITS["ev_to_au"], omx.units.yee_dt(37.8)
+    out, words = [], []
+    for form in (omx.STEP_DEFAULT, omx.STEP_SINGLE_PASS):
+        g = omx.TMxll(3, n, 4, (3,) * 3, dt, dr, precision="fp32")
+        g.set_step_form(form)
+        g.add_plane_source(1, 3, 80, 1e-2, 2.5 * ev, 2 * dt, 3 * dt, 0.0, 1e30)
+        r = np.random.default_rng(1)
+        cells = np.stack([r.integers(20, m - 20, emitters) for m in n], 1).astype(np.int32)
+        par = [np.full((emitters, 1), 2.5 * ev), np.full((emitters, 1), 2.0), np.full((emitters, 1), 4e4),
+               np.full((emitters, 1), 4e3), r.uniform(0.2, 1.0, (emitters, 3))]
+        q = g.add_q_group(omx.Q_MATERIAL, omx.TWO_LEVEL, cells, np.concatenate(par, 1), 1e-5, dt)
+        if tuned:
+            g.autotune(reps=1)
+        g.run(1, 7)
+        words.append(g.algorithmic_bytes(omx.KC_E))
+        out.append([g.read_field(f) for f in range(1, 7)] + [q.read()["rho"]])
+        g.kill()
+    assert words[0] - words[1] == (24 * 160 ** 3 if inplace else 0)
+    assert np.max(np.abs(out[0][0])) > 0 and np.max(np.abs(out[0][-1])) > 0
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
