@@ -366,12 +366,19 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 9 : 5)) k_e3(FieldPtrs<
 // ===================================================================================== 2D
 // TMz (Ez, Hx, Hy): mxll_2D_mod.f90:469-554 and :661-750.
 // TEz (Ex, Ey, Hz): :556-634 and :752-862.
+// A 2D thread's march among the rows' marches.  FP32 blocks are one thread high (block_xy): with the
+// general index k_h2 takes 48 registers instead of 40, and the emitter blocks beside it fewer places
+// (TEz 3000 x 2000 with 2e4 emitters, marches of 32 rows: 95 against 76 us per step).
+template <class R> __device__ __forceinline__ int row_of_block()
+{
+    return (int)(sizeof(R) == 4 ? blockIdx.y : blockIdx.y * blockDim.y + threadIdx.y);
+}
 template <class R, bool EXACT>
 __global__ void __launch_bounds__(128) k_h2(FieldPtrs<R> F, GridArgs<R> G, int jch)
 {
     const Lay L = G.L;
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j0 = 1 + (blockIdx.y * blockDim.y + threadIdx.y) * jch;
+    const int j0 = 1 + row_of_block<R>() * jch;
     if (G.step_inc && i == 1 && j0 == 1) *G.step_inc += 1;   // device-loop step counter
     if (i > L.nx || j0 > L.ny) return;
     const int j1 = min(L.ny, j0 + jch - 1);
@@ -450,7 +457,7 @@ __global__ void __launch_bounds__(128) k_e2(FieldPtrs<R> F, GridArgs<R> G, int j
 {
     const Lay L = G.L;
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j0 = 1 + (blockIdx.y * blockDim.y + threadIdx.y) * jch;
+    const int j0 = 1 + row_of_block<R>() * jch;
     if (i > L.nx || j0 > L.ny) return;
     const int j1 = min(L.ny, j0 + jch - 1);
     const long long mx = (i == 1 && G.per[0]) ? (long long)(L.nx - 1) : -1LL;
