@@ -2203,7 +2203,12 @@ template <class R> int autotune_impl(omx_ctx *c, int reps)
 // Dense FP64 rows go to the host through a device buffer of this size: a kernel unpitches and
 // converts, and each chunk is one copy straight into the caller's pages.  (A copy of the padded FP32
 // array and a host loop over its cells took 40.6 ms for a 4096^2 component; this 2.6 ms.)
+// Below these sizes a plain copy and a host loop cost less than a launch before the copy: a 1D field of
+// 1000 cells 33 against 39 us, of 4000 cells 36 against 35; 16, 1000, 2000
+// emitters 46, 59, 70 against 67, 72, 80 us, 4000 98 against 86.
 constexpr size_t HOST_STAGE = (size_t)1 << 21;   // doubles (16 MB)
+constexpr size_t HOST_FIELD = 4096;              // words of a padded array
+constexpr size_t HOST_EMITTERS = 2500;
 
 double *host_stage(omx_ctx *c, size_t need)
 {
@@ -2233,9 +2238,24 @@ template <class R> void read_field_impl(omx_ctx *c, int field, double *host)
 {
     long long rows;
     const PackArgs P = pack_args(c, field, rows);
+    if (c->felems <= HOST_FIELD) {
+        sync_checked(c, "sync");
+        std::vector<R> tmp(c->felems);
+        ck(cudaMemcpy(tmp.data(), field_ptrs<R>(c).f[field_code_to_index(field)], c->felems * sizeof(R),
+                      cudaMemcpyDeviceToHost), "read field");
+        for (long long r = 0; r < rows; ++r) {
+            const int j = P.lo[1] + (int)(r % P.nj), k = P.lo[2] + (int)(r / P.nj);
+            for (int x = 0; x < P.ni; ++x) {
+                const int i = P.lo[0] + x;
+                const bool ghost = i == P.zero[0] || j == P.zero[1] || k == P.zero[2];
+                host[r * P.ni + x] = ghost ? 0.0 : (double)tmp[(size_t)eindex(c, i, j, k)];
+            }
+        }
+        return;
+    }
     // beside steps that still run, or once they are done; a read that fails leaves the caller's values alone
     const size_t bytes = (size_t)rows * P.ni * sizeof(double);
-    const bool busy = cudaStreamQuery(c->stream) == cudaErrorNotReady;
+    const bool busy = bytes >= omx::TOUCH_LEAST && cudaStreamQuery(c->stream) == cudaErrorNotReady;
     if (busy) omx::touch_pages(host, bytes, true);
     sync_checked(c, "sync");
     const long long per = std::max<long long>(1, (long long)HOST_STAGE / P.ni);
@@ -2995,10 +3015,18 @@ int omx_qgroup_read(omx_ctx *c, int gid, double *dipole, double *dPdt, double *e
     GroupRec &g = *c->groups[gid];
     ck(cudaStreamSynchronize(c->stream), "sync");
     const size_t n = (size_t)g.d.n_systems;
-    // device rows back into the caller's emitter order, on the device
-    double *buf = host_stage(c, n * (size_t)std::max(3, g.nst));
+    // device rows back into the caller's emitter order, on the device unless they are few
+    std::vector<double> tmp;
+    double *buf = n > HOST_EMITTERS ? host_stage(c, n * (size_t)std::max(3, g.nst)) : nullptr;
     auto get = [&](double *out, const double *dev, int w) {
         if (!out) return;
+        if (!buf) {
+            tmp.resize(n * w);
+            ck(cudaMemcpy(tmp.data(), dev, n * w * sizeof(double), cudaMemcpyDeviceToHost), "read");
+            for (size_t r = 0; r < n; ++r)
+                std::copy(tmp.begin() + r * w, tmp.begin() + (r + 1) * w, out + (size_t)g.order[r] * w);
+            return;
+        }
         launch_scatter_rows(dev, g.order_d.p, (long long)n, w, buf, c->stream);
         ck(cudaPeekAtLastError(), "read");
         ck(cudaMemcpyAsync(out, buf, n * w * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "read");

@@ -379,7 +379,7 @@ std::vector<double> qgroup_kernel(int dims, int n_ker)
 
 void touch_pages(void *p, size_t bytes, bool keep)
 {
-    if (bytes < ((size_t)8 << 20)) return;
+    if (bytes < TOUCH_LEAST) return;
     const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), parts = 4;
     const uintptr_t lo = (uintptr_t)p / page * page, hi = (uintptr_t)p + bytes;
     auto touch = [=](uintptr_t part) {   // the last part ends within its last page

@@ -48,6 +48,7 @@ std::vector<double> qgroup_kernel(int dims, int n_ker);
 // one thread, 1.3 ms with four; the copy itself 0.8 ms).  keep: their contents stay (MADV_POPULATE_WRITE,
 // 1.7 ms; reading and writing back a byte per page maps zero pages first and takes 40 ms to replace
 // them).  A kernel without that call leaves the pages to the copy.
+constexpr size_t TOUCH_LEAST = (size_t)8 << 20;   // smaller outputs are left to the copy
 void touch_pages(void *p, size_t bytes, bool keep);
 
 }  // namespace omx

@@ -816,3 +816,48 @@ def test_fd_1d_operator(orc, n, n_der):
         assert t1 < 2.0 * t2                 # 0.64 measured, 2.2 with every component in each component's thread
         P.kill()
     G.kill()
+
+
+# padded arrays of at most 4096 words and groups of at most 2500 emitters are arranged on the host, larger
+# ones on the device; ghost planes of periodic axes read as zero
+@pytest.mark.parametrize("dims,n,bnd,emitters", [
+    (1, (4079,), (3, 1, 1), 2500), (1, (4080,), (3, 1, 1), 2501), (1, (4063,), (3, 1, 1), 1), (2, (60, 62), (2, 3, 1), 7),
+    (2, (60, 63), (3, 2, 1), 3000), (3, (11, 9, 20), (2, 3, 2), 40), (3, (27, 9, 30), (3, 2, 2), 400),
+])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_reads_of_small_and_large_arrays(dims, n, bnd, emitters, precision):
+    """Fields read as written, on both sides of the sizes where the way of reading changes, and emitters in
+    the caller's order, each with the state that it has alone."""
+    dr = 37.8
+    ev, dt = omx.UNITS["ev_to_au"], omx.units.yee_dt(37.8)
+    rng = np.random.default_rng(sum(n))
+    g = omx.TMxll(dims, n, 2, bnd, dt, dr, mode=1, precision=precision)
+    fields = {1: [1, 5], 2: [3, 4, 5], 3: [1, 2, 3, 4, 5, 6]}[dims]
+    for f in fields:
+        lo, hi = g.field_bounds(f)
+        a = np.asfortranarray(rng.standard_normal([h - b + 1 for b, h in zip(lo, hi)]).astype(np.float32).astype(float))
+        g.write_field(f, a)
+        for x in range(dims):
+            if f <= 3 and bnd[x] == 2 and hi[x] == n[x] + 1:
+                a[(slice(None),) * x + (-1,)] = 0.0
+        assert np.array_equal(g.read_field(f), a)
+    cells = np.stack([rng.integers(2, m - 1, emitters) for m in n], 1).astype(np.int32)
+    w = rng.uniform(1.0, 3.0, emitters) * ev
+    par = np.stack([w, np.full(emitters, 2.0), np.full(emitters, 4e4), np.full(emitters, 4e3)], 1)
+    q = g.add_q_group(omx.Q_MATERIAL, omx.TWO_LEVEL, cells,
+                      np.concatenate([par, np.ones((emitters, 3))], 1), 1e-9, dt)
+    g.q_group_step(q, 1)
+    got = q.read()
+    pick = sorted(set(rng.integers(0, emitters, 5)) | {0, emitters - 1})
+    one = omx.TMxll(dims, n, 2, bnd, dt, dr, mode=1, precision=precision)
+    for f in fields:
+        one.write_field(f, g.read_field(f))
+    alone = [one.add_q_group(omx.Q_MATERIAL, omx.TWO_LEVEL, cells[e:e + 1],
+                             np.concatenate([par[e:e + 1], np.ones((1, 3))], 1), 1e-9, dt) for e in pick]
+    for e, r in zip(pick, alone):
+        one.q_group_step(r, 1)
+        for k, v in r.read().items():
+            assert np.array_equal(v[0], got[k][e]), (e, k)
+    assert np.max(np.abs(got["E"])) > 0
+    g.kill()
+    one.kill()
