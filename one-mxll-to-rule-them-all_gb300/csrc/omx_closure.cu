@@ -249,8 +249,7 @@ __device__ __forceinline__ bool cl_wg_masked(int row, int col)
     return (row >= 2 * CL_H && row < 3 * CL_H && col >= CL_W) || (row >= 3 * CL_H && col < CL_W);
 }
 
-// FP32 master -> BF16 weights (row-major and transposed), masked Wg, padded read-out row
-// row of the gate weights in the deployment order: tile b of 128 rows holds hidden units
+// row of the gate weights in the GRU epilogue's order: tile b of 128 rows holds hidden units
 // 32b .. 32b+31, four consecutive rows per unit in gate order r, z, nx, nh (the fused GRU epilogue)
 __device__ __forceinline__ int cl_gate_perm(int r)
 {
@@ -258,7 +257,9 @@ __device__ __forceinline__ int cl_gate_perm(int r)
     return 128 * (j / 32) + 4 * (j % 32) + gate;
 }
 
-__global__ void k_cl_refresh(const float *__restrict__ p, uint16_t *wg, uint16_t *wgT, uint16_t *w1, uint16_t *w1T,
+// FP32 master -> BF16 weights (row-major and transposed; the masked gate weights in the epilogue's order and
+// transposed), padded read-out row
+__global__ void k_cl_refresh(const float *__restrict__ p, uint16_t *wgT, uint16_t *w1, uint16_t *w1T,
                              uint16_t *w2, uint16_t *w2T, uint16_t *w3, uint16_t *w3T, uint16_t *w4, uint16_t *w4T,
                              float *b4pad, uint16_t *wgp, float *bgp)
 {
@@ -266,7 +267,6 @@ __global__ void k_cl_refresh(const float *__restrict__ p, uint16_t *wg, uint16_t
     if (n < (long long)CL_G * CL_XH) {
         const int r = (int)(n / CL_XH), c = (int)(n % CL_XH);
         const uint16_t v = cl_wg_masked(r, c) ? (uint16_t)0 : f32_to_bf16_rn(p[CL_OFF_WG + n]);
-        wg[n] = v;
         wgT[(long long)c * CL_G + r] = v;
         wgp[(long long)cl_gate_perm(r) * CL_XH + c] = v;
     }
@@ -464,7 +464,7 @@ struct omx_closure {
     long long adam_step = 0;
     double e_scale = 1.0, d_scale = 1.0;   // field and dipole scales of the training data
     omx::DBuf<float> p, g, m, v, b4pad, bgp;
-    omx::DBuf<uint16_t> wg, wgT, w1, w1T, w2, w2T, w3, w3T, w4, w4T, wgp;   // wgp, bgp: deployment gate order
+    omx::DBuf<uint16_t> wgT, w1, w1T, w2, w2T, w3, w3T, w4, w4T, wgp;   // wgp, bgp: the GRU epilogue's gate order
     // training / batch work buffers (grown on demand)
     omx::DBuf<float> e, tgt, G, H, cache, A1, A2, A3, Y, dHm, dhd, part;
     omx::DBuf<uint16_t> XH, Hb, A1b, A2b, A3b, dY, dZ1, dZ2, dZ3, dG, T1, T2;
@@ -494,7 +494,7 @@ static bool cl_refresh(omx_closure *c, std::string &err)
 {
     k_cl_refresh<<<cl_blocks((long long)CL_F * CL_F > (long long)CL_G * CL_XH ? (long long)CL_F * CL_F
                                                                             : (long long)CL_G * CL_XH),
-                   256, 0, c->stream>>>(c->p.p, c->wg.p, c->wgT.p, c->w1.p, c->w1T.p, c->w2.p, c->w2T.p, c->w3.p,
+                   256, 0, c->stream>>>(c->p.p, c->wgT.p, c->w1.p, c->w1T.p, c->w2.p, c->w2T.p, c->w3.p,
                                         c->w3T.p, c->w4.p, c->w4T.p, c->b4pad.p, c->wgp.p, c->bgp.p);
     CL_CK(cudaGetLastError());
     return true;
@@ -815,7 +815,7 @@ int omx_closure_create(omx_closure **out)
     omx_closure *c = new omx_closure;
     bool ok = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess && c->p.ensure(CL_NPARAM) &&
               c->g.ensure(CL_NPARAM) && c->m.ensure(CL_NPARAM) && c->v.ensure(CL_NPARAM) && c->b4pad.ensure(CL_OUT) &&
-              c->wg.ensure((size_t)CL_G * CL_XH) && c->wgT.ensure((size_t)CL_G * CL_XH) &&
+              c->wgT.ensure((size_t)CL_G * CL_XH) &&
               c->w1.ensure((size_t)CL_F * CL_H) && c->w1T.ensure((size_t)CL_F * CL_H) &&
               c->w2.ensure((size_t)CL_F * CL_F) && c->w2T.ensure((size_t)CL_F * CL_F) &&
               c->w3.ensure((size_t)CL_F * CL_F) && c->w3T.ensure((size_t)CL_F * CL_F) &&
