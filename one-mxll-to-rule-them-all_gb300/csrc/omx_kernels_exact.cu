@@ -69,10 +69,14 @@ template <class R> void launch_inject(const FieldPtrs<R> &F, const JState &J, co
 }
 // Emitters up to which a group is stepped with one lane per state word (k_emit_lanes) instead of one
 // thread per emitter: few emitters wait on one warp's chain of FP64 instructions, which the lanes
-// shorten, many on the FP64 pipe, for which the lanes' extra instructions count.  Measured, us for the
-// emitter step and scatter, a thread / lanes per emitter: 2-level 300 12.6 / 10.5, 2000 13.7 / 10.5,
-// 10000 15.3 / 13.7, 20000 17.4 / 18.7; 3-level 300 20.9 / 12.7, 2000 21.8 / 12.7, 5000 21.9 / 17.7,
-// 10000 22.9 / 22.9, 20000 29.0 / 36.3.
+// shorten, many on the FP64 pipe, for which the lanes' extra instructions count.  Alone the lanes win up
+// to about 16000 two-level and 9000 three-level emitters (us for the step and scatter, a thread / lanes
+// per emitter: 2-level 3000 14.5 / 10.6, 10000 14.8 / 14.7, 20000 17.5 / 19.6; 3-level 3000 20.8 / 13.1,
+// 6144 21.8 / 18.5, 10000 22.1 / 22.9, 20000 27.3 / 35.5), but beside a field pass their instructions also
+// slow the pass, and the line lies where whole steps cross: 2-level, FP32 TEz 1531 x 1147 with 5000 33.2
+// / 30.2, 6144 33.4 / 32.9, 8192 33.8 / 35.6, 10000 34.5 / 37.9; 128^3 8192 52.5 / 51.3, 12000 53.8 / 53.8;
+// TMz 4096^2 (one fused pass) 10000 130.8 / 129.1, 129 either way from 3000 on; 3-level, 128^3 6144 56.5 /
+// 54.4, 9000 59.4 / 59.5, FP64 TMz 600 x 600 6144 39.3 / 36.8, 8192 39.8 / 40.0.
 constexpr int EMIT_LANES_MOST[2] = {8192, 6144};   // 2-level, 3-level
 template <class R> void launch_emit(const FieldPtrs<R> &F, const Lay &L, const EmitArgs &A, StepParam move, void *s)
 {
