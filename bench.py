@@ -618,8 +618,8 @@ def cfg5_decks(count, side_min=64, side_max=256):
 
 
 def batch_shape_text(shape):
-    """(the batched pass, its tile) from omx_batch_autotune's choice; grids that each step in place keep
-    that form, side by side, where it timed faster than the staged shape the tuner returns."""
+    """(the batched pass, its tile) from omx_batch_autotune's choice, for a batch that does not step its
+    members in place."""
     if shape < 1000:
         return "the two half-step passes of every grid (k_batch3)", "tile depth %d" % shape
     form = shape // 1000 % 1000
@@ -671,15 +671,16 @@ def measure_cfg5(args, dist, K, W, cpu_seconds):
     clk = clocks.stop()
     t_batch = dist.max(t_batch)
     traces_b = [g.drain_detectors()[1] for g in grids]
-    alg = sum(g.algorithmic_bytes(omx.KC_H) + g.algorithmic_bytes(omx.KC_E) for g in grids)   # per step
+    per_grid = [g.algorithmic_bytes(omx.KC_H) + g.algorithmic_bytes(omx.KC_E) for g in grids]   # per step
+    alg = sum(per_grid)
     batch.kill()
     for g in grids:
         g.kill()
     # ---- the same grids one at a time (each its own omx_run, CUDA graphs per grid, the graphs
     # captured before the clock) with the batch's arithmetic (traces compared bit for bit), each
     # grid in the fused shape its own autotuner picks (the fused pass only: its bits are the batch's)
-    t_solo, same = 0.0, True
-    for d, tb in zip(dks, traces_b):
+    t_solo, same, inplace = 0.0, True, False
+    for d, tb, words in zip(dks, traces_b, per_grid):
         g = build_gpu(d, "fp32")[0]
         g.set_step_form(omx.STEP_SINGLE_PASS)
         g.autotune(reps=3)
@@ -692,6 +693,7 @@ def measure_cfg5(args, dist, K, W, cpu_seconds):
         t_solo += time.perf_counter() - t0
         ts = g.drain_detectors()[1]
         same = same and ts.shape == tb.shape and bool(np.array_equal(ts, tb))
+        inplace = inplace or words > g.algorithmic_bytes(omx.KC_E)    # the batch read and wrote more than staged
         g.kill()
     t_solo = dist.max(t_solo)
     value = dist.world * cells * K / t_batch / 1e9
@@ -721,9 +723,9 @@ def measure_cfg5(args, dist, K, W, cpu_seconds):
                        "cells": cells, "sides": sides, "precision": "fp32",
                        "parallelism": f"replicas x{dist.world}" if dist.world > 1 else "single GPU",
                        "l2": "working set %.1f GB > 126 MB L2, no flush" % (cells * 6 * 4 / 1e9),
-                       "loop": "omx_batch_run: each grid in place on one of the batch's streams where that timed "
-                               "faster, else %s; the steps captured in CUDA graphs; shape from "
-                               "omx_batch_autotune: %s" % batch_shape_text(shape),
+                       "loop": "omx_batch_run: %s; the steps captured in CUDA graphs; form from omx_batch_autotune" %
+                               ("each grid in place, side by side on the batch's streams" if inplace else
+                                "%s, %s" % batch_shape_text(shape)),
                        "timing": "wall clock around omx_batch_run + omx_batch_synchronize"},
             "one_at_a_time": {"value": solo_value, "unit": "Gcell-updates/s",
                               "how": "the same grids, each its own omx_run (CUDA graph) in the fused shape "
@@ -731,7 +733,7 @@ def measure_cfg5(args, dist, K, W, cpu_seconds):
                               "batch_speedup": value / solo_value,
                               "detector_traces_bit_identical": same,
                               "arithmetic": "one fused pass per grid and step, as the batch"},
-            "roofline": {"bound": "hbm", "kernel": "k_f3p_h / k_f3p_e side by side, or " + batch_shape_text(shape)[0],
+            "roofline": {"bound": "hbm", "kernel": "k_f3p_h / k_f3p_e side by side" if inplace else batch_shape_text(shape)[0],
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": None, "peak_source": peak_kind,
                          "algorithmic_bytes_per_step": alg,
