@@ -894,13 +894,13 @@ __global__ void __launch_bounds__(32 * TY, 1536 / (32 * TY)) k_f3g_e(Fused3Args 
 // the working set, and thousands of short blocks instead of a hundred that march their planes one
 // by one (f3_inplace_rule has both sides' times).  The H launch advances the device-loop step counter.
 //
-// The march is instruction-bound before it is memory-bound (a 128^3 pass through the general runs'
-// loop issued 226 instructions per warp and plane: 43.6 us per step, 160^3 102 us; this loop 37.9 and
-// 89), so a warp without an x or y slab takes a loop
-// compiled without their terms (XY = false), the slab coefficients of the others are held per
-// thread, and a plane that needs more (a z slab, the media box, the plane source) is a branch that the
-// whole warp takes or leaves.  The operations and their rounding are f3t_hx / f3t_hy / f3t_hz's and
-// f3t_e_general's.
+// The march waits for its loads: of 19 cycles between two instructions of a warp 13 to 15 go to memory,
+// no pipe and no memory level is above 34 % (128^3, 123 and 135 instructions per warp and plane in the
+// H and E pass).  So a warp without an x or y slab takes a loop compiled without their terms (XY =
+// false), the slab coefficients of the others are held per thread, and a plane that needs more (a z
+// slab, the media box, the plane source) is a branch that the whole warp takes or leaves: 128^3 37.9 us
+// per step, 160^3 89, against 43.6 and 102 through the general runs' loop.  The operations and their
+// rounding are f3t_hx / f3t_hy / f3t_hz's and f3t_e_general's.
 constexpr int F3P_H_BLOCKS = 8, F3P_E_BLOCKS = 8;   // blocks per SM: 64 registers (10 and 9: 39, 6: 46 us at 128^3 against 38)
 
 template <bool XY>

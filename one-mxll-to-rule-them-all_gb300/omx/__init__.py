@@ -267,8 +267,8 @@ class TMxll:
         return times[:n].copy(), vals[:n, :npts].copy()
 
     def set_step_form(self, form):
-        """Kernel form of the FP32 step: STEP_DEFAULT, STEP_TWO_PASS (the batch arithmetic) or
-        STEP_SINGLE_PASS."""
+        """Kernel form of the FP32 step: STEP_DEFAULT, STEP_TWO_PASS (the two half-step passes) or
+        STEP_SINGLE_PASS (3D always staged)."""
         self._chk(lib().omx_set_step_form(self._ctx, int(form)))
 
     def drain_async(self):
@@ -404,8 +404,8 @@ def device_count():
 
 
 class Batch:
-    """Several configured 3D grids of one precision advanced together (omx_batch_*): one
-    persistent launch per pass over all grids' tiles, the step captured in a CUDA graph.  Each
+    """Several configured 3D grids of one precision advanced together (omx_batch_*): side by side in
+    place, or few launches per step over all grids' tiles; steps captured in CUDA graphs.  Each
     grid computes exactly what its own `run` would."""
 
     def __init__(self, grids):
@@ -415,8 +415,8 @@ class Batch:
         A.check(lib().omx_batch_create(arr, len(self.grids), C.byref(self._b)))
 
     def autotune(self, reps=10):
-        """Launch shape of the batched passes, timed on the zero initial fields; returns it
-        (encoded as omx_batch_autotune describes)."""
+        """Form and launch shape of the batched steps, timed on the zero initial fields; returns the shape
+        (encoded as omx_batch_autotune describes; set_launch_shape with it keeps the form)."""
         choice = C.c_int()
         A.check(lib().omx_batch_autotune(self._b, int(reps), C.byref(choice)))
         return choice.value
