@@ -4077,7 +4077,9 @@ struct Capture {
     ~Capture()
     {
         cudaGraph_t g = nullptr;
-        if (open && cudaStreamEndCapture(s, &g) == cudaSuccess && g) cudaGraphDestroy(g);
+        if (!open) return;
+        if (cudaStreamEndCapture(s, &g) == cudaSuccess && g) cudaGraphDestroy(g);
+        cudaGetLastError();   // the error that left it is on its way to the caller
     }
     cudaGraph_t end()
     {
